@@ -31,8 +31,10 @@ __global__ void k_build_V(const SubDev *, const double *, const int *, const int
                           const double *, double *);
 __global__ void k_build_Fc(const SubDev *, const double *, const int *, const int *, const double *,
                            const long long *, double *);
-__global__ void k_trsv_fwd(const SubDev *, const double *, double *, long long);
-__global__ void k_trsv_bwd(const SubDev *, const double *, double *, long long);
+size_t ksolve_smem(int max_blocks);
+cudaError_t ksolve_prepare(int optin);
+int ksolve_ctas(const std::vector<int> &blocks);
+cudaError_t ksolve_launch(const SubDev *, const int *, int, const double *, double *, int, int, int *, cudaStream_t);
 __global__ void k_gather_b(int, const int *, const int *, const double *, const double *, double *,
                            const PcpgState *);
 template <typename T>
@@ -497,6 +499,23 @@ int Engine::upload_layout(Problem &p, std::string &err) {
     npart_ = cdiv(nlam_, 256);
     d_partial_ = alloc<double>(npart_, err, rc);
     d_st_ = alloc<PcpgState>(1, err, rc);
+    d_kserr_ = alloc<int>(1, err, rc);
+    if (!rc) CK(cudaMemsetAsync(d_kserr_, 0, sizeof(int), s_));
+    {
+        std::vector<int> order(nsub_), blocks(nsub_);
+        std::iota(order.begin(), order.end(), 0);
+        for (int d = 0; d < nsub_; ++d) blocks[d] = (hs_[d].nr + 31) / 32 + hs_[d].nt;
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return blocks[a] > blocks[b]; });
+        ks_blocks_ = blocks[order[0]];
+        ks_ctas_ = ksolve_ctas(blocks);
+        d_ksord_ = alloc<int>(nsub_, err, rc);
+        if (rc) return rc;
+        CK(cudaMemcpy(d_ksord_, order.data(), nsub_ * sizeof(int), cudaMemcpyHostToDevice));
+        int optin = 0;
+        CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, opt_.device));
+        if (ksolve_smem(ks_blocks_) > size_t(optin)) ks_blocks_ = 0;
+        else CK(ksolve_prepare(optin));
+    }
     d_hist_ = alloc<double>(size_t(std::max(opt_.max_iter, 0)) + 1, err, rc);
     if (rc) return rc;
     {
@@ -1048,6 +1067,13 @@ int Engine::apply(int op, const double *x, double *y, int nrhs, std::string &err
     return HTF_OK;
 }
 
+// v <- K_reg^{-1} v: the cluster kernel of ksolve.cu, or the multi-RHS kernels for subdomains whose results do
+// not fit its shared memory (about 19 000 DOFs)
+void Engine::ksolve(double *v) {
+    if (ks_blocks_ > 0) ksolve_launch(d_subs_, d_ksord_, nsub_, d_K_, v, ks_blocks_, ks_ctas_, d_kserr_, s_);
+    else trsm_multi(v, 1);
+}
+
 // x = K_HT^+ f, d = Bf x, lambda0 = Gf (GfTGf)^{-1} Rf^T f  (Cluster.cpp:1385-1394, 967-1040);
 // with x_solved the triangular solves K_reg^{-1} f were done already (for
 // several load cases at once) and x_solved holds them
@@ -1055,8 +1081,7 @@ void Engine::init_rhs(const double *f, const double *x_solved) {
     const double *x = x_solved;
     if (!x) {
         cudaMemcpyAsync(d_full_, f, nfull_ * sizeof(double), cudaMemcpyDeviceToDevice, s_);
-        k_trsv_fwd<<<dim3(nsub_, 1), 256, 0, s_>>>(d_subs_, d_K_, d_full_, 0);
-        k_trsv_bwd<<<dim3(nsub_, 1), 256, 0, s_>>>(d_subs_, d_K_, d_full_, 0);
+        ksolve(d_full_);
         x = d_full_;
     }
     k_bc_rt<<<nsub_, 256, 0, s_>>>(d_subs_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_R_, x, f, d_t_);
@@ -1087,14 +1112,12 @@ void Engine::reconstruct(const double *f, double *u_dev) {
     k_gather_b<<<cdiv(nslots_, 256), 256, 0, s_>>>(nslots_, d_slot_ptr_, d_slot_ent_, d_lam_, nullptr, d_xb_, nullptr);
     k_full_minus_b<<<nsub_, 256, 0, s_>>>(d_subs_, d_xb_, d_full_);
     cudaMemcpyAsync(d_full2_, d_full_, nfull_ * sizeof(double), cudaMemcpyDeviceToDevice, s_);
-    k_trsv_fwd<<<dim3(nsub_, 1), 256, 0, s_>>>(d_subs_, d_K_, d_full2_, 0);
-    k_trsv_bwd<<<dim3(nsub_, 1), 256, 0, s_>>>(d_subs_, d_K_, d_full2_, 0);
+    ksolve(d_full2_);
     k_bc_rt<<<nsub_, 256, 0, s_>>>(d_subs_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_R_, d_full2_, d_full_, d_t_);
     k_gc<<<cdiv(ngc_total_, 256), 256, 0, s_>>>(ngc_total_, d_gptr_, d_gidx_, d_t_, d_gc_, nullptr);
     coarse_apply(d_gc_, d_s_, nullptr);
     k_sub_bct<<<nsub_, 32, 0, s_>>>(d_subs_, d_cl_, d_bcr_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_s_, d_full_);
-    k_trsv_fwd<<<dim3(nsub_, 1), 256, 0, s_>>>(d_subs_, d_K_, d_full_, 0);
-    k_trsv_bwd<<<dim3(nsub_, 1), 256, 0, s_>>>(d_subs_, d_K_, d_full_, 0);
+    ksolve(d_full_);
     k_add_R<<<nsub_, 256, 0, s_>>>(d_subs_, d_cl_, d_R_, d_H_, d_s_, d_alpha_, d_full_);
     if (u_dev) k_gather_u<<<cdiv(ndof_, 256), 256, 0, s_>>>(ndof_, d_win_, d_full_, u_dev);
 }
@@ -1125,7 +1148,7 @@ int Engine::solve_one(Problem &p, int rhs, double *u_dev, int &iters, double &no
     }
     PcpgState hst;
     const int every = std::max(1, opt_.check_every);
-    launches_ += 27 + 12;     // kernels of the start (x, d, lambda0, g0, Pz) and of the reconstruction
+    launches_ += 24 + 9;      // kernels of the start (x, d, lambda0, g0, Pz) and of the reconstruction
     for (;;) {
         for (int k = 0; k < every; ++k) CK(cudaGraphLaunch(graph_, s_));
         launches_ += (long long)every * kernels_per_iter_;
@@ -1152,6 +1175,14 @@ int Engine::solve_one(Problem &p, int rhs, double *u_dev, int &iters, double &no
     cudaEventDestroy(e1);
     reconstruct(f, u_dev);
     CK(cudaGetLastError());
+    int kserr = 0;
+    CK(cudaMemcpyAsync(&kserr, d_kserr_, sizeof(int), cudaMemcpyDeviceToHost, s_));
+    CK(cudaStreamSynchronize(s_));
+    if (kserr) {
+        CK(cudaMemsetAsync(d_kserr_, 0, sizeof(int), s_));
+        err = "K_reg solve timed out on a barrier";
+        return kserr;
+    }
     if (hst.done == 2) { err = "PCPG breakdown (w'Fw <= 0 or non-finite)"; return HTF_EBREAKDOWN; }
     return HTF_OK;
 }

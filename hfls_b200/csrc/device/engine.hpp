@@ -99,6 +99,7 @@ public:
 private:
     template <typename T> T *alloc(size_t n, std::string &err, int &rc);
     void init_rhs(const double *f, const double *x_solved = nullptr);   // d = Bf K_HT^+ f, lambda0
+    void ksolve(double *v);                               // v = K_reg^{-1} v, one column of nfull
     void trsm_multi(double *v, int nrhs);                 // v_j = K_reg^{-1} v_j, nrhs <= 32 columns of nfull
     void reconstruct(const double *f, double *u_dev);     // u from lambda, alpha
     double pcpg_start(PcpgState *st);                     // g0, Pg, z, Pz; returns nothing useful
@@ -243,6 +244,9 @@ private:
     int tc_smem_ = 0, vt_nch_ = 1, vt_qn_ = 64;
     long long aoff_ = 0;                       // 4-byte words per slab array
     // vectors
+    int *d_kserr_ = nullptr;                   // time-out flag of the K_reg solves
+    int *d_ksord_ = nullptr, ks_ctas_ = 1;     // subdomains largest first, CTAs per cluster
+    int ks_blocks_ = 0;                        // most 32-row blocks of a subdomain (0: too many for ksolve.cu)
     double *d_f_ = nullptr, *d_full_ = nullptr, *d_full2_ = nullptr;
     double *d_lam_ = nullptr, *d_g_ = nullptr, *d_w_ = nullptr, *d_Fw_ = nullptr, *d_Pg_ = nullptr,
            *d_z_ = nullptr, *d_Pz_ = nullptr, *d_d_ = nullptr, *d_tmp_ = nullptr;

@@ -16,7 +16,7 @@
 //  k_lauum_tiles     F = X^T X = (K_reg^{-1})_bb into packed tiles.
 //  k_build_V/Fc      V = [F Bc_b^T, -R_b] and Fc_d = Bc_b F Bc_b^T
 //                    (Cluster.cpp:150-185).
-//  k_trsv_fwd/bwd    batched dense triangular solves with the full factor.
+//  k_trsm_fwd/bwd_multi  batched multi-RHS triangular solves with the full factor.
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -598,78 +598,6 @@ __global__ void k_build_Fc(const SubDev *__restrict__ subs, const double *__rest
         double v = 0.0;
         for (int e = bce_ptr[sd.bce_off + r]; e < bce_ptr[sd.bce_off + r + 1]; ++e) v += bce_val[e] * V[bce_pos[e]];
         out[idx] = v;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// batched dense triangular solves with the full factor (N x N, lower)
-// v: full vectors (N per subdomain at nfull_off, nrhs columns of length ldv)
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_trsv_fwd(const SubDev *__restrict__ subs,
-                                                  const double *__restrict__ Kbuf, double *__restrict__ v,
-                                                  long long ldv) {
-    __shared__ double part[8][32];
-    __shared__ double xs[32];
-    const SubDev &sd = subs[blockIdx.x];
-    double *x = v + sd.nfull_off + (size_t)blockIdx.y * ldv;
-    const int N = sd.N, lane = threadIdx.x % 32, w = threadIdx.x / 32;
-    for (int kb = 0; kb < N; kb += 32) {
-        const int nrow = min(32, N - kb);
-        double acc = 0.0;
-        const int row = kb + lane;
-        if (lane < nrow)
-            for (int c = w; c < kb; c += 8) acc += Kbuf[kidx(sd, row, c)] * x[c];
-        part[w][lane] = acc;
-        __syncthreads();
-        if (w == 0) {
-            double a = (lane < nrow) ? x[row] : 0.0;
-            for (int q = 0; q < 8; ++q) a -= part[q][lane];
-            for (int q = 0; q < nrow; ++q) {
-                double xq = 0.0;
-                if (lane == q) xq = a / Kbuf[kidx(sd, row, row)];
-                xq = __shfl_sync(0xffffffffu, xq, q);
-                if (lane == q) xs[q] = xq;
-                if (lane > q && lane < nrow) a -= Kbuf[kidx(sd, row, kb + q)] * xq;
-            }
-            __syncwarp();
-            if (lane < nrow) x[row] = xs[lane];
-        }
-        __syncthreads();
-    }
-}
-
-__global__ void __launch_bounds__(256) k_trsv_bwd(const SubDev *__restrict__ subs,
-                                                  const double *__restrict__ Kbuf, double *__restrict__ v,
-                                                  long long ldv) {
-    __shared__ double acc_s[32];
-    const SubDev &sd = subs[blockIdx.x];
-    double *x = v + sd.nfull_off + (size_t)blockIdx.y * ldv;
-    const int N = sd.N, lane = threadIdx.x % 32, w = threadIdx.x / 32;
-    const int nblk = (N + 31) / 32;
-    for (int b = nblk - 1; b >= 0; --b) {
-        const int kb = 32 * b, nrow = min(32, N - kb);
-        // acc[r] = x[kb+r] - sum_{c >= kb+nrow} L[c][kb+r] x[c]
-        for (int r = w; r < nrow; r += 8) {
-            const double *col = Kbuf + kcol(sd, kb + r);
-            double s = 0.0;
-            for (int c = kb + nrow + lane; c < N; c += 32) s += col[c] * x[c];
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) acc_s[r] = x[kb + r] - s;
-        }
-        __syncthreads();
-        if (w == 0) {
-            double a = (lane < nrow) ? acc_s[lane] : 0.0;
-            for (int q = nrow - 1; q >= 0; --q) {
-                double xq = 0.0;
-                if (lane == q) xq = a / Kbuf[kidx(sd, kb + q, kb + q)];
-                xq = __shfl_sync(0xffffffffu, xq, q);
-                if (lane == q) acc_s[q] = xq;
-                if (lane < q) a -= Kbuf[kidx(sd, kb + q, kb + lane)] * xq;
-            }
-            __syncwarp();
-            if (lane < nrow) x[kb + lane] = acc_s[lane];
-        }
-        __syncthreads();
     }
 }
 
