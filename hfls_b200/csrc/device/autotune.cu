@@ -30,8 +30,7 @@
 
 namespace htf {
 
-template <typename T>
-__global__ void k_symv_units(const SymvUnit *, const SubDev *, const T *, const double *, const double *, double *,
+__global__ void k_symv_units(const SymvUnit *, const SubDev *, const double *, const double *, const double *, double *,
                              double *, const PcpgState *);
 
 #define CKE(call)                                                          \
@@ -43,6 +42,7 @@ __global__ void k_symv_units(const SymvUnit *, const SubDev *, const T *, const 
 namespace {
 
 constexpr long long SYMV_TUNE_MIN_TILES = 1LL << 17;   // 1 GiB of FP64 tiles
+constexpr long long SYMV_MIN_UNITS = 4 * 148;
 const int CANDIDATES[] = {8, 12, 16, 24, 32, 48, 64, 96};
 
 std::mutex g_mu;
@@ -142,40 +142,41 @@ void write_file(const std::string &path) {
 
 // Units of the given schedule (host side): sets u0 / u1 of every subdomain.
 void Engine::build_units(const std::vector<int> &tiles, std::vector<SymvUnit> &units, long long &yoff,
-                         int &smem, std::vector<int> &rbptr, std::vector<int> &rbunit) {
+                         int &smem, std::vector<int> &rbptr, std::vector<long long> &rboff) {
     units.clear();
     rbptr.assign(1, 0);
-    rbunit.clear();
+    rboff.clear();
     yoff = 0;
     int max_rows = 0;
-    std::vector<std::vector<int>> cover;
+    std::vector<std::vector<long long>> cover;
     for (int d = 0; d < nsub_; ++d) {
         SubDev &h = hs_[d];
         h.u0 = int(units.size());
-        partition(h.nt, tiles[bucket_of(h.nt)], [&](long long t0, long long t1, int kind, int row0, int rows, int rowI) {
+        partition(h.nt, std::min(tiles[bucket_of(h.nt)], unit_cap_), [&](long long t0, long long t1, int kind, int row0, int rows, int rowI) {
             units.push_back(SymvUnit{d, kind, t0, t1, yoff, rows, row0, rowI, 0});
             yoff += rows;
             max_rows = std::max(max_rows, rows);
         });
         h.u1 = int(units.size());
-        // the units covering each 32-row block, in unit order (the order of the partial sums)
-        cover.assign(h.nt, std::vector<int>());
+        // where the partial sums of each 32-row block start, in unit order (the order in which they are added)
+        cover.assign(h.nt, std::vector<long long>());
         for (int k = h.u0; k < h.u1; ++k) {
             const SymvUnit &u = units[k];
             const int seg = u.kind == 2 ? u.rows - TILE : u.rows;
-            for (int R = u.row0 / TILE; R < (u.row0 + seg + TILE - 1) / TILE && R < h.nt; ++R) cover[R].push_back(k);
-            if (u.kind == 2) {
-                const int R = u.rowI / TILE;
-                if (R < h.nt && (cover[R].empty() || cover[R].back() != k)) cover[R].push_back(k);
-            }
+            for (int R = u.row0 / TILE; R < (u.row0 + seg) / TILE && R < h.nt; ++R)
+                if (u.kind != 2 || R != u.rowI / TILE)      // a diagonal tile adds only to its row block
+                    cover[R].push_back(u.y_off + TILE * R - u.row0);
+            if (u.kind == 2) cover[u.rowI / TILE].push_back(u.y_off + seg);
         }
         h.rb_off = int(rbptr.size()) - 1;
         for (int R = 0; R < h.nt; ++R) {
-            rbunit.insert(rbunit.end(), cover[R].begin(), cover[R].end());
-            rbptr.push_back(int(rbunit.size()));
+            rboff.insert(rboff.end(), cover[R].begin(), cover[R].end());
+            rbptr.push_back(int(rboff.size()));
         }
     }
-    for (int d = 0; d < nsub_; ++d) units.push_back(SymvUnit{d, 1, 0, 0, 0, 0, 0, 0, 0});   // V^T x units
+    for (int d = 0; d < nsub_; ++d)                              // V^T x units
+        for (int c = 0; c < hs_[d].c + 6; c += SYMV_VCOLS)
+            units.push_back(SymvUnit{d, 1, c, std::min(c + SYMV_VCOLS, hs_[d].c + 6), 0, 0, 0, 0, 0});
     smem = SYMV_ROW_DOUBLES * max_rows * int(sizeof(double));
 }
 
@@ -190,20 +191,21 @@ int Engine::apply_schedule(const std::vector<int> &tiles, bool subs_on_device, s
         CKE(cudaMemcpyAsync(hs_.data(), d_subs_, nsub_ * sizeof(SubDev), cudaMemcpyDeviceToHost, s_));
         CKE(cudaStreamSynchronize(s_));
     }
-    std::vector<int> rbptr, rbunit;
-    build_units(tiles, units, yoff, smem, rbptr, rbunit);
+    std::vector<int> rbptr;
+    std::vector<long long> rboff;
+    build_units(tiles, units, yoff, smem, rbptr, rboff);
     if ((long long)units.size() > units_cap_ || yoff > ypart_cap_ || smem > symv_smem_cap_ ||
-        (long long)rbptr.size() > rbptr_cap_ || (long long)rbunit.size() > rbunit_cap_) {
+        (long long)rbptr.size() > rbptr_cap_ || (long long)rboff.size() > rboff_cap_) {
         err = "SYMV schedule exceeds its buffers";
         return HTF_EINVAL;
     }
-    nunits_ = int(units.size()) - nsub_;
+    nunits_ = int(units.size()) - nvunits_;
     symv_smem_ = smem;
     schedule_ = tiles;
     CKE(cudaMemcpyAsync(d_units_, units.data(), units.size() * sizeof(SymvUnit), cudaMemcpyHostToDevice, s_));
     CKE(cudaMemcpyAsync(d_rbptr_, rbptr.data(), rbptr.size() * sizeof(int), cudaMemcpyHostToDevice, s_));
-    if (!rbunit.empty())
-        CKE(cudaMemcpyAsync(d_rbunit_, rbunit.data(), rbunit.size() * sizeof(int), cudaMemcpyHostToDevice, s_));
+    if (!rboff.empty())
+        CKE(cudaMemcpyAsync(d_rboff_, rboff.data(), rboff.size() * sizeof(long long), cudaMemcpyHostToDevice, s_));
     // (pageable copies: the host vectors may go out of scope once the calls return)
     if (subs_on_device)
         CKE(cudaMemcpyAsync(d_subs_, hs_.data(), nsub_ * sizeof(SubDev), cudaMemcpyHostToDevice, s_));
@@ -217,6 +219,12 @@ int Engine::alloc_units(std::string &err) {
     int rc = HTF_OK;
     std::vector<int> cands(1, SYMV_DEFAULT_TILES);
     if (opt_.autotune) cands.assign(std::begin(CANDIDATES), std::end(CANDIDATES));
+    // A schedule's unit sizes are upper bounds: a problem of few tiles is cut into at least SYMV_MIN_UNITS units
+    // (four CTAs per SM), down to 4 tiles each, one per warp.  Measured per iteration: 528 tiles (8 subdomains) 59
+    // us with units of 48 tiles, 41 us with 4; 7 900 tiles (32 subdomains) 88 us with 48, 78 with 12, 82 with 4;
+    // from 29 000 tiles on the bound is above 48 and the schedule's own sizes hold (43 000 tiles: 252 us with 32 or
+    // 48, 262 with 16).
+    unit_cap_ = int(std::max<long long>(4, std::min<long long>(ntiles_ / SYMV_MIN_UNITS, 1 << 20)));
     // every unit's row window is at most 32 (ut + 1) rows of 5 doubles: the
     // largest candidate (96 tiles) needs 124 KB, within the 227 KB opt-in limit
     long long bu[SYMV_BUCKETS][8] = {}, by[SYMV_BUCKETS][8] = {};
@@ -226,13 +234,15 @@ int Engine::alloc_units(std::string &err) {
         for (size_t c = 0; c < cands.size(); ++c) {
             long long nu = 0, yr = 0;
             int mr = 0;
-            unit_stats(h.nt, cands[c], nu, yr, mr);
+            unit_stats(h.nt, std::min(cands[c], unit_cap_), nu, yr, mr);
             bu[b][c] += nu;
             by[b][c] += yr;
             scap = std::max(scap, SYMV_ROW_DOUBLES * mr * int(sizeof(double)));
         }
     }
-    long long ucap = nsub_, ycap = 0;
+    nvunits_ = 0;
+    for (auto &h : hs_) nvunits_ += (h.c + 6 + SYMV_VCOLS - 1) / SYMV_VCOLS;
+    long long ucap = nvunits_, ycap = 0;
     for (int b = 0; b < SYMV_BUCKETS; ++b) {
         long long mu = 0, my = 0;
         for (size_t c = 0; c < cands.size(); ++c) { mu = std::max(mu, bu[b][c]); my = std::max(my, by[b][c]); }
@@ -242,20 +252,20 @@ int Engine::alloc_units(std::string &err) {
     units_cap_ = ucap;
     ypart_cap_ = ycap;
     symv_smem_cap_ = scap;
-    // row-block lists: a unit covers at most rows / 32 + 1 blocks (its window and its tile row)
+    // row-block lists: at most one entry per 32 partial rows
     long long ntsum = 0;
     for (auto &h : hs_) ntsum += h.nt;
     rbptr_cap_ = ntsum + 1;
-    rbunit_cap_ = ycap / TILE + 2 * ucap;
+    rboff_cap_ = ycap / TILE;
     d_units_ = alloc<SymvUnit>(ucap, err, rc);
     d_ypart_ = alloc<double>(ycap, err, rc);
     d_rbptr_ = alloc<int>(rbptr_cap_, err, rc);
-    d_rbunit_ = alloc<int>(rbunit_cap_, err, rc);
+    d_rboff_ = alloc<long long>(rboff_cap_, err, rc);
     if (rc) return rc;
-    if (scap > 48 * 1024) {
-        CKE(cudaFuncSetAttribute(k_symv_units<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, scap));
-        CKE(cudaFuncSetAttribute(k_symv_units<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, scap));
-    }
+    // the device's limit whatever this problem needs: the attribute is the process's, not the context's
+    int optin = 0;
+    CKE(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, opt_.device));
+    CKE(cudaFuncSetAttribute(k_symv_units, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
     return apply_schedule(std::vector<int>(SYMV_BUCKETS, SYMV_DEFAULT_TILES), false, err);
 }
 
@@ -303,7 +313,7 @@ int Engine::autotune_symv(std::string &err) {
         int rc = apply_schedule(t, true, err);
         if (rc) return rc;
         auto launch = [&] {
-            k_symv_units<double><<<nunits_, SYMV_WARPS * 32, symv_smem_, s_>>>(d_units_, d_subs_, d_F_, d_V_, d_xb_, d_ypart_,
+            k_symv_units<<<nunits_, SYMV_WARPS * 32, symv_smem_, s_>>>(d_units_, d_subs_, d_F_, d_V_, d_xb_, d_ypart_,
                                                                   d_t_, nullptr);
         };
         launch();

@@ -65,7 +65,7 @@ struct SubDev {
     int bce_off;                          // Bc entries (CSR by compressed Bc row): ptr offset
     long long R_off;                      // R in permuted local order, N x 6 (padded rows 0)
     int u0, u1;                           // SYMV work units of this subdomain [u0, u1)
-    int rb_off;                           // its nt + 1 pointers into the units covering each 32-row block
+    int rb_off;                           // its nt + 1 pointers into the partial sums of each 32-row block
     int fix[6];                           // fix DOFs (positions in permuted order)
     double fix_diag[6];                   // original diagonal at the fix DOFs
 };
@@ -120,7 +120,7 @@ HTF_HD long long kidx(const SubDev &s, int r, int c) { return kcol(s, c) + r; }
 HTF_HD long long kld(const SubDev &s, int k) { return s.K_bset < 0 ? s.N : s.N - k; }
 
 // One SYMV work unit of subdomain d: packed tiles [t0, t1) (kind 0 and 2), or
-// the V^T x_b product (kind 1).  Units write partial y sums over the rows
+// the V^T x_b product of columns [t0, t1) of V (kind 1).  Units write partial y sums over the rows
 // their tiles touch (the unit's window) to scratch at y_off; they are summed
 // in unit order.  Kind 0 (whole tile rows): window rows [row0, row0 + rows).
 // Kind 2 (part of one tile row I, rowI = 32 I): window = rows [row0, row0 +
@@ -141,6 +141,7 @@ constexpr int SYMV_BUCKETS = 5;
 constexpr int SYMV_BUCKET_NT[SYMV_BUCKETS] = {8, 16, 32, 64, 1 << 30};
 constexpr int SYMV_DEFAULT_TILES = 48;
 constexpr int SYMV_WARPS = 4;                 // warps of a SYMV work-unit CTA
+constexpr int SYMV_VCOLS = 4;                 // columns of V per V^T x unit
 constexpr int SYMV_ROW_DOUBLES = 1 + SYMV_WARPS;   // shared doubles per window row: x + the warps' partials
 
 // One CTA of the tensor-core multi-RHS product: 128-row block m of
@@ -219,6 +220,25 @@ __device__ __forceinline__ int step_entry(const StepDesc *st, int cnt, int b, F 
         else hi = mid - 1;
     }
     return lo;
+}
+#endif
+
+#ifdef __CUDACC__
+// Launch as a link of the PCPG chain (pcpg_kernels.cu): the kernel may start
+// before its predecessor in the stream has finished and waits for it itself.
+template <typename... P, typename... A>
+inline cudaError_t launch_chain(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
 }
 #endif
 

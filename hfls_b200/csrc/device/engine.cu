@@ -37,38 +37,31 @@ int ksolve_ctas(const std::vector<int> &blocks);
 cudaError_t ksolve_launch(const SubDev *, const int *, int, const double *, double *, int, int, int *, cudaStream_t);
 __global__ void k_gather_b(int, const int *, const int *, const double *, const double *, double *,
                            const PcpgState *);
-template <typename T>
-__global__ void k_symv_units(const SymvUnit *, const SubDev *, const T *, const double *, const double *, double *,
+__global__ void k_symv_units(const SymvUnit *, const SubDev *, const double *, const double *, const double *, double *,
                              double *, const PcpgState *);
-__global__ void k_reduce_correct(const SubDev *, const SymvUnit *, const int *, const int *, const double *, const ClusterDev *,
+__global__ void k_reduce_correct(const SubDev *, const int *, const long long *, const double *, const ClusterDev *,
                                  const double *, const int *, const double *, double *, const PcpgState *);
 __global__ void k_lbt_x(const int2 *, const SubDev *, const double *, const double *, double *, const PcpgState *);
 __global__ void k_lb_t(const int2 *, const SubDev *, const double *, const double *, const double *, double *,
                        const PcpgState *);
 __global__ void k_pack_M(const int2 *, const ClusterDev *, const double *, double *);
-__global__ void k_msym_rows(const int2 *, const ClusterDev *, const double *, const double *, double *, double *,
-                            const PcpgState *);
+__global__ void k_msym_rows(const int2 *, const ClusterDev *, const double *, const int *, const int *, const double *,
+                            double *, double *, const PcpgState *);
 __global__ void k_msym_reduce(const int2 *, const ClusterDev *, const double *, const double *, double *,
                               const PcpgState *);
-__global__ void k_gf_coef(int, const int *, const double *, const double *, double *, double *, const PcpgState *);
 __global__ void k_gf_apply(int, int, const double *, const int *, const double *, const double *, double *,
-                           const double *, double *, const PcpgState *);
-__global__ void k_gf_apply_fused(int, int, const int *, const double *, const double *, const int *,
-                                 const double *, const double *, double *, double *, double *, const double *,
-                                 double *, const PcpgState *);
-__global__ void k_gc(int, const int *, const int *, const double *, double *, const PcpgState *);
+                           const double *, double *, unsigned *, const PcpgState *);
 __global__ void k_coarse(const ClusterDev *, const double *, const double *, double *, const PcpgState *);
 __global__ void k_correct(const SubDev *, const ClusterDev *, const double *, const int *, const double *,
                           double *, const PcpgState *);
 __global__ void k_rows(int, const int *, const double *, const double *, const double *, double *,
                        const double *, double *, const PcpgState *);
-__global__ void k_gft_partial(const int *, const int *, const int *, const int *, const double *,
-                              const double *, double *, const PcpgState *);
+__global__ void k_gft_partial(const int *, const int *, const int *, const double *, const double *, double *, int,
+                              const int *, const double *, double *, double *, unsigned *, const PcpgState *);
 __global__ void k_gf_mult(int, const int *, const double *, const double *, double *);
 __global__ void k_update_lam_g(int, const double *, int, const double *, const double *, double *, double *,
                                PcpgState *);
-__global__ void k_update_w(int, const double *, int, const double *, double *, PcpgState *);
-__global__ void k_finish_iter(const double *, int, PcpgState *, double *);
+__global__ void k_update_w(int, const double *, int, const double *, double *, PcpgState *, double *, unsigned *);
 __global__ void k_init_state(const double *, int, PcpgState *, double, int);
 __global__ void k_axpby(int, double, const double *, double, double *);
 
@@ -198,10 +191,10 @@ void Engine::release(void *p) {
         }
 }
 
-// s = M gc for every cluster (M = [Ac^{-1}] restricted), from the packed symmetric tiles
-void Engine::coarse_apply(const double *gc, double *s, const PcpgState *st) {
-    k_msym_rows<<<nmt_, 128, 0, s_>>>(d_mt_, d_cl_, d_MT_, gc, d_mD_, d_mP_, st);
-    k_msym_reduce<<<nmt_, TILE, 0, s_>>>(d_mt_, d_cl_, d_mD_, d_mP_, s, st);
+// s = M gc for every cluster (M = [Ac^{-1}] restricted, packed symmetric tiles), gc = the sums of t per coarse row
+void Engine::coarse_apply(const double *t, double *s, const PcpgState *st) {
+    launch_chain(k_msym_rows, nmt_, 128, 0, s_, d_mt_, d_cl_, d_MT_, d_gptr_, d_gidx_, t, d_mD_, d_mP_, st);
+    launch_chain(k_msym_reduce, nmt_, 128, 0, s_, d_mt_, d_cl_, d_mD_, d_mP_, s, st);
 }
 
 Engine::~Engine() {
@@ -500,6 +493,8 @@ int Engine::upload_layout(Problem &p, std::string &err) {
     d_partial_ = alloc<double>(npart_, err, rc);
     d_st_ = alloc<PcpgState>(1, err, rc);
     d_kserr_ = alloc<int>(1, err, rc);
+    d_count_ = alloc<unsigned>(2, err, rc);
+    if (!rc) CK(cudaMemsetAsync(d_count_, 0, 2 * sizeof(unsigned), s_));
     if (!rc) CK(cudaMemsetAsync(d_kserr_, 0, sizeof(int), s_));
     {
         std::vector<int> order(nsub_), blocks(nsub_);
@@ -863,7 +858,6 @@ int Engine::outer_coarse(Problem &p, std::string &err) {
     nchunks_ = int(ch_cl.size());
     d_gcl_ = alloc<int>(gcl.size(), err, rc);
     d_gval_ = alloc<double>(gval.size(), err, rc);
-    d_chunk_cl_ = alloc<int>(nchunks_, err, rc);
     d_chunk_beg_ = alloc<int>(nchunks_, err, rc);
     d_chunk_end_ = alloc<int>(nchunks_, err, rc);
     d_cl_chunk_ptr_ = alloc<int>(ncl_ + 1, err, rc);
@@ -874,7 +868,6 @@ int Engine::outer_coarse(Problem &p, std::string &err) {
     if (rc) return rc;
     CK(cudaMemcpyAsync(d_gcl_, gcl.data(), gcl.size() * sizeof(int), cudaMemcpyHostToDevice, s_));
     CK(cudaMemcpyAsync(d_gval_, gval.data(), gval.size() * sizeof(double), cudaMemcpyHostToDevice, s_));
-    CK(cudaMemcpyAsync(d_chunk_cl_, ch_cl.data(), nchunks_ * sizeof(int), cudaMemcpyHostToDevice, s_));
     CK(cudaMemcpyAsync(d_chunk_beg_, ch_beg.data(), nchunks_ * sizeof(int), cudaMemcpyHostToDevice, s_));
     CK(cudaMemcpyAsync(d_chunk_end_, ch_end.data(), nchunks_ * sizeof(int), cudaMemcpyHostToDevice, s_));
     CK(cudaMemcpyAsync(d_cl_chunk_ptr_, clp.data(), (ncl_ + 1) * sizeof(int), cudaMemcpyHostToDevice, s_));
@@ -923,14 +916,12 @@ int Engine::setup(Problem &p, std::string &err) {
                   " bytes of shared memory, the device allows " + std::to_string(optin) + " per block";
             rc = HTF_EINVAL;
         }
+        // (the attribute is the process's, not the context's: the same value for every problem)
         if (!rc)
-            rc = check(cudaFuncSetAttribute(k_gf_apply_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-                       "cudaFuncSetAttribute(k_gf_apply_fused)", err);
+            rc = check(cudaFuncSetAttribute(k_gft_partial, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 2048),
+                       "cudaFuncSetAttribute(k_gft_partial)", err);
         if (!rc)
-            rc = check(cudaFuncSetAttribute(k_gf_coef, cudaFuncAttributeMaxDynamicSharedMemorySize, smem / 2),
-                       "cudaFuncSetAttribute(k_gf_coef)", err);
-        if (!rc)
-            rc = check(cudaFuncSetAttribute(k_gf_apply, cudaFuncAttributeMaxDynamicSharedMemorySize, smem / 2),
+            rc = check(cudaFuncSetAttribute(k_gf_apply, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 2048),
                        "cudaFuncSetAttribute(k_gf_apply)", err);
     }
     lap(2);
@@ -1008,48 +999,47 @@ int Engine::setup(Problem &p, std::string &err) {
 
 // ---------------------------------------------------------------------------
 void Engine::op_F(const double *w, double *Fw, const double *dotv, double *partial, PcpgState *st) {
-    k_gather_b<<<cdiv(nslots_, 256), 256, 0, s_>>>(nslots_, d_slot_ptr_, d_slot_ent_, w, nullptr, d_xb_, st);
-    k_symv_units<double><<<nunits_ + nsub_, SYMV_WARPS * 32, symv_smem_, s_>>>(d_units_, d_subs_, d_F_, d_V_, d_xb_, d_ypart_, d_t_, st);
-    k_gc<<<cdiv(ngc_total_, 256), 256, 0, s_>>>(ngc_total_, d_gptr_, d_gidx_, d_t_, d_gc_, st);
-    coarse_apply(d_gc_, d_s_, st);
-    k_reduce_correct<<<dim3(nsub_, cdiv(max_nbp_, 256)), 256, 0, s_>>>(d_subs_, d_units_, d_rbptr_, d_rbunit_, d_ypart_, d_cl_, d_V_, d_bcr_,
-                                                                       d_s_, d_yb_, st);
-    k_rows<<<npart_, 256, 0, s_>>>(nlam_, d_rslot_, d_rsign_, d_yb_, nullptr, Fw, dotv, partial, st);
+    launch_chain(k_gather_b, cdiv(nslots_, 256), 256, 0, s_, nslots_, d_slot_ptr_, d_slot_ent_, w, nullptr, d_xb_, st);
+    launch_chain(k_symv_units, nunits_ + nvunits_, SYMV_WARPS * 32, symv_smem_, s_, d_units_, d_subs_, d_F_, d_V_, d_xb_,
+                 d_ypart_, d_t_, st);
+    coarse_apply(d_t_, d_s_, st);
+    launch_chain(k_reduce_correct, dim3(nsub_, cdiv(max_nbp_, 64)), 256, 0, s_, d_subs_, d_rbptr_, d_rboff_, d_ypart_,
+                 d_cl_, d_V_, d_bcr_, d_s_, d_yb_, st);
+    launch_chain(k_rows, npart_, 256, 0, s_, nlam_, d_rslot_, d_rsign_, d_yb_, nullptr, Fw, dotv, partial, st);
 }
 
 void Engine::op_M(const double *x, double *z, PcpgState *st) {
-    k_gather_b<<<cdiv(nslots_, 256), 256, 0, s_>>>(nslots_, d_slot_ptr_, d_slot_ent_, x, d_weight_, d_xb_, st);
+    launch_chain(k_gather_b, cdiv(nslots_, 256), 256, 0, s_, nslots_, d_slot_ptr_, d_slot_ent_, x, d_weight_, d_xb_, st);
     if (implicit_) {
-        k_lbt_x<<<nlblk_, 128, 0, s_>>>(d_lblk_, d_subs_, d_K_, d_xb_, d_tb_, st);
-        k_lb_t<<<nlblk_, 128, 0, s_>>>(d_lblk_, d_subs_, d_K_, d_tb_, d_xb_, d_yb_, st);
-        k_rows<<<npart_, 256, 0, s_>>>(nlam_, d_rslot_, d_rsign_, d_yb_, d_weight_, z, nullptr, nullptr, st);
-        return;
+        launch_chain(k_lbt_x, nlblk_, 128, 0, s_, d_lblk_, d_subs_, d_K_, d_xb_, d_tb_, st);
+        launch_chain(k_lb_t, nlblk_, 128, 0, s_, d_lblk_, d_subs_, d_K_, d_tb_, d_xb_, d_yb_, st);
+    } else {
+        launch_chain(k_symv_units, nunits_, SYMV_WARPS * 32, symv_smem_, s_, d_units_, d_subs_, d_S_, d_V_, d_xb_,
+                     d_ypart_, d_t_, st);
+        launch_chain(k_reduce_correct, dim3(nsub_, cdiv(max_nbp_, 64)), 256, 0, s_, d_subs_, d_rbptr_, d_rboff_,
+                     d_ypart_, d_cl_, d_V_, d_bcr_, nullptr, d_yb_, st);
     }
-    k_symv_units<double><<<nunits_, SYMV_WARPS * 32, symv_smem_, s_>>>(d_units_, d_subs_, d_S_, d_V_, d_xb_, d_ypart_, d_t_, st);
-    k_reduce_correct<<<dim3(nsub_, cdiv(max_nbp_, 256)), 256, 0, s_>>>(d_subs_, d_units_, d_rbptr_, d_rbunit_, d_ypart_, d_cl_, d_V_, d_bcr_,
-                                                                       nullptr, d_yb_, st);
-    k_rows<<<npart_, 256, 0, s_>>>(nlam_, d_rslot_, d_rsign_, d_yb_, d_weight_, z, nullptr, nullptr, st);
+    launch_chain(k_rows, npart_, 256, 0, s_, nlam_, d_rslot_, d_rsign_, d_yb_, d_weight_, z, nullptr, nullptr, st);
 }
 
 void Engine::op_P(const double *x, double *Px, double *alpha_out, const double *dotv, double *partial,
                   PcpgState *st) {
-    k_gft_partial<<<nchunks_, 256, 0, s_>>>(d_chunk_cl_, d_chunk_beg_, d_chunk_end_, d_crow_, d_cval_, x, d_gpart_, st);
-    // the coarse coefficient once, then the rows (k_gf_apply_fused, which
-    // recomputes it in every CTA, stays for the allocation-free entry point)
-    k_gf_coef<<<1, 256, 6 * ncl_ * sizeof(double), s_>>>(ncl_, d_cl_chunk_ptr_, d_gpart_, d_invGtG_, d_a_, alpha_out,
-                                                          st);
-    k_gf_apply<<<npart_, 256, 6 * ncl_ * sizeof(double), s_>>>(nlam_, ncl_, d_a_, d_gcl_, d_gval_, x, Px, dotv,
-                                                                partial, st);
+    const size_t smem = 6 * ncl_ * sizeof(double);
+    launch_chain(k_gft_partial, nchunks_, 256, smem, s_, d_chunk_beg_, d_chunk_end_, d_crow_, d_cval_, x, d_gpart_, ncl_,
+                 d_cl_chunk_ptr_, d_invGtG_, d_a_, alpha_out, d_count_, st);
+    launch_chain(k_gf_apply, npart_, 256, smem, s_, nlam_, ncl_, d_a_, d_gcl_, d_gval_, x, Px, dotv, partial, nullptr,
+                 st);
 }
 
 void Engine::iteration(PcpgState *st) {
     op_F(d_w_, d_Fw_, d_w_, d_partial_, st);
-    k_update_lam_g<<<std::min(npart_, 1184), 256, 0, s_>>>(nlam_, d_partial_, npart_, d_w_, d_Fw_, d_lam_, d_g_, st);
+    launch_chain(k_update_lam_g, std::min(npart_, 1184), 256, 0, s_, nlam_, d_partial_, npart_, d_w_, d_Fw_, d_lam_, d_g_,
+                 st);
     op_P(d_g_, d_Pg_, d_alpha_, nullptr, nullptr, st);
     op_M(d_Pg_, d_z_, st);
     op_P(d_z_, d_Pz_, nullptr, d_g_, d_partial_, st);
-    k_update_w<<<std::min(npart_, 1184), 256, 0, s_>>>(nlam_, d_partial_, npart_, d_Pz_, d_w_, st);
-    k_finish_iter<<<1, 256, 0, s_>>>(d_partial_, npart_, st, d_hist_);
+    launch_chain(k_update_w, std::min(npart_, 1184), 256, 0, s_, nlam_, d_partial_, npart_, d_Pz_, d_w_, st, d_hist_,
+                 d_count_ + 1);
 }
 
 int Engine::apply(int op, const double *x, double *y, int nrhs, std::string &err) {
@@ -1085,8 +1075,7 @@ void Engine::init_rhs(const double *f, const double *x_solved) {
         x = d_full_;
     }
     k_bc_rt<<<nsub_, 256, 0, s_>>>(d_subs_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_R_, x, f, d_t_);
-    k_gc<<<cdiv(ngc_total_, 256), 256, 0, s_>>>(ngc_total_, d_gptr_, d_gidx_, d_t_, d_gc_, nullptr);
-    coarse_apply(d_gc_, d_s_, nullptr);
+    coarse_apply(d_t_, d_s_, nullptr);
     k_full_to_b<<<nsub_, 256, 0, s_>>>(d_subs_, x, d_yb_);
     k_correct<<<nsub_, 256, 0, s_>>>(d_subs_, d_cl_, d_V_, d_bcr_, d_s_, d_yb_, nullptr);
     k_rows<<<npart_, 256, 0, s_>>>(nlam_, d_rslot_, d_rsign_, d_yb_, nullptr, d_d_, nullptr, nullptr, nullptr);
@@ -1114,8 +1103,7 @@ void Engine::reconstruct(const double *f, double *u_dev) {
     cudaMemcpyAsync(d_full2_, d_full_, nfull_ * sizeof(double), cudaMemcpyDeviceToDevice, s_);
     ksolve(d_full2_);
     k_bc_rt<<<nsub_, 256, 0, s_>>>(d_subs_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_R_, d_full2_, d_full_, d_t_);
-    k_gc<<<cdiv(ngc_total_, 256), 256, 0, s_>>>(ngc_total_, d_gptr_, d_gidx_, d_t_, d_gc_, nullptr);
-    coarse_apply(d_gc_, d_s_, nullptr);
+    coarse_apply(d_t_, d_s_, nullptr);
     k_sub_bct<<<nsub_, 32, 0, s_>>>(d_subs_, d_cl_, d_bcr_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_s_, d_full_);
     ksolve(d_full_);
     k_add_R<<<nsub_, 256, 0, s_>>>(d_subs_, d_cl_, d_R_, d_H_, d_s_, d_alpha_, d_full_);
@@ -1253,7 +1241,8 @@ int Engine::solve(Problem &p, int nrhs, const double *f_nodal, double *u, htf_st
 int Engine::project_noalloc(const double *x, double *Px, cudaStream_t stream, std::string &err) {
     double *scr = nullptr;
     size_t cap = 0;
-    int rc = noalloc_scratch(&scr, &cap, err);
+    unsigned *counter = nullptr;
+    int rc = noalloc_scratch(&scr, &cap, &counter, err);
     if (rc) return rc;
     const size_t need = 6 * (size_t)nchunks_;
     if (need > cap) {
@@ -1261,11 +1250,13 @@ int Engine::project_noalloc(const double *x, double *Px, cudaStream_t stream, st
               " doubles of scratch, the static array holds " + std::to_string(cap);
         return HTF_EINVAL;
     }
-    k_gft_partial<<<nchunks_, 256, 0, stream>>>(d_chunk_cl_, d_chunk_beg_, d_chunk_end_, d_crow_, d_cval_, x, scr,
-                                                nullptr);
-    k_gf_apply_fused<<<npart_, 256, 12 * ncl_ * sizeof(double), stream>>>(
-        nlam_, ncl_, d_cl_chunk_ptr_, scr, d_invGtG_, d_gcl_, d_gval_, x, nullptr, nullptr, Px,
-        nullptr, nullptr, nullptr);
+    // the coefficient goes over the partials; the counter is set back by both kernels, so that a call after two
+    // that overlapped starts clean
+    const size_t smem = 6 * ncl_ * sizeof(double);
+    k_gft_partial<<<nchunks_, 256, smem, stream>>>(d_chunk_beg_, d_chunk_end_, d_crow_, d_cval_, x, scr, ncl_,
+                                                   d_cl_chunk_ptr_, d_invGtG_, scr, nullptr, counter, nullptr);
+    launch_chain(k_gf_apply, npart_, 256, smem, stream, nlam_, ncl_, scr, d_gcl_, d_gval_, x, Px, nullptr, nullptr,
+                 counter, nullptr);
     return check(cudaGetLastError(), "htf_projection_noalloc launch", err);
 }
 
@@ -1296,7 +1287,7 @@ int Engine::profile(int reps, htf_profile_info *info, std::string &err) {
     double tri = 0.0, vec = 0.0;
     for (auto &h : hs_) { tri += sz * double(h.nb) * (h.nb + 1) / 2; vec += 16.0 * h.nb; }
     info->symv_F_ms = timeit([&] {
-        k_symv_units<double><<<nunits_, SYMV_WARPS * 32, symv_smem_, s_>>>(d_units_, d_subs_, d_F_, d_V_, d_xb_, d_ypart_, d_t_, nullptr);
+        k_symv_units<<<nunits_, SYMV_WARPS * 32, symv_smem_, s_>>>(d_units_, d_subs_, d_F_, d_V_, d_xb_, d_ypart_, d_t_, nullptr);
     });
     info->symv_F_bytes = tri + vec;
     if (implicit_) {              // the two passes over L_bb (its triangle read twice)
@@ -1307,7 +1298,7 @@ int Engine::profile(int reps, htf_profile_info *info, std::string &err) {
         info->symv_S_bytes = 2.0 * tri + 2.0 * vec;
     } else if (d_S_) {
         info->symv_S_ms = timeit([&] {
-            k_symv_units<double><<<nunits_, SYMV_WARPS * 32, symv_smem_, s_>>>(d_units_, d_subs_, d_S_, d_V_, d_xb_, d_ypart_, d_t_,
+            k_symv_units<<<nunits_, SYMV_WARPS * 32, symv_smem_, s_>>>(d_units_, d_subs_, d_S_, d_V_, d_xb_, d_ypart_, d_t_,
                                                                    nullptr);
         });
         info->symv_S_bytes = tri + vec;

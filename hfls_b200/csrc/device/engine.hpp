@@ -12,7 +12,7 @@
 namespace htf {
 
 // static scratch of the allocation-free entry point (noalloc.cu)
-int noalloc_scratch(double **ptr, size_t *cap, std::string &err);
+int noalloc_scratch(double **ptr, size_t *cap, unsigned **counter, std::string &err);
 
 // tensor-core product over blocks of one or more problems (engine_batch.cu)
 int tc_launch(int K, const GemmBlock *blocks, int nblocks, const TcSet *sets, int which, int smem, int *err,
@@ -120,7 +120,7 @@ private:
     int upload_layout(Problem &p, std::string &err);
     // SYMV work-unit schedules (autotune.cu)
     void build_units(const std::vector<int> &tiles, std::vector<SymvUnit> &units, long long &yoff, int &smem,
-                     std::vector<int> &rbptr, std::vector<int> &rbunit);
+                     std::vector<int> &rbptr, std::vector<long long> &rboff);
     int apply_schedule(const std::vector<int> &tiles, bool subs_on_device, std::string &err);
     int alloc_units(std::string &err);
     std::string schedule_key() const;
@@ -134,7 +134,7 @@ private:
     void op_P(const double *x, double *Px, double *alpha_out, const double *dotv, double *partial,
               PcpgState *st);
     void iteration(PcpgState *st);
-    void coarse_apply(const double *gc, double *s, const PcpgState *st);
+    void coarse_apply(const double *t, double *s, const PcpgState *st);   // s = M gc, gc summed from t
     void release(void *p);
     int solve_one(Problem &p, int rhs, double *u_dev, int &iters, double &norm0, double &rel,
                   double &solve_ms, std::string &err);
@@ -194,7 +194,7 @@ private:
     int *d_gptr_ = nullptr, *d_gidx_ = nullptr;
     int *d_gcl_ = nullptr;
     double *d_gval_ = nullptr;
-    int *d_chunk_cl_ = nullptr, *d_chunk_beg_ = nullptr, *d_chunk_end_ = nullptr, *d_crow_ = nullptr,
+    int *d_chunk_beg_ = nullptr, *d_chunk_end_ = nullptr, *d_crow_ = nullptr,
         *d_cl_chunk_ptr_ = nullptr;
     double *d_cval_ = nullptr, *d_invGtG_ = nullptr;
     int nchunks_ = 0;
@@ -207,14 +207,16 @@ private:
     int rhs_cap_ = 0, ndof_ = 0;
     int kernels_per_iter_ = 0;
     long long launches_ = 0;                   // kernels launched by the current solve call
-    SymvUnit *d_units_ = nullptr;              // SYMV work units (+ one V^T x unit per subdomain)
-    int *d_rbptr_ = nullptr, *d_rbunit_ = nullptr;   // per 32-row block of every subdomain: the units covering it
-    long long rbptr_cap_ = 0, rbunit_cap_ = 0;
+    SymvUnit *d_units_ = nullptr;              // SYMV work units, then the V^T x units
+    int *d_rbptr_ = nullptr;                   // per 32-row block of every subdomain: its partial sums in d_ypart_
+    long long *d_rboff_ = nullptr;
+    long long rbptr_cap_ = 0, rboff_cap_ = 0;
     double *d_ypart_ = nullptr;                // partial y sums of the units (scratch)
-    int nunits_ = 0, max_nbp_ = 0;
+    int nunits_ = 0, nvunits_ = 0, max_nbp_ = 0;
     long long units_cap_ = 0, ypart_cap_ = 0;    // unit buffers, sized for every candidate schedule
     int symv_smem_cap_ = 0;
     std::vector<int> schedule_;                  // unit tiles per size bucket in use
+    int unit_cap_ = 1 << 20;                     // and their bound for problems of few tiles
     bool tuned_ = false;
     // batched mixed-precision form
     int bK_ = 0, nblocks_ = 0, bnpart_ = 0, bnpartP_ = 0;
@@ -253,6 +255,7 @@ private:
     double *d_xb_ = nullptr, *d_yb_ = nullptr, *d_t_ = nullptr, *d_gc_ = nullptr, *d_s_ = nullptr;
     double *d_a_ = nullptr, *d_alpha_ = nullptr, *d_partial_ = nullptr, *d_gpart_ = nullptr;
     PcpgState *d_st_ = nullptr;
+    unsigned *d_count_ = nullptr;              // finished CTAs of the kernels whose last CTA does more (zero between launches)
     double *d_hist_ = nullptr;                 // relative residual per iteration of the running solve
     std::vector<std::vector<double>> hist_;    // per load case (first 64) of the last plain solve
     int npart_ = 0;

@@ -197,8 +197,9 @@ typedef struct htf_profile_info {
      * displacement maps, 5 cluster coarse problems, 6 outer coarse problem,
      * 7 SYMV schedule tuning and tensor-core slabs of the batched form              */
     double setup_phase_ms[8];
-    /* SYMV schedule in use: work-unit tiles for subdomains with at most
-     * 8, 16, 32, 64 and more tile rows; tuned = 1 when it came from the
+    /* SYMV schedule in use: largest work unit, in tiles, for subdomains with
+     * at most 8, 16, 32, 64 and more tile rows (problems of few tiles are cut
+     * into smaller units, enough to fill the GPU); tuned = 1 when it came from the
      * autotuner (option autotune) or its cache                             */
     int symv_unit_tiles[5];
     int symv_tuned;
