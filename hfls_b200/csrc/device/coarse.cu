@@ -27,8 +27,8 @@ namespace htf {
 __global__ void k_potrf_diag(const StepDesc *, const SubDev *, double *, int *);
 __global__ void k_trsm_panel(const StepDesc *, int, const SubDev *, double *, const int *);
 __global__ void k_syrk_update(const StepDesc *, int, const SubDev *, double *, const int *);
-__global__ void k_trsm_fwd_multi(const SubDev *, const double *, double *, long long, int, const int *);
-__global__ void k_trsm_bwd_multi(const SubDev *, const double *, double *, long long, int, const int *);
+cudaError_t ksolve_multi_launch(const SubDev *, const int *, int, const double *, double *, long long, int, const int *,
+                                int, int, int *, cudaStream_t);
 __global__ void k_build_Fc(const SubDev *, const double *, const int *, const int *, const double *,
                            const long long *, double *);
 
@@ -314,18 +314,16 @@ static cudaError_t copy_batched(const std::vector<CopyDesc> &c, DevTmp &tmp, cud
 // triangular solves L L^T X = X for the matrices hm / dm; X of matrix c at
 // x + hm[c].nfull_off with leading dimension hm[c].N and ncols[c] columns
 static cudaError_t solve_batched(const std::vector<SubDev> &hm, const SubDev *dm, const double *buf, double *x,
-                                 const std::vector<int> &ncols, DevTmp &tmp, cudaStream_t s) {
-    int chunks = 0;
+                                 const std::vector<int> &ncols, DevTmp &tmp, int *kserr, cudaStream_t s) {
+    int chunks = 0, blocks = 1;
     for (int c : ncols) chunks = std::max(chunks, cdivc(c, 32));
+    for (auto &m : hm) blocks = std::max(blocks, cdivc(m.N, 32));
     if (chunks == 0 || hm.empty()) return cudaSuccess;
     cudaError_t e = cudaSuccess;
     int *d = tmp.get<int>(ncols.size(), e);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d, ncols.data(), ncols.size() * sizeof(int), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return e;
-    const dim3 grid(int(hm.size()), chunks);
-    k_trsm_fwd_multi<<<grid, 256, 0, s>>>(dm, buf, x, 0, 0, d);
-    k_trsm_bwd_multi<<<grid, 256, 0, s>>>(dm, buf, x, 0, 0, d);
-    return cudaGetLastError();
+    return ksolve_multi_launch(dm, nullptr, int(hm.size()), buf, x, 0, 0, d, chunks, blocks, kserr, s);
 }
 
 #define CKC(call)                                                          \
@@ -490,7 +488,7 @@ int Engine::coarse(Problem &p, std::string &err) {
     CKC(cudaMemcpyAsync(dmS, mS.data(), ncl_ * sizeof(SubDev), cudaMemcpyHostToDevice, s_));
     CKC(copy_batched(cp, tmp, s_));
     CKC(chol_batched(mF, dmF, dF, dst, tmp, s_));
-    CKC(solve_batched(mF, dmF, dF, dW, colsW, tmp, s_));               // [Z | Fi]
+    CKC(solve_batched(mF, dmF, dF, dW, colsW, tmp, d_kserr_, s_));               // [Z | Fi]
     std::vector<GemmDesc> gm;
     for (int c = 0; c < ncl_; ++c) {                                     // Sr = Gc^T Z + H H^T
         const int nc = p.clu[c].nlam_c, na = 6 * int(p.clu[c].subs.size());
@@ -505,7 +503,7 @@ int Engine::coarse(Problem &p, std::string &err) {
         CKC(gemm_batched(b, tmp, s_));
     }
     CKC(chol_batched(mS, dmS, dS, dst + ncl_, tmp, s_));
-    CKC(solve_batched(mS, dmS, dS, dSi, colsS, tmp, s_));              // Si = Sr^{-1}
+    CKC(solve_batched(mS, dmS, dS, dSi, colsS, tmp, d_kserr_, s_));              // Si = Sr^{-1}
     gm.clear();
     for (int c = 0; c < ncl_; ++c) {                                     // ZS = Z Si
         const int nc = p.clu[c].nlam_c, na = 6 * int(p.clu[c].subs.size());
@@ -528,11 +526,17 @@ int Engine::coarse(Problem &p, std::string &err) {
     CKC(copy_batched(cp, tmp, s_));
     CKC(gemm_batched(gm, tmp, s_));
     std::vector<int> status(2 * ncl_);
+    int kserr = 0;
+    CKC(cudaMemcpyAsync(&kserr, d_kserr_, sizeof(int), cudaMemcpyDeviceToHost, s_));
     CKC(cudaMemcpyAsync(status.data(), dst, 2 * ncl_ * sizeof(int), cudaMemcpyDeviceToHost, s_));
     std::vector<double> Hflat(36 * (size_t)nsub_);
     for (int d = 0; d < nsub_; ++d) std::memcpy(&Hflat[36 * (size_t)d], Hd_[d].data(), 36 * sizeof(double));
     CKC(cudaMemcpyAsync(d_H_, Hflat.data(), Hflat.size() * sizeof(double), cudaMemcpyHostToDevice, s_));
     CKC(cudaStreamSynchronize(s_));
+    if (kserr) {
+        err = "coarse solve timed out on a barrier";
+        return kserr;
+    }
     for (int c = 0; c < 2 * ncl_; ++c)
         if (status[c]) {
             err = "cluster coarse matrix of cluster " + std::to_string(c % ncl_) + " is not positive definite";

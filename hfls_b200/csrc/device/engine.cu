@@ -501,15 +501,15 @@ int Engine::upload_layout(Problem &p, std::string &err) {
         std::iota(order.begin(), order.end(), 0);
         for (int d = 0; d < nsub_; ++d) blocks[d] = (hs_[d].nr + 31) / 32 + hs_[d].nt;
         std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return blocks[a] > blocks[b]; });
-        ks_blocks_ = blocks[order[0]];
+        ks_blocks_ = max_blocks_ = blocks[order[0]];
         ks_ctas_ = ksolve_ctas(blocks);
         d_ksord_ = alloc<int>(nsub_, err, rc);
         if (rc) return rc;
         CK(cudaMemcpy(d_ksord_, order.data(), nsub_ * sizeof(int), cudaMemcpyHostToDevice));
         int optin = 0;
         CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, opt_.device));
+        CK(ksolve_prepare(optin));
         if (ksolve_smem(ks_blocks_) > size_t(optin)) ks_blocks_ = 0;
-        else CK(ksolve_prepare(optin));
     }
     d_hist_ = alloc<double>(size_t(std::max(opt_.max_iter, 0)) + 1, err, rc);
     if (rc) return rc;

@@ -248,7 +248,8 @@ private:
     // vectors
     int *d_kserr_ = nullptr;                   // time-out flag of the K_reg solves
     int *d_ksord_ = nullptr, ks_ctas_ = 1;     // subdomains largest first, CTAs per cluster
-    int ks_blocks_ = 0;                        // most 32-row blocks of a subdomain (0: too many for ksolve.cu)
+    int max_blocks_ = 0;                       // most 32-row blocks of a subdomain
+    int ks_blocks_ = 0;                        // the same, 0: too many for the one-column kernel
     double *d_f_ = nullptr, *d_full_ = nullptr, *d_full2_ = nullptr;
     double *d_lam_ = nullptr, *d_g_ = nullptr, *d_w_ = nullptr, *d_Fw_ = nullptr, *d_Pg_ = nullptr,
            *d_z_ = nullptr, *d_Pz_ = nullptr, *d_d_ = nullptr, *d_tmp_ = nullptr;

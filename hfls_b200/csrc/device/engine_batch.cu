@@ -65,8 +65,8 @@ __global__ void k_symv_rows_multi(const int2 *, const SubDev *, const double *, 
 __global__ void k_cols_copy(long long, int, const int *, const double *, double *);
 __global__ void k_alpha_cols(int, int, const int *, const double *, double *);
 __global__ void k_axpby(int, double, const double *, double, double *);
-__global__ void k_trsm_fwd_multi(const SubDev *, const double *, double *, long long, int, const int *);
-__global__ void k_trsm_bwd_multi(const SubDev *, const double *, double *, long long, int, const int *);
+cudaError_t ksolve_multi_launch(const SubDev *, const int *, int, const double *, double *, long long, int, const int *,
+                                int, int, int *, cudaStream_t);
 __global__ void k_gather_b(int, const int *, const int *, const double *, const double *, double *,
                            const PcpgState *);
 __global__ void k_full_minus_b(const SubDev *, const double *, double *);
@@ -500,7 +500,7 @@ int Engine::batch_begin(int r0, int kc, std::string &err) {
     CKB(cudaMemcpyAsync(b_fullB_, d_f_ + (size_t)r0 * nfull_, (size_t)kc * nfull_ * sizeof(double),
                         cudaMemcpyDeviceToDevice, s_));
     trsm_multi(b_fullB_, kc);
-    launches_ += 2;
+    launches_ += 1;
     for (int j = 0; j < kc; ++j) {
         init_rhs(d_f_ + (size_t)(r0 + j) * nfull_, b_fullB_ + (size_t)j * nfull_);
         k_col_set<<<npart_, 256, 0, s_>>>(nlam_, K, j, d_d_, b_d_);
@@ -608,7 +608,7 @@ int Engine::batch_finish(htf_stats *stats, double &ms, std::string &err) {
                                        b_alpha_ + (size_t)j * 6 * ncl_, fa);
         k_gather_u<<<cdivb(ndof_, 256), 256, 0, s_>>>(ndof_, d_win_, fa, d_u_ + (size_t)(r.r0 + j) * ndof_);
     }
-    launches_ += 4 + 9 * kc;
+    launches_ += 2 + 9 * kc;
     for (int j = 0; j < kc; ++j) {
         if (stats && r.r0 + j < 64) {
             stats->iterations[r.r0 + j] = r.st[j].it;
@@ -617,6 +617,14 @@ int Engine::batch_finish(htf_stats *stats, double &ms, std::string &err) {
         }
     }
     CKB(cudaGetLastError());
+    int kserr = 0;
+    CKB(cudaMemcpyAsync(&kserr, d_kserr_, sizeof(int), cudaMemcpyDeviceToHost, s_));
+    CKB(cudaStreamSynchronize(s_));
+    if (kserr) {
+        CKB(cudaMemsetAsync(d_kserr_, 0, sizeof(int), s_));
+        err = "K_reg solve timed out on a barrier";
+        return kserr;
+    }
     for (int j = 0; j < r.kc; ++j)
         if (r.conv[j] == 2) { err = "PCPG did not converge within max_iter"; return HTF_ENOCONV; }
     for (int j = 0; j < r.kc; ++j)
@@ -636,16 +644,14 @@ int Engine::batch_finish(htf_stats *stats, double &ms, std::string &err) {
 
 void Engine::trsm_multi(double *v, int nrhs) {
     if (!waves_) {
-        k_trsm_fwd_multi<<<nsub_, 256, 0, s_>>>(d_subs_, d_K_, v, nfull_, nrhs, nullptr);
-        k_trsm_bwd_multi<<<nsub_, 256, 0, s_>>>(d_subs_, d_K_, v, nfull_, nrhs, nullptr);
+        ksolve_multi_launch(d_subs_, d_ksord_, nsub_, d_K_, v, nfull_, nrhs, nullptr, 1, max_blocks_, d_kserr_, s_);
         return;
     }
     // the factor panels were dropped: assemble and factorise each wave again, then solve its subdomains
     for (size_t w = 0; w < fw_.size(); ++w) {
         factor_wave(int(w), false, nullptr);
         const int a = fw_[w].a, nw = fw_[w].b - fw_[w].a;
-        k_trsm_fwd_multi<<<nw, 256, 0, s_>>>(d_subs_ + a, d_K_, v, nfull_, nrhs, nullptr);
-        k_trsm_bwd_multi<<<nw, 256, 0, s_>>>(d_subs_ + a, d_K_, v, nfull_, nrhs, nullptr);
+        ksolve_multi_launch(d_subs_ + a, nullptr, nw, d_K_, v, nfull_, nrhs, nullptr, 1, max_blocks_, d_kserr_, s_);
     }
 }
 

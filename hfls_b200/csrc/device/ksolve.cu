@@ -28,6 +28,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 #include <vector>
 
 #include "device.cuh"
@@ -231,6 +232,9 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) k_ksolve(const SubDev *__res
     cluster_sync_all();
 }
 
+__global__ void k_ksolve_multi(const SubDev *, const int *, const double *, double *, long long, int, const int *, int,
+                               int *);
+
 // shared memory of k_ksolve for subdomains of at most max_blocks 32-row blocks
 size_t ksolve_smem(int max_blocks) {
     return (32 * size_t(max_blocks) + KS_WARPS * 32 * 33) * sizeof(double) + 2 * size_t(max_blocks) * sizeof(uint64_t);
@@ -238,7 +242,9 @@ size_t ksolve_smem(int max_blocks) {
 
 // allows the kernel `optin` bytes (the device's limit, so that contexts of different sizes set the same value)
 cudaError_t ksolve_prepare(int optin) {
-    return cudaFuncSetAttribute(k_ksolve, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    const cudaError_t e = cudaFuncSetAttribute(k_ksolve, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_ksolve_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 48 * 1024);
 }
 
 // CTAs per cluster for subdomains of blocks[i] 32-row blocks: the width with
@@ -282,6 +288,276 @@ cudaError_t ksolve_launch(const SubDev *subs, const int *order, int nsub, const 
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_ksolve, subs, order, K, v, max_blocks, err);
+}
+
+// ---------------------------------------------------------------------------
+// Up to 32 right-hand sides per cluster (blockIdx.y: chunk of 32), the same
+// dataflow with a CTA instead of a warp per 32-row block: X_b = L_bb^{-1}
+// (V_b - sum_k L_bk X_k), then the transposed pass.  Results are exchanged
+// through the vectors in global memory, with a transaction barrier per block
+// in every CTA of the cluster.  The 32 x 32 x 32 products run on the FP64
+// tensor path out of double-buffered shared memory (both tiles column by
+// column with a stride of 36 doubles: no bank conflicts), factor tiles
+// prefetched two ahead into registers, X one ahead when it is known already;
+// warp w owns row tiles 2 (w / 4), + 1 and one column tile, or, with fewer
+// than 25 right-hand sides, a part of the k range of a column tile, the parts
+// added in order.  (Fragments loaded straight from global memory touch eight
+// lines per load and were bound by L1: 4.1 ms where this takes 2.2 for 64 x
+// 2 187 DOFs and 32 right-hand sides; one CTA per subdomain took 7.4.)  Also
+// the coarse problems' solves (plain N x N factors, clusters of one CTA, many
+// chunks).
+//
+// Column j of subdomain d is at v + nfull_off + j * ld (ld = ldv, or N when
+// ldv <= 0); nrhs columns, or ncols[d] when ncols is given.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void dmma_ks(double &d0, double &d1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}
+
+__device__ __forceinline__ bool bar_poll(uint64_t *bar) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(smem_u32(bar))
+        : "memory");
+    return done;
+}
+
+__device__ __forceinline__ bool bar_wait_cluster(uint64_t *bar) {
+    uint32_t done = 0;
+    for (unsigned it = 0; it < TC_WAIT_LIMIT; ++it) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0, %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(smem_u32(bar)), "r"(TC_WAIT_HINT_NS)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+// the CTA's global writes before the last __syncthreads are visible to whoever sees bar complete
+__device__ __forceinline__ void publish(uint64_t *bar, uint32_t ctas) {
+    __threadfence();
+    for (uint32_t c = 0; c < ctas; ++c)
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(map_to_cta(smem_u32(bar), c))
+                     : "memory");
+}
+
+__global__ void __launch_bounds__(256, 2) k_ksolve_multi(const SubDev *__restrict__ subs,
+                                                         const int *__restrict__ order,
+                                                         const double *__restrict__ K, double *v, long long ldv,
+                                                         int nrhs, const int *__restrict__ ncols, int max_blocks,
+                                                         int *__restrict__ err) {
+    constexpr int S = 36;
+    extern __shared__ __align__(16) uint64_t km_bars[];              // forward, then backward barriers
+    __shared__ double Ls[32][33];                                    // diagonal block
+    __shared__ __align__(16) double buf[4 * 32 * S];                 // two (factor, X) tile pairs; then the parts
+    __shared__ double rinv[32];
+    double(*T)[32][34] = reinterpret_cast<double(*)[32][34]>(buf);   // [4][32][34]: partial sums per k part
+    const uint32_t C = cluster_ctas(), rank = cluster_rank();
+    const int si = blockIdx.x / C;
+    const SubDev &sd = subs[order ? order[si] : si];
+    const bool plain = sd.K_bset < 0;
+    const int nr = plain ? sd.N : sd.nr, nI = (nr + 31) / 32, nblk = nI + (plain ? 0 : sd.nt);
+    const long long ld = ldv > 0 ? ldv : sd.N;
+    const int col0 = 32 * blockIdx.y;
+    const int nc = ncols ? min(32, ncols[si] - col0) : nrhs;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, t4 = lane & 3;
+    uint64_t *fwd = km_bars, *bwd = km_bars + max_blocks;
+    for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
+        mbar_init(&fwd[b], 1);
+        mbar_init(&bwd[b], 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    cluster_sync_all();
+    if (nc > 0) {
+        double *x = v + sd.nfull_off + (size_t)col0 * ld;
+        auto start = [&](int b) { return b < nI ? 32 * b : nr + 32 * (b - nI); };
+        auto width = [&](int b) { return b < nI ? min(32, nr - 32 * b) : 32; };
+        // column tiles in use and parts of the k range per column tile
+        const int nct = nc <= 8 ? 1 : nc <= 16 ? 2 : 4, parts = 4 / nct;
+        const int rt = 2 * (warp >> 2), ct = (warp & 3) % nct, part = (warp & 3) / nct;
+        bool ok = true;
+        double d[2][2];
+        // sum over the tiles k = first, first + inc, .. (count of them) of A_k X_k; load_a(r, k, c): element (lane,
+        // column c) of the factor tile; TR: A is its transpose.  Thread (lane, warp) stages columns warp, warp + 8, ..
+        auto sweep = [&](auto tr, int first, int inc, int count, uint64_t *bars, auto &&load_a) {
+            constexpr bool TR = decltype(tr)::value;
+            double la[4], lb[4], xr[4];
+            bool got = false;
+            auto load_l = [&](double (&l)[4], int k) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) l[i] = load_a(k, warp + 8 * i);
+            };
+            auto load_x = [&](int k) {
+                const int w = width(k), r0 = start(k);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int j = warp + 8 * i;
+                    xr[i] = (lane < w && j < nc) ? __ldcg(x + r0 + lane + (size_t)j * ld) : 0.0;
+                }
+            };
+            auto tile = [&](double (&l)[4], int i) {
+                const int k = first + i * inc;
+                double *At = buf + (i & 1) * (2 * 32 * S), *Xt = At + 32 * S;
+                if (!got) {
+                    if (ok) ok = bar_wait_cluster(&bars[k]);
+                    load_x(k);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    At[(warp + 8 * q) * S + lane] = l[q];
+                    Xt[(warp + 8 * q) * S + lane] = xr[q];
+                }
+                got = false;
+                if (i + 1 < count && bar_poll(&bars[k + inc])) {
+                    got = true;
+                    load_x(k + inc);
+                }
+                if (i + 2 < count) load_l(l, k + 2 * inc);
+                __syncthreads();
+                auto mul = [&](int kg) {
+                    const double b = Xt[(8 * ct + g) * S + 4 * kg + t4];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const double a = TR ? At[(8 * (rt + u) + g) * S + 4 * kg + t4]
+                                            : At[(4 * kg + t4) * S + 8 * (rt + u) + g];
+                        dmma_ks(d[u][0], d[u][1], a, b);
+                    }
+                };
+                if (parts == 1) {
+#pragma unroll
+                    for (int kg = 0; kg < 8; ++kg) mul(kg);
+                } else {
+                    for (int kg = part * (8 / parts); kg < (part + 1) * (8 / parts); ++kg) mul(kg);
+                }
+            };
+            d[0][0] = d[0][1] = d[1][0] = d[1][1] = 0.0;
+            if (count > 0) load_l(la, first);
+            if (count > 1) load_l(lb, first + inc);
+            for (int i = 0; i < count; i += 2) {
+                tile(la, i);
+                if (i + 1 < count) tile(lb, i + 1);
+            }
+            __syncthreads();                                          // the tiles are consumed: buf takes the parts
+        };
+        auto load_diag = [&](int b) {
+            const int s = start(b), w = width(b);
+            const double *col = K + kcol(sd, s) + s + lane;
+            const long long lk = kld(sd, s);
+#pragma unroll
+            for (int c = warp; c < 32; c += 8) Ls[lane][c] = (c <= lane && lane < w) ? col[c * lk] : 0.0;
+            __syncthreads();
+            if (threadIdx.x < 32) rinv[lane] = lane < w ? 1.0 / Ls[lane][lane] : 0.0;
+        };
+        // a[q]: row `lane`, column 4 warp + q of V_b (or Y_b) minus the product
+        auto gather = [&](int r0, int w, double (&a)[4]) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                T[part][8 * (rt + u) + g][8 * ct + 2 * t4] = d[u][0];
+                T[part][8 * (rt + u) + g][8 * ct + 2 * t4 + 1] = d[u][1];
+            }
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int j = 4 * warp + q;
+                double s = 0.0;
+                if (j < 8 * nct) {
+                    s = T[0][lane][j];
+                    for (int p = 1; p < parts; ++p) s += T[p][lane][j];
+                }
+                a[q] = (lane < w && j < nc) ? __ldcg(x + r0 + lane + (size_t)j * ld) - s : 0.0;
+            }
+        };
+        auto store = [&](int r0, int w, const double (&a)[4]) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int j = 4 * warp + q;
+                if (lane < w && j < nc) x[r0 + lane + (size_t)j * ld] = a[q];
+            }
+            __syncthreads();
+        };
+        for (int b = int(rank); b < nblk; b += int(C)) {
+            const int r0 = start(b), wb = width(b);
+            load_diag(b);
+            sweep(std::false_type(), 0, 1, b, fwd, [&](int k, int c) {
+                const int s = start(k);
+                return (c < width(k) && lane < wb) ? K[kcol(sd, s) + c * kld(sd, s) + r0 + lane] : 0.0;
+            });
+            double a[4];
+            gather(r0, wb, a);
+            if (4 * warp < nc)
+                for (int p = 0; p < wb; ++p) {
+                    const double rp = rinv[p], lp = Ls[lane][p];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const double y = __shfl_sync(0xffffffffu, a[q] * rp, p);
+                        if (lane == p) a[q] = y;
+                        else if (lane > p) a[q] -= lp * y;
+                    }
+                }
+            store(r0, wb, a);
+            if (threadIdx.x == 0) publish(&fwd[b], C);
+        }
+        // a result overwrites y_b only when every y is known, so when no forward step reads it any more
+        for (int b = int(rank) + (nblk - 1 - int(rank)) / int(C) * int(C); b >= 0 && int(rank) < nblk; b -= int(C)) {
+            const int r0 = start(b), wb = width(b);
+            load_diag(b);
+            if (ok) ok = bar_wait_cluster(&fwd[nblk - 1]);
+            const double *colA = K + kcol(sd, r0) + lane;
+            const long long lk = kld(sd, r0);
+            sweep(std::true_type(), nblk - 1, -1, nblk - 1 - b, bwd, [&](int k, int c) {
+                return (c < wb && lane < width(k)) ? colA[c * lk + start(k)] : 0.0;
+            });
+            double a[4];
+            gather(r0, wb, a);
+            if (4 * warp < nc)
+                for (int p = wb - 1; p >= 0; --p) {
+                    const double rp = rinv[p], lp = Ls[p][lane];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const double y = __shfl_sync(0xffffffffu, a[q] * rp, p);
+                        if (lane == p) a[q] = y;
+                        else if (lane < p) a[q] -= lp * y;
+                    }
+                }
+            store(r0, wb, a);
+            if (threadIdx.x == 0) publish(&bwd[b], C);
+        }
+        if (!ok && lane == 0) atomicExch(err, HTF_ETIMEDOUT);
+    }
+    cluster_sync_all();                                               // no CTA leaves while arrivals are on their way
+}
+
+// V <- K_reg^{-1} V (or the plain factors' inverse) for nsub matrices of at
+// most max_blocks 32-row blocks and `chunks` chunks of 32 columns.  Clusters
+// of up to 8 CTAs while all of them are resident (two per SM).
+cudaError_t ksolve_multi_launch(const SubDev *subs, const int *order, int nsub, const double *K, double *v,
+                                long long ldv, int nrhs, const int *ncols, int chunks, int max_blocks, int *err,
+                                cudaStream_t s) {
+    int ctas = 8;
+    while (ctas > 1 && ((long long)nsub * chunks * ctas > 2 * 148 || ctas > max_blocks)) ctas /= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nsub * ctas, chunks);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = 2 * size_t(max_blocks) * sizeof(uint64_t);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_ksolve_multi, subs, order, K, v, ldv, nrhs, ncols, max_blocks, err);
 }
 
 }  // namespace htf

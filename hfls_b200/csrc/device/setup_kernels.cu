@@ -16,7 +16,6 @@
 //  k_lauum_tiles     F = X^T X = (K_reg^{-1})_bb into packed tiles.
 //  k_build_V/Fc      V = [F Bc_b^T, -R_b] and Fc_d = Bc_b F Bc_b^T
 //                    (Cluster.cpp:150-185).
-//  k_trsm_fwd/bwd_multi  batched multi-RHS triangular solves with the full factor.
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -598,170 +597,6 @@ __global__ void k_build_Fc(const SubDev *__restrict__ subs, const double *__rest
         double v = 0.0;
         for (int e = bce_ptr[sd.bce_off + r]; e < bce_ptr[sd.bce_off + r + 1]; ++e) v += bce_val[e] * V[bce_pos[e]];
         out[idx] = v;
-    }
-}
-
-}  // namespace htf
-
-namespace htf {
-
-// ---------------------------------------------------------------------------
-// batched dense triangular solves with the full factor for up to 32
-// right-hand sides at once (the load cases of a batch): the factor is read
-// once per call instead of once per load case.  Column j of subdomain d lives
-// at v + nfull_off + j*ld (ld = ldv, or N when ldv <= 0).  One CTA of 8 warps
-// per (subdomain, chunk of 32 columns = blockIdx.y); warp w owns columns
-// 4w..4w+3 of the chunk, lane = row inside the current 32-row block.  The
-// chunk has nrhs columns, or min(32, ncols[d] - 32*blockIdx.y) when ncols is
-// given.  The next 32x32 block of L and of X is loaded into registers while
-// the current one is multiplied out of shared memory.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_trsm_fwd_multi(const SubDev *__restrict__ subs,
-                                                        const double *__restrict__ Kbuf, double *__restrict__ v,
-                                                        long long ldv, int nrhs, const int *__restrict__ ncols) {
-    __shared__ double Ls[32][36];
-    __shared__ double Xs[32][36];
-    __shared__ double rinv[32];
-    const SubDev &sd = subs[blockIdx.x];
-    const long long ld = ldv > 0 ? ldv : sd.N;
-    const int c0 = 32 * blockIdx.y;
-    if (ncols) nrhs = min(32, ncols[blockIdx.x] - c0);
-    if (nrhs <= 0) return;
-    double *x = v + sd.nfull_off + (size_t)c0 * ld;
-    const int N = sd.N, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int nblk = (N + 31) / 32;
-    for (int b = 0; b < nblk; ++b) {
-        const int kb = 32 * b, nrow = min(32, N - kb);
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        double d[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-        double lr[4], xr[4];
-        // chunk cb: L rows kb.., columns 32cb.. (all < kb <= N); X rows 32cb..
-        auto load = [&](int cb) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int c = w + 8 * i;
-                lr[i] = (lane < nrow) ? Kbuf[kidx(sd, kb + lane, 32 * cb + c)] : 0.0;
-                xr[i] = (c < nrhs) ? x[(32 * cb + lane) + (size_t)c * ld] : 0.0;
-            }
-        };
-        if (b > 0) load(0);
-        for (int cb = 0; cb < b; ++cb) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                Ls[lane][w + 8 * i] = lr[i];
-                Xs[lane][w + 8 * i] = xr[i];
-            }
-            __syncthreads();
-            if (cb + 1 < b) load(cb + 1);
-            trsm_block_mma<false>(Ls, Xs, w, lane, d);
-            __syncthreads();
-        }
-        if (b > 0) trsm_gather(Xs, d, w, lane, acc);
-        // diagonal block: forward substitution, one shuffle per row
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int c = w + 8 * i;
-            Ls[lane][c] = (lane < nrow && c <= lane) ? Kbuf[kidx(sd, kb + lane, kb + c)] : 0.0;
-        }
-        __syncthreads();
-        if (threadIdx.x < 32) rinv[lane] = (lane < nrow) ? 1.0 / Ls[lane][lane] : 0.0;
-        __syncthreads();
-        double a[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int j = 4 * w + q;
-            a[q] = (lane < nrow && j < nrhs) ? x[(kb + lane) + (size_t)j * ld] - acc[q] : 0.0;
-        }
-        for (int p = 0; p < nrow; ++p) {
-            const double rp = rinv[p], lp = Ls[lane][p];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const double y = __shfl_sync(0xffffffffu, a[q] * rp, p);
-                if (lane == p) a[q] = y;
-                else if (lane > p) a[q] -= lp * y;
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int j = 4 * w + q;
-            if (lane < nrow && j < nrhs) x[(kb + lane) + (size_t)j * ld] = a[q];
-        }
-        __syncthreads();
-    }
-}
-
-__global__ void __launch_bounds__(256) k_trsm_bwd_multi(const SubDev *__restrict__ subs,
-                                                        const double *__restrict__ Kbuf, double *__restrict__ v,
-                                                        long long ldv, int nrhs, const int *__restrict__ ncols) {
-    __shared__ double Ls[32][36];
-    __shared__ double Xs[32][36];
-    __shared__ double rinv[32];
-    const SubDev &sd = subs[blockIdx.x];
-    const long long ld = ldv > 0 ? ldv : sd.N;
-    const int c0 = 32 * blockIdx.y;
-    if (ncols) nrhs = min(32, ncols[blockIdx.x] - c0);
-    if (nrhs <= 0) return;
-    double *x = v + sd.nfull_off + (size_t)c0 * ld;
-    const int N = sd.N, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int nblk = (N + 31) / 32;
-    for (int b = nblk - 1; b >= 0; --b) {
-        const int kb = 32 * b, nrow = min(32, N - kb);
-        double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        double d[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-        double lr[4], xr[4];
-        // chunk cb > b: rows c = 32cb + lane of L's columns kb.. (L^T), X rows c
-        auto load = [&](int cb) {
-            const int c = 32 * cb + lane;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = w + 8 * i;
-                lr[i] = (c < N && r < nrow) ? Kbuf[kidx(sd, c, kb + r)] : 0.0;
-                xr[i] = (c < N && r < nrhs) ? x[c + (size_t)r * ld] : 0.0;
-            }
-        };
-        if (b + 1 < nblk) load(b + 1);
-        for (int cb = b + 1; cb < nblk; ++cb) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                Ls[lane][w + 8 * i] = lr[i];          // Ls[c][r] = L[32cb + c][kb + r]
-                Xs[lane][w + 8 * i] = xr[i];
-            }
-            __syncthreads();
-            if (cb + 1 < nblk) load(cb + 1);
-            trsm_block_mma<true>(Ls, Xs, w, lane, d);
-            __syncthreads();
-        }
-        if (b + 1 < nblk) trsm_gather(Xs, d, w, lane, acc);
-        // diagonal block: Ls[p][r] = L[kb + p][kb + r], r <= p; back substitution with L^T
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = w + 8 * i;
-            Ls[lane][r] = (lane < nrow && r <= lane) ? Kbuf[kidx(sd, kb + lane, kb + r)] : 0.0;
-        }
-        __syncthreads();
-        if (threadIdx.x < 32) rinv[lane] = (lane < nrow) ? 1.0 / Ls[lane][lane] : 0.0;
-        __syncthreads();
-        double a[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int j = 4 * w + q;
-            a[q] = (lane < nrow && j < nrhs) ? x[(kb + lane) + (size_t)j * ld] - acc[q] : 0.0;
-        }
-        for (int p = nrow - 1; p >= 0; --p) {
-            const double rp = rinv[p], lp = Ls[p][lane];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const double y = __shfl_sync(0xffffffffu, a[q] * rp, p);
-                if (lane == p) a[q] = y;
-                else if (lane < p) a[q] -= lp * y;
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int j = 4 * w + q;
-            if (lane < nrow && j < nrhs) x[(kb + lane) + (size_t)j * ld] = a[q];
-        }
-        __syncthreads();
     }
 }
 
