@@ -26,7 +26,7 @@ CU_SOURCES = ["device/setup_kernels.cu", "device/pcpg_kernels.cu", "device/engin
               "device/autotune.cu", "device/kernel_fix.cu", "device/frontend.cu", "device/ksolve.cu"]
 CPP_SOURCES = ["host/mesh.cpp", "host/problem.cpp", "host/vtk.cpp", "host/dump.cpp", "capi.cpp", "server.cpp",
                "cxx/surface.cpp"]
-HEADERS = ["device/device.cuh", "device/mbar.cuh", "device/engine.hpp", "host/problem.hpp"]
+HEADERS = ["device/device.cuh", "device/mbar.cuh", "device/arena.hpp", "device/engine.hpp", "host/problem.hpp"]
 
 INC = ["-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",

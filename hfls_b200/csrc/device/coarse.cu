@@ -205,14 +205,10 @@ __global__ void k_copy_batched(const CopyDesc *__restrict__ desc) {
 namespace {
 
 struct DevTmp {                        // device scratch freed when the coarse set-up ends
-    std::vector<void *> p;
-    ~DevTmp() {
-        for (void *q : p) cudaFree(q);
-    }
+    DevArena mem;
     template <typename T> T *get(size_t n, cudaError_t &e) {
         void *q = nullptr;
-        if (e == cudaSuccess) e = cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T));
-        if (e == cudaSuccess) p.push_back(q);
+        if (e == cudaSuccess) e = mem.get(&q, n * sizeof(T));
         return static_cast<T *>(q);
     }
 };

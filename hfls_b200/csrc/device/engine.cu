@@ -182,14 +182,7 @@ __global__ void k_gather_u(int ndof, const int *__restrict__ win, const double *
 
 // ---------------------------------------------------------------------------
 // free one of the engine's buffers before the end of its life
-void Engine::release(void *p) {
-    for (size_t i = 0; i < bufs_.size(); ++i)
-        if (bufs_[i].p == p) {
-            cudaFree(p);
-            bufs_.erase(bufs_.begin() + i);
-            return;
-        }
-}
+void Engine::release(void *p) { mem_.release(p); }
 
 // s = M gc for every cluster (M = [Ac^{-1}] restricted, packed symmetric tiles), gc = the sums of t per coarse row
 void Engine::coarse_apply(const double *t, double *s, const PcpgState *st) {
@@ -204,15 +197,11 @@ Engine::~Engine() {
     if (bgraph_) cudaGraphExecDestroy(bgraph_);
     if (run_e0_) cudaEventDestroy(run_e0_);
     if (run_e1_) cudaEventDestroy(run_e1_);
-    for (auto &b : bufs_) cudaFree(b.p);
+    mem_.clear();
     if (own_s_) cudaStreamDestroy(own_s_);
 }
 
-size_t Engine::device_bytes() const {
-    size_t t = 0;
-    for (auto &b : bufs_) t += b.bytes;
-    return t;
-}
+size_t Engine::device_bytes() const { return mem_.bytes(); }
 
 int Engine::check(cudaError_t e, const char *what, std::string &err, const char *file, int line) {
     if (e == cudaSuccess) return HTF_OK;

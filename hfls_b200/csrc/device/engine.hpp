@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../host/problem.hpp"
+#include "arena.hpp"
 #include "device.cuh"
 
 namespace htf {
@@ -43,11 +44,6 @@ struct BatchRun {
 // replacements.
 constexpr int MIXED_STALL_LIMIT = 10;
 constexpr int MIXED_STALL_ITERATIONS = 500;
-
-struct DevBuf {
-    void *p = nullptr;
-    size_t bytes = 0;
-};
 
 class Engine {
 public:
@@ -142,7 +138,7 @@ private:
 
     Options opt_;
     cudaStream_t s_ = nullptr, own_s_ = nullptr;
-    std::vector<DevBuf> bufs_;
+    DevArena mem_;
     int nsub_ = 0, ncl_ = 0, nlam_ = 0, nslots_ = 0, nfull_ = 0, ngc_total_ = 0, nt_total_ = 0;
     long long ntiles_ = 0;
     std::vector<SubDev> hs_;
@@ -280,13 +276,12 @@ template <typename T> T *Engine::alloc(size_t n, std::string &err, int &rc) {
     if (rc) return nullptr;
     void *p = nullptr;
     const size_t bytes = (n > 0 ? n : 1) * sizeof(T);
-    const cudaError_t e = cudaMalloc(&p, bytes);
+    const cudaError_t e = mem_.get(&p, bytes);
     if (e != cudaSuccess) {
         rc = check(e, "cudaMalloc", err);
         err += " (" + std::to_string(bytes) + " bytes)";
         return nullptr;
     }
-    bufs_.push_back({p, bytes});
     return static_cast<T *>(p);
 }
 

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "../host/problem.hpp"
+#include "arena.hpp"
 
 namespace htf {
 namespace {
@@ -321,14 +322,10 @@ __global__ void k_fe_ent_fill(long long nl, const int *__restrict__ rsub, const 
 
 // device scratch released at scope exit
 struct FeMem {
-    std::vector<void *> p;
-    ~FeMem() {
-        for (void *q : p) cudaFree(q);
-    }
+    DevArena mem;
     template <typename T> T *get(size_t n, cudaError_t &e) {
         void *q = nullptr;
-        if (e == cudaSuccess) e = cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T));
-        if (e == cudaSuccess) p.push_back(q);
+        if (e == cudaSuccess) e = mem.get(&q, n * sizeof(T));
         return static_cast<T *>(q);
     }
 };

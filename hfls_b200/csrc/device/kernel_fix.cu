@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "../host/problem.hpp"
+#include "arena.hpp"
 
 namespace htf {
 
@@ -174,9 +175,12 @@ __global__ void __launch_bounds__(KF_THREADS) k_kernel_fix(const double *__restr
     }
 }
 
-template <typename T> int upload(T *&dst, const std::vector<T> &src, std::string &err, size_t n_alloc = 0) {
+template <typename T>
+int upload(DevArena &mem, T *&dst, const std::vector<T> &src, std::string &err, size_t n_alloc = 0) {
     const size_t bytes = std::max<size_t>(std::max(src.size(), n_alloc), 1) * sizeof(T);
-    cudaError_t e = cudaMalloc(&dst, bytes);
+    void *q = nullptr;
+    cudaError_t e = mem.get(&q, bytes);
+    dst = static_cast<T *>(q);
     if (e == cudaSuccess && !src.empty()) e = cudaMemcpy(dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         err = std::string("kernel detection upload: ") + cudaGetErrorString(e);
@@ -217,27 +221,28 @@ int kernels_fix_on_device(const Mesh &m, std::vector<Subdomain> &subs, int devic
         r_off[d + 1] = r_off[d] + 6LL * s.n;
         n_off[d + 1] = n_off[d] + 6LL * s.nb;
     }
+    DevArena mem;
     double *dc = nullptr, *dR = nullptr, *dN = nullptr, *dW = nullptr;
     int *dnp = nullptr, *dn = nullptr, *dbp = nullptr, *db = nullptr, *dpiv = nullptr, *dfix = nullptr;
     long long *dro = nullptr, *dno = nullptr;
-    int rc = upload(dc, m.coords, err);
-    if (!rc) rc = upload(dnp, node_ptr, err);
-    if (!rc) rc = upload(dn, nodes, err);
-    if (!rc) rc = upload(dbp, b_ptr, err);
-    if (!rc) rc = upload(db, bidx, err);
-    if (!rc) rc = upload(dro, r_off, err);
-    if (!rc) rc = upload(dno, n_off, err);
-    if (!rc) rc = upload(dR, std::vector<double>(), err, size_t(r_off[ns]));
-    if (!rc) rc = upload(dN, std::vector<double>(), err, size_t(n_off[ns]) + 1);
-    if (!rc) rc = upload(dpiv, std::vector<int>(), err, size_t(n_off[ns] / 6) + 1);
-    if (!rc) rc = upload(dfix, std::vector<int>(), err, size_t(6 * ns));
+    int rc = upload(mem, dc, m.coords, err);
+    if (!rc) rc = upload(mem, dnp, node_ptr, err);
+    if (!rc) rc = upload(mem, dn, nodes, err);
+    if (!rc) rc = upload(mem, dbp, b_ptr, err);
+    if (!rc) rc = upload(mem, db, bidx, err);
+    if (!rc) rc = upload(mem, dro, r_off, err);
+    if (!rc) rc = upload(mem, dno, n_off, err);
+    if (!rc) rc = upload(mem, dR, std::vector<double>(), err, size_t(r_off[ns]));
+    if (!rc) rc = upload(mem, dN, std::vector<double>(), err, size_t(n_off[ns]) + 1);
+    if (!rc) rc = upload(mem, dpiv, std::vector<int>(), err, size_t(n_off[ns] / 6) + 1);
+    if (!rc) rc = upload(mem, dfix, std::vector<int>(), err, size_t(6 * ns));
     std::vector<double> R(r_off[ns]);
     std::vector<int> fix(6 * ns);
     int smem = max_n * int(sizeof(double)), optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     if (!rc && smem > optin - 4096) {          // too large for shared memory: global scratch
         smem = 0;
-        rc = upload(dW, std::vector<double>(), err, size_t(r_off[ns] / 6) + 1);
+        rc = upload(mem, dW, std::vector<double>(), err, size_t(r_off[ns] / 6) + 1);
     } else if (!rc && smem > 0) {
         // static + dynamic shared memory above 48 KB needs the opt-in; set it
         // for every size (the static arrays count against the same 48 KB)
@@ -266,9 +271,7 @@ int kernels_fix_on_device(const Mesh &m, std::vector<Subdomain> &subs, int devic
             rc = HTF_ECUDA;
         }
     }
-    for (void *p : {(void *)dc, (void *)dR, (void *)dN, (void *)dW, (void *)dnp, (void *)dn, (void *)dbp, (void *)db,
-                    (void *)dpiv, (void *)dfix, (void *)dro, (void *)dno})
-        if (p) cudaFree(p);
+    mem.clear();
     if (rc) return rc;
     if (timing_ms) {
         timing_ms[0] = std::chrono::duration<double, std::milli>(t1 - t0).count();
