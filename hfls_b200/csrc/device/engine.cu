@@ -198,10 +198,11 @@ Engine::~Engine() {
     if (run_e0_) cudaEventDestroy(run_e0_);
     if (run_e1_) cudaEventDestroy(run_e1_);
     mem_.clear();
+    bmem_.clear();
     if (own_s_) cudaStreamDestroy(own_s_);
 }
 
-size_t Engine::device_bytes() const { return mem_.bytes(); }
+size_t Engine::device_bytes() const { return mem_.bytes() + bmem_.bytes(); }
 
 int Engine::check(cudaError_t e, const char *what, std::string &err, const char *file, int line) {
     if (e == cudaSuccess) return HTF_OK;
@@ -1197,17 +1198,33 @@ int Engine::solve(Problem &p, int nrhs, const double *f_nodal, double *u, htf_st
     k_build_f<<<cdiv(nfull_, 256), 256, 0, s_>>>(nfull_, ndof_, nrhs, d_fbody_, d_own_, f_nodal ? d_fn_ : nullptr, d_f_);
     CK(cudaGetLastError());
     double total_ms = 0.0;
-    for (int r = 0; r < nrhs; ++r) {
+    for (int r = 0; r < nrhs;) {
+        // the remaining load cases together, or one (the last few, or a problem the batched form does not take)
+        const int kc = ready_batch64(nrhs - r) ? std::min(nrhs - r, bK_) : 1;
         int it = 0;
         double n0 = 0, rel = 0, ms = 0;
-        rc = solve_one(p, r, d_u_ + (size_t)r * ndof_, it, n0, rel, ms, err);
+        if (kc > 1) rc = solve_chunk64(r, kc, ms, err);
+        else rc = solve_one(p, r, d_u_ + (size_t)r * ndof_, it, n0, rel, ms, err);
         total_ms += ms;
-        if (stats && r < 64) { stats->iterations[r] = it; stats->norm_gPz0[r] = n0; stats->final_rel[r] = rel; }
-        if (rc) return rc;
-        if (it >= opt_.max_iter && !(rel < opt_.eps_iter)) {
-            if (stats) stats->solve_ms = total_ms;
-            err = "PCPG did not converge within max_iter";
-            return HTF_ENOCONV;
+        if (kc > 1 && rc) return rc;
+        for (int j = 0; j < kc; ++j, ++r) {
+            if (kc > 1) {
+                const PcpgState &st = run_.st[j];
+                it = st.it;
+                n0 = st.norm0;
+                rel = st.rel;
+                if (st.done == 2) {
+                    err = "PCPG breakdown (w'Fw <= 0 or non-finite)";
+                    rc = HTF_EBREAKDOWN;
+                }
+            }
+            if (stats && r < 64) { stats->iterations[r] = it; stats->norm_gPz0[r] = n0; stats->final_rel[r] = rel; }
+            if (rc) return rc;
+            if (it >= opt_.max_iter && !(rel < opt_.eps_iter)) {
+                if (stats) stats->solve_ms = total_ms;
+                err = "PCPG did not converge within max_iter";
+                return HTF_ENOCONV;
+            }
         }
     }
     if (u) CK(cudaMemcpyAsync(u, d_u_, (size_t)ndof_ * nrhs * sizeof(double), cudaMemcpyDeviceToHost, s_));

@@ -59,6 +59,7 @@ public:
     int history(int rhs, double *out, int cap, std::string &err) const;
     // batched mixed-precision form (engine_batch.cu)
     int setup_batch(int K, std::string &err);
+    int alloc_batch(int K, std::string &err);
     int plan_slabs(int K, std::string &err);       // tensor-core blocks and slab buffers
     int solve_batch(Problem &p, int nrhs, const double *f_nodal, double *u, htf_stats *stats, std::string &err);
     int apply_batch(int op, const double *x, double *y, int nrhs, std::string &err);
@@ -112,6 +113,15 @@ private:
     void op_M_batch(const double *x, double *z);
     void op_P_batch(const double *x, double *Px, double *alpha_out, const double *dotv, double *partial);
     void iteration_batch();
+    int batch_rhs(int r0, int kc, std::string &err);
+    int batch_reconstruct(int r0, int kc, std::string &err);
+    void symv_multi(const double *tiles, const double *scoarse);
+    // FP64 form, several load cases at once (engine_batch.cu)
+    bool ready_batch64(int nrhs);
+    void op_F_batch64(const double *w, double *Fw, const double *dotv, double *partial);
+    void op_M_batch64(const double *x, double *z);
+    void iteration_batch64();
+    int solve_chunk64(int r0, int kc, double &ms, std::string &err);
     int check(cudaError_t e, const char *what, std::string &err, const char *file = nullptr, int line = 0);
     int upload_layout(Problem &p, std::string &err);
     // SYMV work-unit schedules (autotune.cu)
@@ -138,7 +148,8 @@ private:
 
     Options opt_;
     cudaStream_t s_ = nullptr, own_s_ = nullptr;
-    DevArena mem_;
+    DevArena mem_, bmem_;                      // buffers; batch vectors of the FP64 form
+    DevArena *into_ = &mem_;                   // where alloc puts the next buffer
     int nsub_ = 0, ncl_ = 0, nlam_ = 0, nslots_ = 0, nfull_ = 0, ngc_total_ = 0, nt_total_ = 0;
     long long ntiles_ = 0;
     std::vector<SubDev> hs_;
@@ -237,6 +248,8 @@ private:
     void *d_rowblk_ = nullptr;                         // (subdomain, 32-row block) list of the FP64 multi-RHS SYMV
     int nrowblk_ = 0;
     PcpgState *b_st_ = nullptr;
+    bool b64_off_ = false;                     // FP64 form: the batched form was found not to apply
+    double *b_hist_ = nullptr;                 // FP64 form: relative residuals, [iteration][column]
     cudaGraphExec_t bgraph_ = nullptr;
     int bkernels_per_iter_ = 0;
     int tc_smem_ = 0, vt_nch_ = 1, vt_qn_ = 64;
@@ -276,7 +289,7 @@ template <typename T> T *Engine::alloc(size_t n, std::string &err, int &rc) {
     if (rc) return nullptr;
     void *p = nullptr;
     const size_t bytes = (n > 0 ? n : 1) * sizeof(T);
-    const cudaError_t e = mem_.get(&p, bytes);
+    const cudaError_t e = into_->get(&p, bytes);
     if (e != cudaSuccess) {
         rc = check(e, "cudaMalloc", err);
         err += " (" + std::to_string(bytes) + " bytes)";

@@ -55,7 +55,9 @@ __global__ void k_update_lam_g_multi(int, int, const double *, const double *, c
                                      double *, PcpgState *);
 __global__ void k_dot_multi(int, int, const double *, const double *, double *);
 __global__ void k_update_w_multi(int, int, const double *, const double *, double *, const PcpgState *);
-__global__ void k_finish_multi(int, const double *, const double *, PcpgState *);
+__global__ void k_finish_multi(int, const double *, const double *, PcpgState *, double *);
+template <int K>
+__global__ void k_msym_rows_multi(const int2 *, const ClusterDev *, const double *, const double *, double *);
 __global__ void k_col_get(int, int, int, const double *, double *);
 __global__ void k_col_set(int, int, int, const double *, double *);
 __global__ void k_build_f(int, int, int, const double *, const int *, const double *, double *);
@@ -185,6 +187,17 @@ int Engine::setup_batch(int K, std::string &err) {
         CKB(cudaFuncSetAttribute(k_tc_gemm<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem_));
     else
         CKB(cudaFuncSetAttribute(k_tc_gemm<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem_));
+    if ((rc = alloc_batch(K, err))) return rc;
+    bK_ = K;
+    const TcSet ts = tc_set();
+    CKB(cudaMemcpyAsync(d_tcset_, &ts, sizeof(TcSet), cudaMemcpyHostToDevice, s_));
+    CKB(cudaStreamSynchronize(s_));
+    return HTF_OK;
+}
+
+// vectors of a batch of K load cases (mixed and FP64 form)
+int Engine::alloc_batch(int K, std::string &err) {
+    int rc = HTF_OK;
     // batch vectors
     const size_t nl = (size_t)nlam_ * K;
     int ntot = 0;
@@ -224,12 +237,7 @@ int Engine::setup_batch(int K, std::string &err) {
     b_fullA_ = alloc<double>((size_t)nfull_ * K, err, rc);
     b_fullB_ = alloc<double>((size_t)nfull_ * K, err, rc);
     b_srec_ = alloc<double>((size_t)ngc_total_ * K, err, rc);
-    if (rc) return rc;
-    bK_ = K;
-    const TcSet ts = tc_set();
-    CKB(cudaMemcpyAsync(d_tcset_, &ts, sizeof(TcSet), cudaMemcpyHostToDevice, s_));
-    CKB(cudaStreamSynchronize(s_));
-    return HTF_OK;
+    return rc;
 }
 
 // the coarse correction of the F product runs after it (k_correct_multi in
@@ -291,6 +299,11 @@ void Engine::coarse_batch() {
     }
     k_gc_multi<<<cdivb((long long)ngc_total_ * K, 256), 256, 0, s_>>>(ngc_total_, K, vt_nch_, d_gptr_, d_gidx_, b_t_,
                                                                       b_gc_);
+    if (!d_M_) {                                    // FP64 form: packed symmetric tiles
+        if (K == 32) k_msym_rows_multi<32><<<nmt_, 256, 0, s_>>>(d_mt_, d_cl_, d_MT_, b_gc_, b_s_);
+        else k_msym_rows_multi<16><<<nmt_, 256, 0, s_>>>(d_mt_, d_cl_, d_MT_, b_gc_, b_s_);
+        return;
+    }
     if (K == 32) k_coarse_multi<32><<<dim3(ncl_, cdivb(maxg, 32)), 128, 0, s_>>>(d_cl_, d_M_, b_gc_, b_s_);
     else k_coarse_multi<16><<<dim3(ncl_, cdivb(maxg, 32)), 128, 0, s_>>>(d_cl_, d_M_, b_gc_, b_s_);
 }
@@ -351,7 +364,7 @@ void Engine::iter_c() {
     op_P_batch(b_z_, b_Pz_, nullptr, b_g_, b_part_);
     k_colsum<<<K, 256, 0, s_>>>(b_part_, bnpart_, K, b_gPz_);
     k_update_w_multi<<<nk, 256, 0, s_>>>(nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_);
-    k_finish_multi<<<1, 32, 0, s_>>>(K, b_wFw_, b_gPz_, b_st_);
+    k_finish_multi<<<1, 32, 0, s_>>>(K, b_wFw_, b_gPz_, b_st_, nullptr);
 }
 
 void Engine::iteration_batch() {
@@ -396,6 +409,15 @@ int Engine::batch_loads(int nrhs, const double *f_nodal, std::string &err) {
     return HTF_OK;
 }
 
+// y_b = A_d x_b (packed FP64 tiles) [- V_d s_d] for the K columns of the batch vector b_xb_
+void Engine::symv_multi(const double *tiles, const double *scoarse) {
+    const int2 *rb = static_cast<const int2 *>(d_rowblk_);
+    if (bK_ == 32)
+        k_symv_rows_multi<32><<<nrowblk_, 256, 0, s_>>>(rb, d_subs_, tiles, b_xb_, b_yb_, d_cl_, d_V_, d_bcr_, scoarse);
+    else
+        k_symv_rows_multi<16><<<nrowblk_, 256, 0, s_>>>(rb, d_subs_, tiles, b_xb_, b_yb_, d_cl_, d_V_, d_bcr_, scoarse);
+}
+
 // FP64 residuals of the load cases j with sel[j] (Cluster.cpp:1398-1412 from
 // the current lambda), all in one pass over the FP64 tiles: g = F lambda - d,
 // P g (alpha), z = M P g, P z and g'Pz.  They replace the batch residual
@@ -407,19 +429,11 @@ int Engine::fp64_residual_batch(const std::vector<int> &sel, const std::vector<i
     const auto t_start = std::chrono::steady_clock::now();
     const int K = bK_;
     const long long nk = (long long)nlam_ * K;
-    auto symv = [&](const double *tiles, const double *scoarse) {
-        if (K == 32)
-            k_symv_rows_multi<32><<<nrowblk_, 256, 0, s_>>>(static_cast<const int2 *>(d_rowblk_), d_subs_, tiles, b_xb_,
-                                                           b_yb_, d_cl_, d_V_, d_bcr_, scoarse);
-        else
-            k_symv_rows_multi<16><<<nrowblk_, 256, 0, s_>>>(static_cast<const int2 *>(d_rowblk_), d_subs_, tiles, b_xb_,
-                                                           b_yb_, d_cl_, d_V_, d_bcr_, scoarse);
-    };
     // g = F lambda - d
     k_gather_multi<<<nslots_ / 32, 256, 0, s_>>>(nslots_, K, d_slot_ptr_, d_slot_ent_, b_lam_, nullptr, b_xb_, nullptr,
                                                  nullptr, 0.f);
     coarse_batch();
-    symv(d_F_, b_s_);
+    symv_multi(d_F_, b_s_);
     k_rows_multi<<<bnpart_, 256, 0, s_>>>(nlam_, K, d_rslot_, d_rsign_, b_yb_, nullptr, b_tmp_, nullptr, nullptr);
     k_axpby<<<cdivb(nk, 256), 256, 0, s_>>>(int(nk), -1.0, b_d_, 1.0, b_tmp_);
     op_P_batch(b_tmp_, b_Pg_, b_alpha2_, nullptr, nullptr);
@@ -427,7 +441,7 @@ int Engine::fp64_residual_batch(const std::vector<int> &sel, const std::vector<i
     if (d_S_) {
         k_gather_multi<<<nslots_ / 32, 256, 0, s_>>>(nslots_, K, d_slot_ptr_, d_slot_ent_, b_Pg_, d_weight_, b_xb_,
                                                      nullptr, nullptr, 0.f);
-        symv(d_S_, nullptr);
+        symv_multi(d_S_, nullptr);
         k_rows_multi<<<bnpart_, 256, 0, s_>>>(nlam_, K, d_rslot_, d_rsign_, b_yb_, d_weight_, b_z_, nullptr, nullptr);
     } else {
         op_M_batch(b_Pg_, b_z_);      // S_i only as tensor-core slabs: the tensor-core product
@@ -476,6 +490,25 @@ int Engine::fp64_residual_batch(const std::vector<int> &sel, const std::vector<i
     return HTF_OK;
 }
 
+// d and lambda0 of kc load cases from r0 on into the batch vectors (other columns zero)
+int Engine::batch_rhs(int r0, int kc, std::string &err) {
+    const int K = bK_;
+    CKB(cudaMemsetAsync(b_lam_, 0, (size_t)nlam_ * K * sizeof(double), s_));
+    CKB(cudaMemsetAsync(b_d_, 0, (size_t)nlam_ * K * sizeof(double), s_));
+    // K_reg^{-1} f for the whole chunk: the factor is read once
+    CKB(cudaMemcpyAsync(b_fullB_, d_f_ + (size_t)r0 * nfull_, (size_t)kc * nfull_ * sizeof(double),
+                        cudaMemcpyDeviceToDevice, s_));
+    trsm_multi(b_fullB_, kc);
+    launches_ += 1;
+    for (int j = 0; j < kc; ++j) {
+        init_rhs(d_f_ + (size_t)(r0 + j) * nfull_, b_fullB_ + (size_t)j * nfull_);
+        k_col_set<<<npart_, 256, 0, s_>>>(nlam_, K, j, d_d_, b_d_);
+        k_col_set<<<npart_, 256, 0, s_>>>(nlam_, K, j, d_lam_, b_lam_);
+        launches_ += 25;
+    }
+    return HTF_OK;
+}
+
 int Engine::batch_begin(int r0, int kc, std::string &err) {
     const int K = bK_;
     if (kc < 1 || kc > K) { err = "bad load-case chunk"; return HTF_EINVAL; }
@@ -493,23 +526,11 @@ int Engine::batch_begin(int r0, int kc, std::string &err) {
     r.best_it.assign(K, 0);
     r.stall.assign(K, 0);
     r.conv.assign(K, 0);
-    CKB(cudaMemsetAsync(b_lam_, 0, (size_t)nlam_ * K * sizeof(double), s_));
-    CKB(cudaMemsetAsync(b_d_, 0, (size_t)nlam_ * K * sizeof(double), s_));
     CKB(cudaMemsetAsync(d_tcerr_, 0, sizeof(int), s_));
-    // K_reg^{-1} f for the whole chunk: the factor is read once
-    CKB(cudaMemcpyAsync(b_fullB_, d_f_ + (size_t)r0 * nfull_, (size_t)kc * nfull_ * sizeof(double),
-                        cudaMemcpyDeviceToDevice, s_));
-    trsm_multi(b_fullB_, kc);
-    launches_ += 1;
-    for (int j = 0; j < kc; ++j) {
-        init_rhs(d_f_ + (size_t)(r0 + j) * nfull_, b_fullB_ + (size_t)j * nfull_);
-        k_col_set<<<npart_, 256, 0, s_>>>(nlam_, K, j, d_d_, b_d_);
-        k_col_set<<<npart_, 256, 0, s_>>>(nlam_, K, j, d_lam_, b_lam_);
-        launches_ += 25;
-    }
+    int rc = batch_rhs(r0, kc, err);
+    if (rc) return rc;
     CKB(cudaEventRecord(run_e0_, s_));
     for (int j = 0; j < K; ++j) r.st[j].done = 1;
-    int rc;
     std::vector<int> sel(K, 0), reset(K, 0);
     for (int j = 0; j < kc; ++j) {
         r.st[j].eps = opt_.eps_iter * opt_.mixed_eps_factor;
@@ -566,21 +587,14 @@ int Engine::batch_check(bool &all_done, std::string &err) {
     return HTF_OK;
 }
 
-// displacements of the chunk's load cases into d_u_; per-load-case stats
-int Engine::batch_finish(htf_stats *stats, double &ms, std::string &err) {
-    BatchRun &r = run_;
+// displacements of kc load cases from r0 on: lambda in b_lam_, alpha in b_alpha_ (column-major)
+int Engine::batch_reconstruct(int r0, int kc, std::string &err) {
     const int K = bK_;
-    CKB(cudaEventRecord(run_e1_, s_));
-    CKB(cudaEventSynchronize(run_e1_));
-    float fms = 0.f;
-    cudaEventElapsedTime(&fms, run_e0_, run_e1_);
-    ms = fms;
     // u_j = K_HT^+(f_j - Bf^T lambda_j) - Rf alpha_j (Cluster.cpp:1648-1678) for the whole
     // chunk, with the two K_reg^{-1} solves of every load case done at once
-    const int kc = r.kc;
     int maxg = 0;
     for (auto &c : hc_) maxg = std::max(maxg, c.ngc);
-    CKB(cudaMemcpyAsync(b_fullA_, d_f_ + (size_t)r.r0 * nfull_, (size_t)kc * nfull_ * sizeof(double),
+    CKB(cudaMemcpyAsync(b_fullA_, d_f_ + (size_t)r0 * nfull_, (size_t)kc * nfull_ * sizeof(double),
                         cudaMemcpyDeviceToDevice, s_));
     for (int j = 0; j < kc; ++j) {
         double *fa = b_fullA_ + (size_t)j * nfull_;
@@ -595,9 +609,13 @@ int Engine::batch_finish(htf_stats *stats, double &ms, std::string &err) {
         double *fa = b_fullA_ + (size_t)j * nfull_;
         k_bc_rt<<<nsub_, 256, 0, s_>>>(d_subs_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_R_, b_fullB_ + (size_t)j * nfull_,
                                        fa, d_t_);
-        k_gc<<<cdivb(ngc_total_, 256), 256, 0, s_>>>(ngc_total_, d_gptr_, d_gidx_, d_t_, d_gc_, nullptr);
-        k_coarse<<<dim3(ncl_, cdivb(maxg, 8)), 256, 0, s_>>>(d_cl_, d_M_, d_gc_, b_srec_ + (size_t)j * ngc_total_,
-                                                            nullptr);
+        if (d_M_) {
+            k_gc<<<cdivb(ngc_total_, 256), 256, 0, s_>>>(ngc_total_, d_gptr_, d_gidx_, d_t_, d_gc_, nullptr);
+            k_coarse<<<dim3(ncl_, cdivb(maxg, 8)), 256, 0, s_>>>(d_cl_, d_M_, d_gc_, b_srec_ + (size_t)j * ngc_total_,
+                                                                nullptr);
+        } else {
+            coarse_apply(d_t_, b_srec_ + (size_t)j * ngc_total_, nullptr);
+        }
         k_sub_bct<<<nsub_, 32, 0, s_>>>(d_subs_, d_cl_, d_bcr_, d_bce_ptr_, d_bce_pos_, d_bce_val_,
                                         b_srec_ + (size_t)j * ngc_total_, fa);
     }
@@ -606,9 +624,23 @@ int Engine::batch_finish(htf_stats *stats, double &ms, std::string &err) {
         double *fa = b_fullA_ + (size_t)j * nfull_;
         k_add_R<<<nsub_, 256, 0, s_>>>(d_subs_, d_cl_, d_R_, d_H_, b_srec_ + (size_t)j * ngc_total_,
                                        b_alpha_ + (size_t)j * 6 * ncl_, fa);
-        k_gather_u<<<cdivb(ndof_, 256), 256, 0, s_>>>(ndof_, d_win_, fa, d_u_ + (size_t)(r.r0 + j) * ndof_);
+        k_gather_u<<<cdivb(ndof_, 256), 256, 0, s_>>>(ndof_, d_win_, fa, d_u_ + (size_t)(r0 + j) * ndof_);
     }
     launches_ += 2 + 9 * kc;
+    return HTF_OK;
+}
+
+// displacements of the chunk's load cases into d_u_; per-load-case stats
+int Engine::batch_finish(htf_stats *stats, double &ms, std::string &err) {
+    BatchRun &r = run_;
+    int rc0;
+    CKB(cudaEventRecord(run_e1_, s_));
+    CKB(cudaEventSynchronize(run_e1_));
+    float fms = 0.f;
+    cudaEventElapsedTime(&fms, run_e0_, run_e1_);
+    ms = fms;
+    const int kc = r.kc;
+    if ((rc0 = batch_reconstruct(r.r0, kc, err))) return rc0;
     for (int j = 0; j < kc; ++j) {
         if (stats && r.r0 + j < 64) {
             stats->iterations[r.r0 + j] = r.st[j].it;
@@ -700,6 +732,185 @@ int Engine::solve_batch(Problem &p, int nrhs, const double *f_nodal, double *u, 
         stats->n_rhs = nrhs;
         stats->status_sub = status_sub;
         stats->kernel_launches = launches_;
+    }
+    return HTF_OK;
+}
+
+// ---------------------------------------------------------------------------
+// FP64 form, several load cases at once: Cluster::pcpg per column with the
+// matrices read once per iteration for up to 32 of them.  F_i, S_i and M are
+// applied from their packed FP64 tiles on the FP64 tensor path
+// (k_symv_rows_multi, k_msym_rows_multi), everything else by the kernels of
+// the mixed form; the recurrences and the stopping rule are those of
+// solve_one.  With one load case the SYMV is bound by the tiles' bytes; with
+// B64_MIN or more the products' 4 n_b^2 flops per load case cost less than
+// reading the tiles again for each.
+// ---------------------------------------------------------------------------
+constexpr int B64_MIN = 3;
+
+// Batch vectors for nrhs load cases; false when the batched form does not
+// apply: too many Bc rows per subdomain, no explicit S_i tiles, or vectors
+// that would take more than a quarter of the free device memory.
+bool Engine::ready_batch64(int nrhs) {
+    if (b64_off_ || mixed_ || implicit_ || !d_S_ || nrhs < B64_MIN) return false;
+    const int K = nrhs <= 16 ? 16 : 32;
+    if (bK_ >= K) return true;
+    for (auto &h : hs_)
+        if ((h.c + 6) * K > 2048) {
+            b64_off_ = bK_ == 0;
+            return bK_ > 0;
+        }
+    long long tn = 0, nch = 1;
+    for (auto &h : hs_) {
+        tn = std::max<long long>(tn, h.t_off + h.c + 6);
+        nch = std::max<long long>(nch, (h.nb + 127) / 128);
+    }
+    const double need = 8.0 * K *
+                        (9.0 * nlam_ + 2.0 * nslots_ + 2.0 * nfull_ + double(tn) * nch + 3.0 * ngc_total_ +
+                         6.0 * nchunks_ + 1184.0 + double(std::max(opt_.max_iter, 0)) + 1.0);
+    size_t fr = 0, tot = 0;
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || need > 0.25 * double(fr)) {
+        cudaGetLastError();
+        b64_off_ = bK_ == 0;
+        return bK_ > 0;
+    }
+    if (cudaStreamSynchronize(s_) != cudaSuccess) return false;
+    if (bgraph_) cudaGraphExecDestroy(bgraph_);
+    bgraph_ = nullptr;
+    bK_ = 0;
+    bmem_.clear();
+    std::string why;
+    into_ = &bmem_;
+    int rc = alloc_batch(K, why);
+    b_hist_ = alloc<double>((size_t(std::max(opt_.max_iter, 0)) + 1) * K, why, rc);
+    into_ = &mem_;
+    if (rc) {                                       // one load case at a time needs none of it
+        cudaGetLastError();
+        bmem_.clear();
+        b64_off_ = true;
+        return false;
+    }
+    bK_ = K;
+    return true;
+}
+
+// F and S products, projections and recurrences of one iteration of every running column
+void Engine::iteration_batch64() {
+    const int K = bK_;
+    const int nk = cdivb((long long)nlam_ * K, 256);
+    op_F_batch64(b_w_, b_Fw_, b_w_, b_part_);
+    k_colsum<<<K, 256, 0, s_>>>(b_part_, bnpart_, K, b_wFw_);
+    k_update_lam_g_multi<<<nk, 256, 0, s_>>>(nlam_, K, b_wFw_, nullptr, b_w_, b_Fw_, b_lam_, b_g_, b_st_);
+    op_P_batch(b_g_, b_Pg_, b_alpha2_, nullptr, nullptr);
+    op_M_batch64(b_Pg_, b_z_);
+    op_P_batch(b_z_, b_Pz_, nullptr, b_g_, b_part_);
+    k_colsum<<<K, 256, 0, s_>>>(b_part_, bnpart_, K, b_gPz_);
+    k_update_w_multi<<<nk, 256, 0, s_>>>(nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_);
+    k_finish_multi<<<1, 32, 0, s_>>>(K, b_wFw_, b_gPz_, b_st_, b_hist_);
+}
+
+void Engine::op_F_batch64(const double *w, double *Fw, const double *dotv, double *partial) {
+    k_gather_multi<<<nslots_ / 32, 256, 0, s_>>>(nslots_, bK_, d_slot_ptr_, d_slot_ent_, w, nullptr, b_xb_, nullptr,
+                                                 nullptr, 0.f);
+    coarse_batch();
+    symv_multi(d_F_, b_s_);
+    k_rows_multi<<<bnpart_, 256, 0, s_>>>(nlam_, bK_, d_rslot_, d_rsign_, b_yb_, nullptr, Fw, dotv, partial);
+}
+
+void Engine::op_M_batch64(const double *x, double *z) {
+    k_gather_multi<<<nslots_ / 32, 256, 0, s_>>>(nslots_, bK_, d_slot_ptr_, d_slot_ent_, x, d_weight_, b_xb_, nullptr,
+                                                 nullptr, 0.f);
+    symv_multi(d_S_, nullptr);
+    k_rows_multi<<<bnpart_, 256, 0, s_>>>(nlam_, bK_, d_rslot_, d_rsign_, b_yb_, d_weight_, z, nullptr, nullptr);
+}
+
+// load cases [r0, r0 + kc) together: per-column results in run_.st, displacements in d_u_
+int Engine::solve_chunk64(int r0, int kc, double &ms, std::string &err) {
+    BatchRun &r = run_;
+    const int K = bK_;
+    if (!run_e0_) {
+        CKB(cudaEventCreate(&run_e0_));
+        CKB(cudaEventCreate(&run_e1_));
+    }
+    if (!bgraph_) {
+        cudaGraph_t g;
+        CKB(cudaStreamBeginCapture(s_, cudaStreamCaptureModeThreadLocal));
+        iteration_batch64();
+        CKB(cudaStreamEndCapture(s_, &g));
+        size_t nn = 0;
+        CKB(cudaGraphGetNodes(g, nullptr, &nn));
+        bkernels_per_iter_ = int(nn);
+        CKB(cudaGraphInstantiate(&bgraph_, g, 0));
+        cudaGraphDestroy(g);
+    }
+    int rc = batch_rhs(r0, kc, err);
+    if (rc) return rc;
+    CKB(cudaEventRecord(run_e0_, s_));
+    // g0 = F lambda0 - d, Pg, z, Pz, g'Pz (pcpg_start)
+    const long long nk = (long long)nlam_ * K;
+    op_F_batch64(b_lam_, b_g_, nullptr, nullptr);
+    k_axpby<<<cdivb(nk, 256), 256, 0, s_>>>(int(nk), -1.0, b_d_, 1.0, b_g_);
+    op_P_batch(b_g_, b_Pg_, b_alpha2_, nullptr, nullptr);
+    op_M_batch64(b_Pg_, b_z_);
+    op_P_batch(b_z_, b_Pz_, nullptr, b_g_, b_part_);
+    k_colsum<<<K, 256, 0, s_>>>(b_part_, bnpart_, K, b_gPz_);
+    CKB(cudaMemcpyAsync(b_w_, b_Pz_, nk * sizeof(double), cudaMemcpyDeviceToDevice, s_));
+    launches_ += 18;
+    std::vector<double> gPz(K);
+    CKB(cudaMemcpyAsync(gPz.data(), b_gPz_, K * sizeof(double), cudaMemcpyDeviceToHost, s_));
+    CKB(cudaStreamSynchronize(s_));
+    r.st.assign(K, PcpgState{});
+    for (int j = 0; j < K; ++j) {
+        PcpgState &st = r.st[j];
+        st.done = 1;
+        if (j >= kc) continue;
+        st.gPz = st.gPz_prev = gPz[j];
+        st.norm0 = std::sqrt(gPz[j]);
+        st.rel = 1.0;
+        st.eps = opt_.eps_iter;
+        st.max_iter = opt_.max_iter;
+        st.wFw = 1.0;
+        st.done = (gPz[j] > 0.0 && std::isfinite(gPz[j])) ? (opt_.max_iter <= 0 ? 3 : 0) : (gPz[j] == 0.0 ? 1 : 2);
+    }
+    CKB(cudaMemcpyAsync(b_st_, r.st.data(), K * sizeof(PcpgState), cudaMemcpyHostToDevice, s_));
+    for (;;) {
+        for (int k = 0; k < std::max(1, opt_.check_every); ++k) CKB(cudaGraphLaunch(bgraph_, s_));
+        launches_ += (long long)std::max(1, opt_.check_every) * bkernels_per_iter_;
+        CKB(cudaMemcpyAsync(r.st.data(), b_st_, K * sizeof(PcpgState), cudaMemcpyDeviceToHost, s_));
+        CKB(cudaStreamSynchronize(s_));
+        bool all = true;
+        for (int j = 0; j < kc; ++j) all &= r.st[j].done != 0;
+        if (all) break;
+    }
+    CKB(cudaEventRecord(run_e1_, s_));
+    CKB(cudaEventSynchronize(run_e1_));
+    float fms = 0.f;
+    cudaEventElapsedTime(&fms, run_e0_, run_e1_);
+    ms = fms;
+    // residual histories of the first 64 load cases
+    int itmax = 0;
+    for (int j = 0; j < kc; ++j) itmax = std::max(itmax, std::min(r.st[j].it, opt_.max_iter));
+    std::vector<double> h((size_t(std::max(itmax, 0)) + 1) * K);
+    CKB(cudaMemcpy(h.data(), b_hist_, h.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    for (int j = 0; j < kc && r0 + j < 64; ++j) {
+        std::vector<double> c(size_t(std::max(0, std::min(r.st[j].it, opt_.max_iter))) + 1, 1.0);
+        for (size_t i = 1; i < c.size(); ++i) c[i] = h[i * K + j];
+        if (int(hist_.size()) <= r0 + j) hist_.resize(r0 + j + 1);
+        hist_[r0 + j] = std::move(c);
+    }
+    // alpha of the final residuals, column-major
+    std::vector<int> ones(K, 1);
+    CKB(cudaMemcpyAsync(d_mask_, ones.data(), K * sizeof(int), cudaMemcpyHostToDevice, s_));
+    k_alpha_cols<<<1, 256, 0, s_>>>(6 * ncl_, K, d_mask_, b_alpha2_, b_alpha_);
+    if ((rc = batch_reconstruct(r0, kc, err))) return rc;
+    CKB(cudaGetLastError());
+    int kserr = 0;
+    CKB(cudaMemcpyAsync(&kserr, d_kserr_, sizeof(int), cudaMemcpyDeviceToHost, s_));
+    CKB(cudaStreamSynchronize(s_));
+    if (kserr) {
+        CKB(cudaMemsetAsync(d_kserr_, 0, sizeof(int), s_));
+        err = "K_reg solve timed out on a barrier";
+        return kserr;
     }
     return HTF_OK;
 }

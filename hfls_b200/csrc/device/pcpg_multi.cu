@@ -537,11 +537,11 @@ __global__ void k_update_lam_g_multi(int n, int K, const double *__restrict__ wF
     if (id >= (long long)n * K) return;
     const int j = int(id % K);
     if (st[j].done) return;
-    // step length -g'w / w'Fw: equal to -g'Pz / w'Fw in exact arithmetic, and
-    // still the exact line minimum along w after the residual g has been
-    // replaced by the FP64 one
+    // mixed form: step length -g'w / w'Fw, equal to -g'Pz / w'Fw in exact
+    // arithmetic and still the exact line minimum along w after the residual
+    // g has been replaced by the FP64 one; FP64 form (no gw): -g'Pz / w'Fw
     const double d = wFw[j];
-    double rho = -gw[j] / d;
+    double rho = -(gw ? gw[j] : st[j].gPz) / d;
     if (!(d > 0.0) || !isfinite(rho)) rho = 0.0;
     lam[id] += rho * w[id];
     g[id] += rho * Fw[id];
@@ -570,8 +570,9 @@ __global__ void k_update_w_multi(int n, int K, const double *__restrict__ gPz_ne
     w[id] = Pz[id] + (gPz_new[j] / st[j].gPz) * w[id];
 }
 
+// hist (FP64 form): relative residual of column j after iteration it at hist[it * K + j]
 __global__ void k_finish_multi(int K, const double *__restrict__ wFw, const double *__restrict__ gPz_new,
-                               PcpgState *__restrict__ st) {
+                               PcpgState *__restrict__ st, double *__restrict__ hist) {
     const int j = threadIdx.x;
     if (j >= K || st[j].done) return;
     const double gPz = gPz_new[j];
@@ -581,6 +582,7 @@ __global__ void k_finish_multi(int K, const double *__restrict__ wFw, const doub
     st[j].gPz = gPz;
     st[j].it += 1;
     st[j].rel = sqrt(gPz) / st[j].norm0;
+    if (hist && st[j].it <= st[j].max_iter) hist[(size_t)st[j].it * K + j] = st[j].rel;
     if (!(wFw[j] > 0.0) || !isfinite(gPz)) st[j].done = 2;   // hand back to the FP64 residual check
     else if (sqrt(gPz) < st[j].eps * st[j].norm0) st[j].done = 1;
     else if (st[j].it >= st[j].max_iter) st[j].done = 3;
@@ -612,6 +614,61 @@ namespace htf {
 // the coarse correction y_b -= V_d s_d is applied before the store.
 // ---------------------------------------------------------------------------
 
+// rows [32 I, 32 I + 32) of A X for the symmetric A of nt tile rows packed at
+// base, X = x (RHS-interleaved, rows < nx; zero beyond): acc[q] = this
+// thread's entries of row 8 band + g, columns 8 (cb0 + q) + 2 t4, + 1
+template <int K>
+__device__ __forceinline__ void sym_rows_product(const double *__restrict__ base, int nt, int I, const double *x,
+                                                 int nx, double (&acc)[K / 16][2]) {
+    constexpr int NT = K / 16;                      // 8x8 output tiles per warp
+    constexpr int TS = 36, XS = K + 4;              // row strides (doubles): conflict-free fragment loads
+    __shared__ double Ts[32 * TS];
+    __shared__ double Xs[32 * XS];
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int g = lane >> 2, t4 = lane & 3;         // fragment row / column groups
+    const int band = warp & 3, cb0 = (warp >> 2) * NT;
+#pragma unroll
+    for (int q = 0; q < NT; ++q) acc[q][0] = acc[q][1] = 0.0;
+    double tr[TILE_ELEMS / 256], xr[TILE * K / 256];
+    auto fetch = [&](int J) {
+        const double *tp = base + (J <= I ? (long long)I * (I + 1) / 2 + J : (long long)J * (J + 1) / 2 + I) * TILE_ELEMS;
+#pragma unroll
+        for (int u = 0; u < TILE_ELEMS / 256; ++u) tr[u] = tp[threadIdx.x + 256 * u];
+#pragma unroll
+        for (int u = 0; u < TILE * K / 256; ++u) {
+            const int e = threadIdx.x + 256 * u, r = TILE * J + e / K;
+            xr[u] = r < nx ? x[(size_t)r * K + e % K] : 0.0;
+        }
+    };
+    fetch(0);
+    for (int J = 0; J < nt; ++J) {
+        const bool lower = J <= I;
+#pragma unroll
+        for (int u = 0; u < TILE_ELEMS / 256; ++u) {
+            const int e = threadIdx.x + 256 * u, rr = e / TILE, cc = e % TILE;
+            if (lower) Ts[rr * TS + cc] = tr[u];    // stored tile (I, J): A[32I + rr][32J + cc]
+            else Ts[cc * TS + rr] = tr[u];          // tile (J, I): A[32I + cc][32J + rr]
+        }
+#pragma unroll
+        for (int u = 0; u < TILE * K / 256; ++u) {
+            const int e = threadIdx.x + 256 * u;
+            Xs[(e / K) * XS + e % K] = xr[u];
+        }
+        __syncthreads();
+        if (J + 1 < nt) fetch(J + 1);               // in flight during the products
+#pragma unroll
+        for (int kk = 0; kk < TILE / 4; ++kk) {
+            const double a = Ts[(8 * band + g) * TS + 4 * kk + t4];
+#pragma unroll
+            for (int q = 0; q < NT; ++q) {
+                const double bq = Xs[(4 * kk + t4) * XS + 8 * (cb0 + q) + g];
+                dmma_8x8x4(acc[q][0], acc[q][1], a, bq);
+            }
+        }
+        __syncthreads();
+    }
+}
+
 template <int K>
 __global__ void __launch_bounds__(256) k_symv_rows_multi(const int2 *__restrict__ rowblk,
                                                          const SubDev *__restrict__ subs,
@@ -621,45 +678,15 @@ __global__ void __launch_bounds__(256) k_symv_rows_multi(const int2 *__restrict_
                                                          const double *__restrict__ Vbuf,
                                                          const int *__restrict__ bcrows,
                                                          const double *__restrict__ s) {
-    constexpr int NT = K / 16;                      // 8x8 output tiles per warp
-    constexpr int TS = 36, XS = K + 4;              // row strides (doubles): conflict-free fragment loads
-    __shared__ double Ts[32 * TS];
-    __shared__ double Xs[32 * XS];
+    constexpr int NT = K / 16;
     const int2 rb = rowblk[blockIdx.x];
     const SubDev &sd = subs[rb.x];
     const int I = rb.y;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int g = lane >> 2, t4 = lane & 3;         // fragment row / column groups
+    const int g = lane >> 2, t4 = lane & 3;
     const int band = warp & 3, cb0 = (warp >> 2) * NT;
-    const double *base = tiles + sd.T_off * TILE_ELEMS;
     double acc[NT][2];
-#pragma unroll
-    for (int q = 0; q < NT; ++q) acc[q][0] = acc[q][1] = 0.0;
-    for (int J = 0; J < sd.nt; ++J) {
-        const bool lower = J <= I;
-        const double *tp = base + (lower ? (long long)I * (I + 1) / 2 + J : (long long)J * (J + 1) / 2 + I) * TILE_ELEMS;
-        for (int e = threadIdx.x; e < TILE_ELEMS; e += blockDim.x) {
-            const int rr = e / TILE, cc = e % TILE;
-            const double v = tp[e];                 // stored tile, row rr, column cc
-            if (lower) Ts[rr * TS + cc] = v;        // A[32I + rr][32J + cc]
-            else Ts[cc * TS + rr] = v;              // tile (J, I): A[32I + cc][32J + rr]
-        }
-        for (int e = threadIdx.x; e < TILE * K; e += blockDim.x) {
-            const int c = e / K, j = e % K;
-            Xs[c * XS + j] = xb[(size_t)(sd.xb_off + TILE * J + c) * K + j];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < TILE / 4; ++kk) {
-            const double a = Ts[(8 * band + g) * TS + 4 * kk + t4];
-#pragma unroll
-            for (int q = 0; q < NT; ++q) {
-                const double b = Xs[(4 * kk + t4) * XS + 8 * (cb0 + q) + g];
-                dmma_8x8x4(acc[q][0], acc[q][1], a, b);
-            }
-        }
-        __syncthreads();
-    }
+    sym_rows_product<K>(tiles + sd.T_off * TILE_ELEMS, sd.nt, I, xb + (size_t)sd.xb_off * K, sd.nbp, acc);
     const int row = TILE * I + 8 * band + g;        // this thread's output row
     if (s && row < sd.nb) {
         const int gc_off = cl[sd.cluster].gc_off;
@@ -688,6 +715,36 @@ template __global__ void k_symv_rows_multi<16>(const int2 *, const SubDev *, con
                                                const ClusterDev *, const double *, const int *, const double *);
 template __global__ void k_symv_rows_multi<32>(const int2 *, const SubDev *, const double *, const double *, double *,
                                                const ClusterDev *, const double *, const int *, const double *);
+
+// S = M G per cluster from the packed symmetric tiles of M (pcpg_kernels.cu):
+// CTA (cluster, 32-row block), the product of k_symv_rows_multi
+template <int K>
+__global__ void __launch_bounds__(256) k_msym_rows_multi(const int2 *__restrict__ mt,
+                                                         const ClusterDev *__restrict__ cl,
+                                                         const double *__restrict__ T, const double *__restrict__ gc,
+                                                         double *__restrict__ s) {
+    constexpr int NT = K / 16;
+    const int2 b = mt[blockIdx.x];
+    const ClusterDev c = cl[b.x];
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int band = warp & 3, cb0 = (warp >> 2) * NT;
+    double acc[NT][2];
+    sym_rows_product<K>(T + c.MT_off * TILE_ELEMS, c.mt, b.y, gc + (size_t)c.gc_off * K, c.ngc, acc);
+    const int row = TILE * b.y + 8 * band + g;
+    if (row >= c.ngc) return;
+    double *y = s + (size_t)(c.gc_off + row) * K;
+#pragma unroll
+    for (int u = 0; u < NT; ++u) {
+        const int col = 8 * (cb0 + u) + 2 * t4;
+        y[col] = acc[u][0];
+        y[col + 1] = acc[u][1];
+    }
+}
+template __global__ void k_msym_rows_multi<16>(const int2 *, const ClusterDev *, const double *, const double *,
+                                               double *);
+template __global__ void k_msym_rows_multi<32>(const int2 *, const ClusterDev *, const double *, const double *,
+                                               double *);
 
 // B(:, j) = A(:, j) for the columns j with mask[j] (n rows, K-interleaved)
 __global__ void k_cols_copy(long long n, int K, const int *__restrict__ mask, const double *__restrict__ A,
