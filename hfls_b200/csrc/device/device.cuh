@@ -224,6 +224,13 @@ __device__ __forceinline__ int step_entry(const StepDesc *st, int cnt, int b, F 
 #endif
 
 #ifdef __CUDACC__
+// Links of a chain of programmatic dependent launches: let the successor
+// start once all CTAs of this kernel have started or ended; wait until the
+// predecessor has completed (a no-op in an ordinary launch).  Every kernel of
+// a chain waits, so a completed one implies all before it.
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Launch as a link of the PCPG chain (pcpg_kernels.cu): the kernel may start
 // before its predecessor in the stream has finished and waits for it itself.
 template <typename... P, typename... A>

@@ -112,6 +112,8 @@ private:
     void op_F_batch(const double *w, double *Fw, const double *dotv, double *partial);
     void op_M_batch(const double *x, double *z);
     void op_P_batch(const double *x, double *Px, double *alpha_out, const double *dotv, double *partial);
+    template <typename... P, typename... A>
+    void link(void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args);
     void iteration_batch();
     int batch_rhs(int r0, int kc, std::string &err);
     int batch_reconstruct(int r0, int kc, std::string &err);

@@ -82,6 +82,8 @@ __global__ void k_add_R(const SubDev *, const ClusterDev *, const double *, cons
                         const double *, double *);
 __global__ void k_gather_u(int, const int *, const double *, double *);
 
+constexpr int GFT_SMEM = 1024 * (6 * 8 + 4);        // k_gft_partial_multi: one chunk's rows and Gf values
+
 static inline int cdivb(long long a, long long b) { return int((a + b - 1) / b); }
 
 #define CKB(call)                                                  \
@@ -89,6 +91,14 @@ static inline int cdivb(long long a, long long b) { return int((a + b - 1) / b);
         int _rc = check((call), #call, err, "engine_batch.cu", __LINE__); \
         if (_rc) return _rc;                                       \
     } while (0)
+
+// launch on the engine's stream: as a link of the iteration's chain (device.cuh) on its own stream; in an ordinary
+// way on a server's, whose captured graphs fork and join several streams around shared launches
+template <typename... P, typename... A>
+void Engine::link(void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+    if (s_ == own_s_) launch_chain(k, grid, block, smem, s_, args...);
+    else k<<<grid, block, smem, s_>>>(args...);
+}
 
 // tensor-core blocks and slab buffers (once; before the factorisation
 // when S_i is made into slabs wave by wave)
@@ -198,6 +208,7 @@ int Engine::setup_batch(int K, std::string &err) {
 // vectors of a batch of K load cases (mixed and FP64 form)
 int Engine::alloc_batch(int K, std::string &err) {
     int rc = HTF_OK;
+    CKB(cudaFuncSetAttribute(k_gft_partial_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, GFT_SMEM));
     // batch vectors
     const size_t nl = (size_t)nlam_ * K;
     int ntot = 0;
@@ -252,7 +263,7 @@ void Engine::gather_x(const double *w, const double *weight, double *xb) {
     const int K = bK_;
     cudaMemsetAsync(d_xmax_, 0, K * sizeof(unsigned), s_);
     k_colmax<<<std::max(1, std::min(cdivb((long long)nlam_ * K, 256), 1184)), 256, 0, s_>>>(nlam_, K, w, d_xmax_);
-    k_gather_multi<<<nslots_ / 32, 256, 0, s_>>>(nslots_, K, d_slot_ptr_, d_slot_ent_, w, weight, xb, d_Xs_, d_xmax_,
+    link(k_gather_multi, nslots_ / 32, 256, 0, nslots_, K, d_slot_ptr_, d_slot_ent_, w, weight, xb, d_Xs_, d_xmax_,
                                                  xbound_);
 }
 
@@ -290,36 +301,36 @@ void Engine::coarse_batch() {
     for (auto &c : hc_) maxg = std::max(maxg, c.ngc);
     const dim3 gv(nsub_, vt_nch_);
     if (K == 32) {
-        if (vt_qn_ == 32) k_vt_multi<32, 32><<<gv, 256, 0, s_>>>(vt_nch_, d_subs_, d_V_, b_xb_, b_t_);
-        else k_vt_multi<32, 64><<<gv, 256, 0, s_>>>(vt_nch_, d_subs_, d_V_, b_xb_, b_t_);
+        if (vt_qn_ == 32) link(k_vt_multi<32, 32>, gv, 256, 0, vt_nch_, d_subs_, d_V_, b_xb_, b_t_);
+        else link(k_vt_multi<32, 64>, gv, 256, 0, vt_nch_, d_subs_, d_V_, b_xb_, b_t_);
     } else {
-        if (vt_qn_ == 32) k_vt_multi<16, 32><<<gv, 256, 0, s_>>>(vt_nch_, d_subs_, d_V_, b_xb_, b_t_);
-        else if (vt_qn_ == 64) k_vt_multi<16, 64><<<gv, 256, 0, s_>>>(vt_nch_, d_subs_, d_V_, b_xb_, b_t_);
-        else k_vt_multi<16, 128><<<gv, 256, 0, s_>>>(vt_nch_, d_subs_, d_V_, b_xb_, b_t_);
+        if (vt_qn_ == 32) link(k_vt_multi<16, 32>, gv, 256, 0, vt_nch_, d_subs_, d_V_, b_xb_, b_t_);
+        else if (vt_qn_ == 64) link(k_vt_multi<16, 64>, gv, 256, 0, vt_nch_, d_subs_, d_V_, b_xb_, b_t_);
+        else link(k_vt_multi<16, 128>, gv, 256, 0, vt_nch_, d_subs_, d_V_, b_xb_, b_t_);
     }
-    k_gc_multi<<<cdivb((long long)ngc_total_ * K, 256), 256, 0, s_>>>(ngc_total_, K, vt_nch_, d_gptr_, d_gidx_, b_t_,
+    link(k_gc_multi, cdivb((long long)ngc_total_ * K, 256), 256, 0, ngc_total_, K, vt_nch_, d_gptr_, d_gidx_, b_t_,
                                                                       b_gc_);
     if (!d_M_) {                                    // FP64 form: packed symmetric tiles
-        if (K == 32) k_msym_rows_multi<32><<<nmt_, 256, 0, s_>>>(d_mt_, d_cl_, d_MT_, b_gc_, b_s_);
-        else k_msym_rows_multi<16><<<nmt_, 256, 0, s_>>>(d_mt_, d_cl_, d_MT_, b_gc_, b_s_);
+        if (K == 32) link(k_msym_rows_multi<32>, nmt_, 256, 0, d_mt_, d_cl_, d_MT_, b_gc_, b_s_);
+        else link(k_msym_rows_multi<16>, nmt_, 256, 0, d_mt_, d_cl_, d_MT_, b_gc_, b_s_);
         return;
     }
-    if (K == 32) k_coarse_multi<32><<<dim3(ncl_, cdivb(maxg, 32)), 128, 0, s_>>>(d_cl_, d_M_, b_gc_, b_s_);
-    else k_coarse_multi<16><<<dim3(ncl_, cdivb(maxg, 32)), 128, 0, s_>>>(d_cl_, d_M_, b_gc_, b_s_);
+    if (K == 32) link(k_coarse_multi<32>, dim3(ncl_, cdivb(maxg, 32)), 128, 0, d_cl_, d_M_, b_gc_, b_s_);
+    else link(k_coarse_multi<16>, dim3(ncl_, cdivb(maxg, 32)), 128, 0, d_cl_, d_M_, b_gc_, b_s_);
 }
 
 void Engine::f_post(double *Fw, const double *dotv, double *partial) {
     const dim3 gc(nsub_, cdivb(max_nbp_, 128));
-    if (bK_ == 32) k_correct_multi<32><<<gc, 256, 0, s_>>>(d_subs_, d_cl_, d_V_, d_bcr_, b_s_, b_yb_);
-    else k_correct_multi<16><<<gc, 256, 0, s_>>>(d_subs_, d_cl_, d_V_, d_bcr_, b_s_, b_yb_);
-    k_rows_multi<<<bnpart_, 256, 0, s_>>>(nlam_, bK_, d_rslot_, d_rsign_, b_yb_, nullptr, Fw, dotv, partial);
+    if (bK_ == 32) link(k_correct_multi<32>, gc, 256, 0, d_subs_, d_cl_, d_V_, d_bcr_, b_s_, b_yb_);
+    else link(k_correct_multi<16>, gc, 256, 0, d_subs_, d_cl_, d_V_, d_bcr_, b_s_, b_yb_);
+    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, nullptr, Fw, dotv, partial);
 }
 
 // the preconditioner uses the same FP16-pair products as F
 void Engine::m_pre(const double *x) { gather_x(x, d_weight_, nullptr); }
 
 void Engine::m_post(double *z) {
-    k_rows_multi<<<bnpart_, 256, 0, s_>>>(nlam_, bK_, d_rslot_, d_rsign_, b_yb_, d_weight_, z, nullptr, nullptr);
+    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, d_weight_, z, nullptr, nullptr);
 }
 
 void Engine::op_F_batch(const double *w, double *Fw, const double *dotv, double *partial) {
@@ -336,10 +347,10 @@ void Engine::op_M_batch(const double *x, double *z) {
 
 void Engine::op_P_batch(const double *x, double *Px, double *alpha_out, const double *dotv, double *partial) {
     const int K = bK_;
-    k_gft_partial_multi<<<nchunks_, 256, 0, s_>>>(K, d_chunk_beg_, d_chunk_end_, d_crow_, d_cval_, x, b_gpart_);
-    k_gt_sum_multi<<<ncl_, 6 * K, 0, s_>>>(K, d_cl_chunk_ptr_, b_gpart_, b_gt_);
-    k_gf_coef_multi<<<1, 1024, 0, s_>>>(K, ncl_, d_invGtG_, b_gt_, b_acoef_, alpha_out);
-    k_gf_apply_multi<<<bnpart_, 256, 0, s_>>>(nlam_, K, b_acoef_, d_gcl_, d_gval_, x, Px, dotv, partial);
+    link(k_gft_partial_multi, nchunks_, 256, GFT_SMEM, K, d_chunk_beg_, d_chunk_end_, d_crow_, d_cval_, x, b_gpart_);
+    link(k_gt_sum_multi, 6 * ncl_, K, 0, K, d_cl_chunk_ptr_, b_gpart_, b_gt_);
+    link(k_gf_coef_multi, 6 * ncl_, K, 0, K, ncl_, d_invGtG_, b_gt_, b_acoef_, alpha_out);
+    link(k_gf_apply_multi, bnpart_, 256, 0, nlam_, K, b_acoef_, d_gcl_, d_gval_, x, Px, dotv, partial);
 }
 
 // one batched iteration = iter_a | F product | iter_b | S product | iter_c
@@ -349,10 +360,10 @@ void Engine::iter_b() {
     const int K = bK_;
     const int nk = cdivb((long long)nlam_ * K, 256);
     f_post(b_Fw_, b_w_, b_part_);
-    k_colsum<<<K, 256, 0, s_>>>(b_part_, bnpart_, K, b_wFw_);
-    k_dot_multi<<<bnpart_, 256, 0, s_>>>(nlam_, K, b_g_, b_w_, b_part_);
-    k_colsum<<<K, 256, 0, s_>>>(b_part_, bnpart_, K, b_gw_);
-    k_update_lam_g_multi<<<nk, 256, 0, s_>>>(nlam_, K, b_wFw_, b_gw_, b_w_, b_Fw_, b_lam_, b_g_, b_st_);
+    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_wFw_);
+    link(k_dot_multi, bnpart_, 256, 0, nlam_, K, b_g_, b_w_, b_part_);
+    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gw_);
+    link(k_update_lam_g_multi, nk, 256, 0, nlam_, K, b_wFw_, b_gw_, b_w_, b_Fw_, b_lam_, b_g_, b_st_);
     op_P_batch(b_g_, b_Pg_, nullptr, nullptr, nullptr);
     m_pre(b_Pg_);
 }
@@ -362,9 +373,9 @@ void Engine::iter_c() {
     const int nk = cdivb((long long)nlam_ * K, 256);
     m_post(b_z_);
     op_P_batch(b_z_, b_Pz_, nullptr, b_g_, b_part_);
-    k_colsum<<<K, 256, 0, s_>>>(b_part_, bnpart_, K, b_gPz_);
-    k_update_w_multi<<<nk, 256, 0, s_>>>(nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_);
-    k_finish_multi<<<1, 32, 0, s_>>>(K, b_wFw_, b_gPz_, b_st_, nullptr);
+    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_);
+    link(k_update_w_multi, nk, 256, 0, nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_);
+    link(k_finish_multi, 1, 32, 0, K, b_wFw_, b_gPz_, b_st_, nullptr);
 }
 
 void Engine::iteration_batch() {
@@ -413,9 +424,9 @@ int Engine::batch_loads(int nrhs, const double *f_nodal, std::string &err) {
 void Engine::symv_multi(const double *tiles, const double *scoarse) {
     const int2 *rb = static_cast<const int2 *>(d_rowblk_);
     if (bK_ == 32)
-        k_symv_rows_multi<32><<<nrowblk_, 256, 0, s_>>>(rb, d_subs_, tiles, b_xb_, b_yb_, d_cl_, d_V_, d_bcr_, scoarse);
+        link(k_symv_rows_multi<32>, nrowblk_, 256, 0, rb, d_subs_, tiles, b_xb_, b_yb_, d_cl_, d_V_, d_bcr_, scoarse);
     else
-        k_symv_rows_multi<16><<<nrowblk_, 256, 0, s_>>>(rb, d_subs_, tiles, b_xb_, b_yb_, d_cl_, d_V_, d_bcr_, scoarse);
+        link(k_symv_rows_multi<16>, nrowblk_, 256, 0, rb, d_subs_, tiles, b_xb_, b_yb_, d_cl_, d_V_, d_bcr_, scoarse);
 }
 
 // FP64 residuals of the load cases j with sel[j] (Cluster.cpp:1398-1412 from
@@ -430,24 +441,24 @@ int Engine::fp64_residual_batch(const std::vector<int> &sel, const std::vector<i
     const int K = bK_;
     const long long nk = (long long)nlam_ * K;
     // g = F lambda - d
-    k_gather_multi<<<nslots_ / 32, 256, 0, s_>>>(nslots_, K, d_slot_ptr_, d_slot_ent_, b_lam_, nullptr, b_xb_, nullptr,
+    link(k_gather_multi, nslots_ / 32, 256, 0, nslots_, K, d_slot_ptr_, d_slot_ent_, b_lam_, nullptr, b_xb_, nullptr,
                                                  nullptr, 0.f);
     coarse_batch();
     symv_multi(d_F_, b_s_);
-    k_rows_multi<<<bnpart_, 256, 0, s_>>>(nlam_, K, d_rslot_, d_rsign_, b_yb_, nullptr, b_tmp_, nullptr, nullptr);
+    link(k_rows_multi, bnpart_, 256, 0, nlam_, K, d_rslot_, d_rsign_, b_yb_, nullptr, b_tmp_, nullptr, nullptr);
     k_axpby<<<cdivb(nk, 256), 256, 0, s_>>>(int(nk), -1.0, b_d_, 1.0, b_tmp_);
     op_P_batch(b_tmp_, b_Pg_, b_alpha2_, nullptr, nullptr);
     // z = M P g, P z, g'Pz
     if (d_S_) {
-        k_gather_multi<<<nslots_ / 32, 256, 0, s_>>>(nslots_, K, d_slot_ptr_, d_slot_ent_, b_Pg_, d_weight_, b_xb_,
+        link(k_gather_multi, nslots_ / 32, 256, 0, nslots_, K, d_slot_ptr_, d_slot_ent_, b_Pg_, d_weight_, b_xb_,
                                                      nullptr, nullptr, 0.f);
         symv_multi(d_S_, nullptr);
-        k_rows_multi<<<bnpart_, 256, 0, s_>>>(nlam_, K, d_rslot_, d_rsign_, b_yb_, d_weight_, b_z_, nullptr, nullptr);
+        link(k_rows_multi, bnpart_, 256, 0, nlam_, K, d_rslot_, d_rsign_, b_yb_, d_weight_, b_z_, nullptr, nullptr);
     } else {
         op_M_batch(b_Pg_, b_z_);      // S_i only as tensor-core slabs: the tensor-core product
     }
     op_P_batch(b_z_, b_Pz_, nullptr, b_tmp_, b_part_);
-    k_colsum<<<K, 256, 0, s_>>>(b_part_, bnpart_, K, b_gPz_);
+    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_);
     // the selected columns back into the recurrence
     std::vector<int> masks(2 * K, 0);
     for (int j = 0; j < K; ++j) {
@@ -799,29 +810,29 @@ void Engine::iteration_batch64() {
     const int K = bK_;
     const int nk = cdivb((long long)nlam_ * K, 256);
     op_F_batch64(b_w_, b_Fw_, b_w_, b_part_);
-    k_colsum<<<K, 256, 0, s_>>>(b_part_, bnpart_, K, b_wFw_);
-    k_update_lam_g_multi<<<nk, 256, 0, s_>>>(nlam_, K, b_wFw_, nullptr, b_w_, b_Fw_, b_lam_, b_g_, b_st_);
+    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_wFw_);
+    link(k_update_lam_g_multi, nk, 256, 0, nlam_, K, b_wFw_, nullptr, b_w_, b_Fw_, b_lam_, b_g_, b_st_);
     op_P_batch(b_g_, b_Pg_, b_alpha2_, nullptr, nullptr);
     op_M_batch64(b_Pg_, b_z_);
     op_P_batch(b_z_, b_Pz_, nullptr, b_g_, b_part_);
-    k_colsum<<<K, 256, 0, s_>>>(b_part_, bnpart_, K, b_gPz_);
-    k_update_w_multi<<<nk, 256, 0, s_>>>(nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_);
-    k_finish_multi<<<1, 32, 0, s_>>>(K, b_wFw_, b_gPz_, b_st_, b_hist_);
+    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_);
+    link(k_update_w_multi, nk, 256, 0, nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_);
+    link(k_finish_multi, 1, 32, 0, K, b_wFw_, b_gPz_, b_st_, b_hist_);
 }
 
 void Engine::op_F_batch64(const double *w, double *Fw, const double *dotv, double *partial) {
-    k_gather_multi<<<nslots_ / 32, 256, 0, s_>>>(nslots_, bK_, d_slot_ptr_, d_slot_ent_, w, nullptr, b_xb_, nullptr,
+    link(k_gather_multi, nslots_ / 32, 256, 0, nslots_, bK_, d_slot_ptr_, d_slot_ent_, w, nullptr, b_xb_, nullptr,
                                                  nullptr, 0.f);
     coarse_batch();
     symv_multi(d_F_, b_s_);
-    k_rows_multi<<<bnpart_, 256, 0, s_>>>(nlam_, bK_, d_rslot_, d_rsign_, b_yb_, nullptr, Fw, dotv, partial);
+    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, nullptr, Fw, dotv, partial);
 }
 
 void Engine::op_M_batch64(const double *x, double *z) {
-    k_gather_multi<<<nslots_ / 32, 256, 0, s_>>>(nslots_, bK_, d_slot_ptr_, d_slot_ent_, x, d_weight_, b_xb_, nullptr,
+    link(k_gather_multi, nslots_ / 32, 256, 0, nslots_, bK_, d_slot_ptr_, d_slot_ent_, x, d_weight_, b_xb_, nullptr,
                                                  nullptr, 0.f);
     symv_multi(d_S_, nullptr);
-    k_rows_multi<<<bnpart_, 256, 0, s_>>>(nlam_, bK_, d_rslot_, d_rsign_, b_yb_, d_weight_, z, nullptr, nullptr);
+    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, d_weight_, z, nullptr, nullptr);
 }
 
 // load cases [r0, r0 + kc) together: per-column results in run_.st, displacements in d_u_
@@ -853,7 +864,7 @@ int Engine::solve_chunk64(int r0, int kc, double &ms, std::string &err) {
     op_P_batch(b_g_, b_Pg_, b_alpha2_, nullptr, nullptr);
     op_M_batch64(b_Pg_, b_z_);
     op_P_batch(b_z_, b_Pz_, nullptr, b_g_, b_part_);
-    k_colsum<<<K, 256, 0, s_>>>(b_part_, bnpart_, K, b_gPz_);
+    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_);
     CKB(cudaMemcpyAsync(b_w_, b_Pz_, nk * sizeof(double), cudaMemcpyDeviceToDevice, s_));
     launches_ += 18;
     std::vector<double> gPz(K);

@@ -32,9 +32,6 @@ constexpr unsigned FULL = 0xffffffffu;
 // small problem's kernel costs one pass over the vectors it depends on instead
 // of a launch plus a chain of dependent loads.  Pointers to data that the
 // chain writes are not __restrict__, so that no load of them moves up.
-__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // sum over the CTA's 256 threads in a fixed order (all threads get it); red: 8 doubles of shared memory
 __device__ __forceinline__ double cta_sum(double v, double *red) {
 #pragma unroll

@@ -29,9 +29,11 @@ __device__ __forceinline__ void dmma_8x8x4(double &d0, double &d1, double a, dou
 // 32); the values go through shared memory so both outputs are written
 // coalesced.
 __global__ void k_gather_multi(int nslots, int K, const int *__restrict__ ptr, const int *__restrict__ ent,
-                               const double *__restrict__ w, const double *__restrict__ weight,
-                               double *__restrict__ xb, float *__restrict__ Xs, const unsigned *__restrict__ xmax,
+                               const double *w, const double *__restrict__ weight,
+                               double *xb, float *__restrict__ Xs, const unsigned *xmax,
                                float xbound) {
+    pdl_next();
+    pdl_wait();
     __shared__ double vs[32 * 33];
     __shared__ int ex[32];
     const int i0 = blockIdx.x * 32;
@@ -76,8 +78,8 @@ __global__ void k_gather_multi(int nslots, int K, const int *__restrict__ ptr, c
 // CTA (subdomain, chunk), 256 threads.
 template <int K, int QN>
 __global__ void __launch_bounds__(256) k_vt_multi(int nch, const SubDev *__restrict__ subs,
-                                                  const double *__restrict__ Vbuf, const double *__restrict__ xb,
-                                                  double *__restrict__ tpart) {
+                                                  const double *__restrict__ Vbuf, const double *xb,
+                                                  double *tpart) {
     constexpr int VS = 36, XS = K + 4;
     constexpr int T = QN * K / 512;                 // 8x8 tiles per warp
     constexpr int UX = 32 * K / 256, UV = QN / 8;   // staged values per thread
@@ -95,19 +97,24 @@ __global__ void __launch_bounds__(256) k_vt_multi(int nch, const SubDev *__restr
 #pragma unroll
     for (int u = 0; u < T; ++u) acc[u][0] = acc[u][1] = 0.0;
     double xr[UX], vr[UV];
-    auto fetch = [&](int i0) {
+    auto fetch_x = [&](int i0) {
 #pragma unroll
         for (int u = 0; u < UX; ++u) {
             const int o = threadIdx.x + 256 * u, ii = o / K;
             xr[u] = (i0 + ii < r_end) ? x[(size_t)(i0 + ii) * K + (o % K)] : 0.0;
         }
+    };
+    auto fetch_v = [&](int i0) {
 #pragma unroll
         for (int u = 0; u < UV; ++u) {
             const int o = threadIdx.x + 256 * u, q = o / 32, ii = o % 32;
             vr[u] = (q < ncol && i0 + ii < r_end) ? V[(size_t)q * sd.nbp + i0 + ii] : 0.0;
         }
     };
-    if (ch * 128 < r_end) fetch(ch * 128);
+    pdl_next();
+    if (ch * 128 < r_end) fetch_v(ch * 128);
+    pdl_wait();
+    if (ch * 128 < r_end) fetch_x(ch * 128);
     for (int i0 = ch * 128; i0 < r_end; i0 += 32) {
 #pragma unroll
         for (int u = 0; u < UX; ++u) {
@@ -120,7 +127,10 @@ __global__ void __launch_bounds__(256) k_vt_multi(int nch, const SubDev *__restr
             Vs[(o / 32) * VS + o % 32] = vr[u];
         }
         __syncthreads();
-        if (i0 + 32 < r_end) fetch(i0 + 32);        // next piece in flight during the products
+        if (i0 + 32 < r_end) {                      // next piece in flight during the products
+            fetch_x(i0 + 32);
+            fetch_v(i0 + 32);
+        }
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
 #pragma unroll
@@ -155,7 +165,9 @@ HTF_VT(32, 64)
 
 // gc[q][j] = sum over the t entries of coarse row q and their row chunks
 __global__ void k_gc_multi(int ngc_total, int K, int nch, const int *__restrict__ gptr, const int *__restrict__ gidx,
-                           const double *__restrict__ tpart, double *__restrict__ gc) {
+                           const double *tpart, double *gc) {
+    pdl_next();
+    pdl_wait();
     const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (id >= (long long)ngc_total * K) return;
     const int q = int(id / K), j = int(id % K);
@@ -172,8 +184,8 @@ __global__ void k_gc_multi(int ngc_total, int K, int nch, const int *__restrict_
 // 8w .. 8w + 7 and all K columns (K / 8 tiles sharing one A fragment).
 template <int K>
 __global__ void __launch_bounds__(128) k_coarse_multi(const ClusterDev *__restrict__ cl,
-                                                      const double *__restrict__ Mbuf, const double *__restrict__ gc,
-                                                      double *__restrict__ s) {
+                                                      const double *__restrict__ Mbuf, const double *gc,
+                                                      double *s) {
     constexpr int PK = 64, MS = PK + 4, GS = K + 4, NT = K / 8;
     constexpr int UM = 32 * PK / 128, UG = PK * K / 128;
     __shared__ double Ms[32 * MS];                  // [r][p]
@@ -189,19 +201,24 @@ __global__ void __launch_bounds__(128) k_coarse_multi(const ClusterDev *__restri
 #pragma unroll
     for (int u = 0; u < NT; ++u) acc[u][0] = acc[u][1] = 0.0;
     double mr[UM], gr[UG];
-    auto fetch = [&](int p0) {
+    auto fetch_m = [&](int p0) {
 #pragma unroll
         for (int u = 0; u < UM; ++u) {
             const int o = threadIdx.x + 128 * u, r = o / PK, pp = o % PK;
             mr[u] = (row0 + r < c.ngc && p0 + pp < c.ngc) ? M[(size_t)(row0 + r) * c.ngc + p0 + pp] : 0.0;
         }
+    };
+    auto fetch_g = [&](int p0) {
 #pragma unroll
         for (int u = 0; u < UG; ++u) {
             const int o = threadIdx.x + 128 * u, pp = o / K;
             gr[u] = (p0 + pp < c.ngc) ? G[(size_t)(p0 + pp) * K + (o % K)] : 0.0;
         }
     };
-    fetch(0);
+    pdl_next();
+    fetch_m(0);
+    pdl_wait();
+    fetch_g(0);
     for (int p0 = 0; p0 < c.ngc; p0 += PK) {
 #pragma unroll
         for (int u = 0; u < UM; ++u) {
@@ -214,7 +231,10 @@ __global__ void __launch_bounds__(128) k_coarse_multi(const ClusterDev *__restri
             Gs[(o / K) * GS + o % K] = gr[u];
         }
         __syncthreads();
-        if (p0 + PK < c.ngc) fetch(p0 + PK);        // next tiles in flight during the products
+        if (p0 + PK < c.ngc) {                      // next tiles in flight during the products
+            fetch_m(p0 + PK);
+            fetch_g(p0 + PK);
+        }
 #pragma unroll
         for (int kk = 0; kk < PK / 4; ++kk) {
             const double av = Ms[(8 * warp + g) * MS + 4 * kk + t4];
@@ -238,7 +258,7 @@ template __global__ void k_coarse_multi<32>(const ClusterDev *, const double *, 
 
 // per-block, per-column tree sum of prod over the block's rows (256 / K rows,
 // threads j, j+K, ...) -> partial[block][j]
-__device__ __forceinline__ void block_col_partial(double prod, int K, double *__restrict__ partial) {
+__device__ __forceinline__ void block_col_partial(double prod, int K, double *partial) {
     __shared__ double red[256];
     const int rows_per_block = 256 / K;
     const int lr = threadIdx.x / K, j = threadIdx.x % K;
@@ -256,7 +276,7 @@ __device__ __forceinline__ void block_col_partial(double prod, int K, double *__
 // so the partials and their sums are the same on every run); each thread
 // has the loads of two of its rows in flight and adds them in row order.
 __device__ __forceinline__ double row_value(int r, int K, int j, const int *__restrict__ rslot,
-                                            const double *__restrict__ rsign, const double *__restrict__ yb,
+                                            const double *__restrict__ rsign, const double *yb,
                                             const double *__restrict__ weight) {
     const int2 sl = reinterpret_cast<const int2 *>(rslot)[r];
     const double2 sg = reinterpret_cast<const double2 *>(rsign)[r];
@@ -281,7 +301,7 @@ template <int K>
 __global__ void __launch_bounds__(256, 2) k_correct_multi(const SubDev *__restrict__ subs,
                                                        const ClusterDev *__restrict__ cl,
                                                        const double *__restrict__ V, const int *__restrict__ bcr,
-                                                       const double *__restrict__ s, double *__restrict__ yb) {
+                                                       const double *s, double *yb) {
     constexpr int QC = 16;                            // V columns per shared-memory chunk
     constexpr int JG = K / 4;                         // case groups (4 cases per thread)
     constexpr int RG = 256 / JG;                      // row groups
@@ -293,11 +313,7 @@ __global__ void __launch_bounds__(256, 2) k_correct_multi(const SubDev *__restri
     if (r0 >= sd.nb) return;
     const int nc = sd.c + 6;
     const int gc_off = cl[sd.cluster].gc_off;
-    for (int o = threadIdx.x; o < nc * K; o += blockDim.x) {
-        const int q = o / K, j = o % K;
-        const int pos = q < sd.c ? bcr[sd.bcr_off + q] : sd.alpha_pos + (q - sd.c);
-        ss[o] = s[((size_t)gc_off + pos) * K + j];
-    }
+    pdl_next();
     const int rend = min(128, sd.nb - r0);
     const int jg = threadIdx.x % JG, rg = threadIdx.x / JG;
     const double *Vd = V + sd.V_off + r0;
@@ -317,6 +333,12 @@ __global__ void __launch_bounds__(256, 2) k_correct_multi(const SubDev *__restri
         }
     };
     fetch(0);
+    pdl_wait();
+    for (int o = threadIdx.x; o < nc * K; o += blockDim.x) {
+        const int q = o / K, j = o % K;
+        const int pos = q < sd.c ? bcr[sd.bcr_off + q] : sd.alpha_pos + (q - sd.c);
+        ss[o] = s[((size_t)gc_off + pos) * K + j];
+    }
     // this thread's y entries, read now so their latency overlaps the products
     double yv[RPT][4];
 #pragma unroll
@@ -366,9 +388,11 @@ template __global__ void k_correct_multi<32>(const SubDev *, const ClusterDev *,
                                              const double *, double *);
 
 __global__ void k_rows_multi(int nlam, int K, const int *__restrict__ rslot, const double *__restrict__ rsign,
-                             const double *__restrict__ yb, const double *__restrict__ weight,
-                             double *__restrict__ out, const double *__restrict__ dotv,
-                             double *__restrict__ partial) {
+                             const double *yb, const double *__restrict__ weight,
+                             double *out, const double *dotv,
+                             double *partial) {
+    pdl_next();
+    pdl_wait();
     const int rows_per_block = 256 / K;
     const int lr = threadIdx.x / K, j = threadIdx.x % K;
     const int stride = gridDim.x * rows_per_block;
@@ -397,47 +421,59 @@ __global__ void k_rows_multi(int nlam, int K, const int *__restrict__ rslot, con
 }
 
 // Gf^T x per chunk and column: partial[ch][q][j].  The chunk's row indices
-// and Gf values are staged in shared memory 256 entries at a time; thread
-// (lr, j) walks every (256/K)-th entry with eight x loads in flight, adding
-// its entries in the order lr, lr + 256/K, ...; the 6 sums are then reduced
-// over lr in one pass through shared memory.
+// and Gf values (up to 1024 entries) are staged in shared memory at once;
+// thread (lr, j) walks every (256/K)-th entry with sixteen x loads in flight,
+// adding its entries in the order lr, lr + 256/K, ...; the 6 sums are then
+// reduced over lr in one pass through shared memory.  Bound by the latency of
+// the x loads, a row of K values each.
+constexpr int GFT_CHUNK = 1024;                    // most entries of a chunk
 __global__ void __launch_bounds__(256) k_gft_partial_multi(int K, const int *__restrict__ chunk_beg,
                                                            const int *__restrict__ chunk_end,
                                                            const int *__restrict__ crow,
                                                            const double *__restrict__ cval,
-                                                           const double *__restrict__ x,
-                                                           double *__restrict__ partial) {
-    __shared__ double red[6 * 256];
-    __shared__ double cs[6 * 256];
-    __shared__ int rs[256];
+                                                           const double *x,
+                                                           double *partial) {
+    extern __shared__ double gft_sm[];
+    double *cs = gft_sm;                            // [6 GFT_CHUNK]; then [6][256] sums
+    int *rs = reinterpret_cast<int *>(gft_sm + 6 * GFT_CHUNK);
     const int ch = blockIdx.x;
     const int j = threadIdx.x % K, nl = 256 / K, lr = threadIdx.x / K;
-    const int beg = chunk_beg[ch], end = chunk_end[ch];
+    const int beg = chunk_beg[ch], n = chunk_end[ch] - beg;
+    pdl_next();
+    const double2 *cv2 = reinterpret_cast<const double2 *>(cval + 6 * (size_t)beg);
+#pragma unroll
+    for (int u = 0; u < GFT_CHUNK / 256; ++u) {
+        const int o = int(threadIdx.x) + 256 * u;
+        if (o < n) rs[o] = crow[beg + o];
+    }
+#pragma unroll
+    for (int u = 0; u < 3 * GFT_CHUNK / 256; ++u) {
+        const int o = int(threadIdx.x) + 256 * u;
+        if (o < 3 * n) reinterpret_cast<double2 *>(cs)[o] = cv2[o];
+    }
+    pdl_wait();
+    __syncthreads();
     double s[6] = {0, 0, 0, 0, 0, 0};
-    for (int e0 = beg; e0 < end; e0 += 256) {
-        const int n = min(256, end - e0);
-        __syncthreads();                            // the previous stage is consumed
-        if (threadIdx.x < n) rs[threadIdx.x] = crow[e0 + threadIdx.x];
-        for (int o = threadIdx.x; o < 6 * n; o += 256) cs[o] = cval[6 * (size_t)e0 + o];
-        __syncthreads();
-        int e = lr;
-        for (; e + 7 * nl < n; e += 8 * nl) {
-            double xv[8];
+    constexpr int U = 16;
+    int e = lr;
+    for (; e + (U - 1) * nl < n; e += U * nl) {
+        double xv[U];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) xv[u] = x[(size_t)rs[e + u * nl] * K + j];
+        for (int u = 0; u < U; ++u) xv[u] = x[(size_t)rs[e + u * nl] * K + j];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const double *cv = cs + 6 * (e + u * nl);
+        for (int u = 0; u < U; ++u) {
+            const double *cv = cs + 6 * (e + u * nl);
 #pragma unroll
-                for (int q = 0; q < 6; ++q) s[q] += cv[q] * xv[u];
-            }
-        }
-        for (; e < n; e += nl) {
-            const double xv = x[(size_t)rs[e] * K + j];
-#pragma unroll
-            for (int q = 0; q < 6; ++q) s[q] += cs[6 * e + q] * xv;
+            for (int q = 0; q < 6; ++q) s[q] += cv[q] * xv[u];
         }
     }
+    for (; e < n; e += nl) {
+        const double xv = x[(size_t)rs[e] * K + j];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) s[q] += cs[6 * e + q] * xv;
+    }
+    __syncthreads();                                // the staged values are consumed
+    double *red = cs;
 #pragma unroll
     for (int q = 0; q < 6; ++q) red[q * 256 + threadIdx.x] = s[q];
     __syncthreads();
@@ -452,39 +488,42 @@ __global__ void __launch_bounds__(256) k_gft_partial_multi(int K, const int *__r
         for (int q = 0; q < 6; ++q) partial[((size_t)ch * 6 + q) * K + j] = red[q * 256 + j];
 }
 
-// gt[c][i][j] = sum of the chunk partials of cluster c (fixed order); CTA per
-// cluster, thread (i, j)
-__global__ void k_gt_sum_multi(int K, const int *__restrict__ cl_chunk_ptr, const double *__restrict__ gpart,
-                               double *__restrict__ gt) {
-    const int c = blockIdx.x;
-    for (int o = threadIdx.x; o < 6 * K; o += blockDim.x) {
-        const int i = o / K, j = o % K;
-        double s = 0.0;
-        for (int chk = cl_chunk_ptr[c]; chk < cl_chunk_ptr[c + 1]; ++chk) s += gpart[((size_t)chk * 6 + i) * K + j];
-        gt[((size_t)c * 6 + i) * K + j] = s;
-    }
+// gt[c][i][j] = sum of the chunk partials of cluster c (in chunk order); CTA
+// (cluster, mode i), thread j
+__global__ void k_gt_sum_multi(int K, const int *__restrict__ cl_chunk_ptr, const double *gpart,
+                               double *gt) {
+    pdl_next();
+    pdl_wait();
+    const int c = blockIdx.x / 6, i = blockIdx.x % 6, j = threadIdx.x;
+    double s = 0.0;
+#pragma unroll 8
+    for (int chk = cl_chunk_ptr[c]; chk < cl_chunk_ptr[c + 1]; ++chk) s += gpart[((size_t)chk * 6 + i) * K + j];
+    gt[(size_t)blockIdx.x * K + j] = s;
 }
 
-// a = (Gf^T Gf)^{-1} gt per column (gt = Gf^T x from k_gt_sum_multi); one
-// CTA; alpha_out = -a when requested.
-__global__ void k_gf_coef_multi(int K, int ncl, const double *__restrict__ invGtG, const double *__restrict__ gt,
-                                double *__restrict__ a, double *__restrict__ alpha_out) {
-    const int m = 6 * ncl;
-    for (int o = threadIdx.x; o < m * K; o += blockDim.x) {
-        const int q = o / K, j = o % K;
-        double s = 0.0;
-        for (int p = 0; p < m; ++p) s += invGtG[q + (size_t)p * m] * gt[p * K + j];
-        a[o] = s;
-        if (alpha_out) alpha_out[o] = -s;
-    }
+// a = (Gf^T Gf)^{-1} gt per column (gt = Gf^T x from k_gt_sum_multi), CTA per
+// row, thread per column; alpha_out = -a when requested.  (All rows in one
+// CTA: 23.7 us for 8 clusters and 32 load cases, 2.9 us here.)
+__global__ void k_gf_coef_multi(int K, int ncl, const double *__restrict__ invGtG, const double *gt,
+                                double *a, double *alpha_out) {
+    pdl_next();
+    pdl_wait();
+    const int m = 6 * ncl, q = blockIdx.x, j = threadIdx.x;
+    double s = 0.0;
+#pragma unroll 16
+    for (int p = 0; p < m; ++p) s += invGtG[q + (size_t)p * m] * gt[(size_t)p * K + j];
+    a[(size_t)q * K + j] = s;
+    if (alpha_out) alpha_out[(size_t)q * K + j] = -s;
 }
 
 // Px = x - Gf a; partial dot with dotv per (block, j); blocks stride over
 // row groups like k_rows_multi
-__global__ void k_gf_apply_multi(int nlam, int K, const double *__restrict__ a, const int *__restrict__ gcl,
-                                 const double *__restrict__ gval, const double *__restrict__ x,
-                                 double *__restrict__ Px, const double *__restrict__ dotv,
-                                 double *__restrict__ partial) {
+__global__ void k_gf_apply_multi(int nlam, int K, const double *a, const int *__restrict__ gcl,
+                                 const double *__restrict__ gval, const double *x,
+                                 double *Px, const double *dotv,
+                                 double *partial) {
+    pdl_next();
+    pdl_wait();
     const int rows_per_block = 256 / K;
     const int lr = threadIdx.x / K, j = threadIdx.x % K;
     double prod = 0.0;
@@ -524,15 +563,19 @@ __device__ double col_sum(const double *partial, int np, int K, int j) {
 }
 
 // per column: scalar = sum of partials -> out[j]
-__global__ void k_colsum(const double *__restrict__ partial, int np, int K, double *__restrict__ out) {
+__global__ void k_colsum(const double *partial, int np, int K, double *out) {
+    pdl_next();
+    pdl_wait();
     const double s = col_sum(partial, np, K, blockIdx.x);
     if (threadIdx.x == 0) out[blockIdx.x] = s;
 }
 
 // rho_j = -gPz_j / wFw_j ; lam += rho w ; g += rho Fw  (skips finished columns)
-__global__ void k_update_lam_g_multi(int n, int K, const double *__restrict__ wFw, const double *__restrict__ gw,
-                                     const double *__restrict__ w, const double *__restrict__ Fw,
-                                     double *__restrict__ lam, double *__restrict__ g, PcpgState *__restrict__ st) {
+__global__ void k_update_lam_g_multi(int n, int K, const double *wFw, const double *gw,
+                                     const double *w, const double *Fw,
+                                     double *lam, double *g, PcpgState *st) {
+    pdl_next();
+    pdl_wait();
     const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (id >= (long long)n * K) return;
     const int j = int(id % K);
@@ -549,8 +592,10 @@ __global__ void k_update_lam_g_multi(int n, int K, const double *__restrict__ wF
 
 // partial[blk][j] = sum over the rows of block blk of a[r][j] * b[r][j]
 // (row groups of 256 / K rows, strided like k_rows_multi)
-__global__ void k_dot_multi(int nlam, int K, const double *__restrict__ a, const double *__restrict__ b,
-                            double *__restrict__ partial) {
+__global__ void k_dot_multi(int nlam, int K, const double *a, const double *b,
+                            double *partial) {
+    pdl_next();
+    pdl_wait();
     const int rows_per_block = 256 / K;
     const int lr = threadIdx.x / K, j = threadIdx.x % K;
     double prod = 0.0;
@@ -561,8 +606,10 @@ __global__ void k_dot_multi(int nlam, int K, const double *__restrict__ a, const
     block_col_partial(prod, K, partial);
 }
 
-__global__ void k_update_w_multi(int n, int K, const double *__restrict__ gPz_new, const double *__restrict__ Pz,
-                                 double *__restrict__ w, const PcpgState *__restrict__ st) {
+__global__ void k_update_w_multi(int n, int K, const double *gPz_new, const double *Pz,
+                                 double *w, const PcpgState *st) {
+    pdl_next();
+    pdl_wait();
     const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (id >= (long long)n * K) return;
     const int j = int(id % K);
@@ -571,8 +618,10 @@ __global__ void k_update_w_multi(int n, int K, const double *__restrict__ gPz_ne
 }
 
 // hist (FP64 form): relative residual of column j after iteration it at hist[it * K + j]
-__global__ void k_finish_multi(int K, const double *__restrict__ wFw, const double *__restrict__ gPz_new,
-                               PcpgState *__restrict__ st, double *__restrict__ hist) {
+__global__ void k_finish_multi(int K, const double *wFw, const double *gPz_new,
+                               PcpgState *st, double *hist) {
+    pdl_next();
+    pdl_wait();
     const int j = threadIdx.x;
     if (j >= K || st[j].done) return;
     const double gPz = gPz_new[j];
@@ -616,56 +665,75 @@ namespace htf {
 
 // rows [32 I, 32 I + 32) of A X for the symmetric A of nt tile rows packed at
 // base, X = x (RHS-interleaved, rows < nx; zero beyond): acc[q] = this
-// thread's entries of row 8 band + g, columns 8 (cb0 + q) + 2 t4, + 1
+// thread's entries of row 8 band + g, columns 8 (cb0 + q) + 2 t4, + 1.  Tiles
+// and X pieces are double-buffered in shared memory (one barrier each) and
+// prefetched two ahead into registers; a tile above the diagonal is stored as
+// it is and read transposed by the fragments.
 template <int K>
 __device__ __forceinline__ void sym_rows_product(const double *__restrict__ base, int nt, int I, const double *x,
                                                  int nx, double (&acc)[K / 16][2]) {
     constexpr int NT = K / 16;                      // 8x8 output tiles per warp
     constexpr int TS = 36, XS = K + 4;              // row strides (doubles): conflict-free fragment loads
-    __shared__ double Ts[32 * TS];
-    __shared__ double Xs[32 * XS];
+    constexpr int TU = TILE_ELEMS / 256, XU = TILE * K / 256;
+    __shared__ double Ts[2][32 * TS];
+    __shared__ double Xs[2][32 * XS];
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int g = lane >> 2, t4 = lane & 3;         // fragment row / column groups
     const int band = warp & 3, cb0 = (warp >> 2) * NT;
 #pragma unroll
     for (int q = 0; q < NT; ++q) acc[q][0] = acc[q][1] = 0.0;
-    double tr[TILE_ELEMS / 256], xr[TILE * K / 256];
-    auto fetch = [&](int J) {
+    double ta[TU], tb[TU], xa[XU], xc[XU];
+    auto fetch_t = [&](double (&tr)[TU], int J) {
         const double *tp = base + (J <= I ? (long long)I * (I + 1) / 2 + J : (long long)J * (J + 1) / 2 + I) * TILE_ELEMS;
 #pragma unroll
-        for (int u = 0; u < TILE_ELEMS / 256; ++u) tr[u] = tp[threadIdx.x + 256 * u];
+        for (int u = 0; u < TU; ++u) tr[u] = tp[threadIdx.x + 256 * u];
+    };
+    auto fetch_x = [&](double (&xr)[XU], int J) {
 #pragma unroll
-        for (int u = 0; u < TILE * K / 256; ++u) {
+        for (int u = 0; u < XU; ++u) {
             const int e = threadIdx.x + 256 * u, r = TILE * J + e / K;
             xr[u] = r < nx ? x[(size_t)r * K + e % K] : 0.0;
         }
     };
-    fetch(0);
-    for (int J = 0; J < nt; ++J) {
-        const bool lower = J <= I;
+    auto tile = [&](double (&tr)[TU], double (&xr)[XU], int J) {
+        double *T = Ts[J & 1], *X = Xs[J & 1];
 #pragma unroll
-        for (int u = 0; u < TILE_ELEMS / 256; ++u) {
-            const int e = threadIdx.x + 256 * u, rr = e / TILE, cc = e % TILE;
-            if (lower) Ts[rr * TS + cc] = tr[u];    // stored tile (I, J): A[32I + rr][32J + cc]
-            else Ts[cc * TS + rr] = tr[u];          // tile (J, I): A[32I + cc][32J + rr]
+        for (int u = 0; u < TU; ++u) {
+            const int e = threadIdx.x + 256 * u;
+            T[(e / TILE) * TS + e % TILE] = tr[u];
         }
 #pragma unroll
-        for (int u = 0; u < TILE * K / 256; ++u) {
+        for (int u = 0; u < XU; ++u) {
             const int e = threadIdx.x + 256 * u;
-            Xs[(e / K) * XS + e % K] = xr[u];
+            X[(e / K) * XS + e % K] = xr[u];
         }
         __syncthreads();
-        if (J + 1 < nt) fetch(J + 1);               // in flight during the products
+        if (J + 2 < nt) {
+            fetch_t(tr, J + 2);
+            fetch_x(xr, J + 2);
+        }
+        const bool lower = J <= I;                  // tile (I, J): A[32I + r][32J + c]; else (J, I), transposed
+        const double *Ta = T + (lower ? (8 * band + g) * TS + t4 : t4 * TS + 8 * band + g);
+        const int step = lower ? 4 : 4 * TS;
 #pragma unroll
         for (int kk = 0; kk < TILE / 4; ++kk) {
-            const double a = Ts[(8 * band + g) * TS + 4 * kk + t4];
+            const double a = Ta[kk * step];
 #pragma unroll
             for (int q = 0; q < NT; ++q) {
-                const double bq = Xs[(4 * kk + t4) * XS + 8 * (cb0 + q) + g];
+                const double bq = X[(4 * kk + t4) * XS + 8 * (cb0 + q) + g];
                 dmma_8x8x4(acc[q][0], acc[q][1], a, bq);
             }
         }
-        __syncthreads();
+    };
+    pdl_next();
+    fetch_t(ta, 0);
+    if (nt > 1) fetch_t(tb, 1);
+    pdl_wait();
+    fetch_x(xa, 0);
+    if (nt > 1) fetch_x(xc, 1);
+    for (int J = 0; J < nt; J += 2) {
+        tile(ta, xa, J);
+        if (J + 1 < nt) tile(tb, xc, J + 1);
     }
 }
 
@@ -673,11 +741,11 @@ template <int K>
 __global__ void __launch_bounds__(256) k_symv_rows_multi(const int2 *__restrict__ rowblk,
                                                          const SubDev *__restrict__ subs,
                                                          const double *__restrict__ tiles,
-                                                         const double *__restrict__ xb, double *__restrict__ yb,
+                                                         const double *xb, double *yb,
                                                          const ClusterDev *__restrict__ cl,
                                                          const double *__restrict__ Vbuf,
                                                          const int *__restrict__ bcrows,
-                                                         const double *__restrict__ s) {
+                                                         const double *s) {
     constexpr int NT = K / 16;
     const int2 rb = rowblk[blockIdx.x];
     const SubDev &sd = subs[rb.x];
@@ -721,8 +789,8 @@ template __global__ void k_symv_rows_multi<32>(const int2 *, const SubDev *, con
 template <int K>
 __global__ void __launch_bounds__(256) k_msym_rows_multi(const int2 *__restrict__ mt,
                                                          const ClusterDev *__restrict__ cl,
-                                                         const double *__restrict__ T, const double *__restrict__ gc,
-                                                         double *__restrict__ s) {
+                                                         const double *__restrict__ T, const double *gc,
+                                                         double *s) {
     constexpr int NT = K / 16;
     const int2 b = mt[blockIdx.x];
     const ClusterDev c = cl[b.x];
@@ -756,7 +824,7 @@ __global__ void k_cols_copy(long long n, int K, const int *__restrict__ mask, co
 
 // per-column alpha (m values per column, column-major) of the columns with
 // mask[j] from the projector's K-interleaved output
-__global__ void k_alpha_cols(int m, int K, const int *__restrict__ mask, const double *__restrict__ a,
+__global__ void k_alpha_cols(int m, int K, const int *__restrict__ mask, const double *a,
                              double *__restrict__ alpha) {
     for (int o = threadIdx.x; o < m * K; o += blockDim.x) {
         const int q = o / K, j = o % K;

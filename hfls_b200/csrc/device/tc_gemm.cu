@@ -180,6 +180,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_tc_gemm(const GemmBlock *__re
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base;
+    pdl_next();
+    pdl_wait();                                            // X slabs and their scales; yb's readers
 
     if (warp == 0) {
         if (lane == 0) {                                  // producer
