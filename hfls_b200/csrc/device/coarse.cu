@@ -26,7 +26,7 @@ namespace htf {
 
 __global__ void k_potrf_diag(const StepDesc *, const SubDev *, double *, int *);
 __global__ void k_trsm_panel(const StepDesc *, int, const SubDev *, double *, const int *);
-__global__ void k_syrk_update(const StepDesc *, int, const SubDev *, double *, const int *);
+__global__ void k_syrk_update(const StepDesc *, int, int, const SubDev *, double *, const int *, int *);
 cudaError_t ksolve_multi_launch(const SubDev *, const int *, int, const double *, double *, long long, int, const int *,
                                 int, int, int *, cudaStream_t);
 __global__ void k_build_Fc(const SubDev *, const double *, const int *, const int *, const double *,
@@ -229,7 +229,7 @@ int cdivc(long long a, long long b) { return int((a + b - 1) / b); }
 
 // Launches the batched Cholesky of the matrices described by hm / dm (N, K_off).
 static cudaError_t chol_batched(const std::vector<SubDev> &hm, const SubDev *dm, double *buf, int *status,
-                                DevTmp &tmp, cudaStream_t s) {
+                                DevTmp &tmp, int *kserr, cudaStream_t s) {
     std::vector<std::vector<StepDesc>> steps;
     chol_steps(hm, steps);
     std::vector<StepDesc> flat;
@@ -238,8 +238,8 @@ static cudaError_t chol_batched(const std::vector<SubDev> &hm, const SubDev *dm,
     for (auto &v : steps) {
         int tri = 0, rb = 0;
         for (auto &x : v) {
-            const int rows = hm[x.d].N - x.k - x.nb, nbr = (rows + 63) / 64;
-            x.tri0 = tri; tri += nbr * (nbr + 1) / 2;
+            const int rows = hm[x.d].N - x.k - x.nb;
+            x.tri0 = tri; tri += syrk_tiles(rows);
             x.rb0 = rb; rb += (rows + 127) / 128;
         }
         ntri.push_back(tri);
@@ -268,7 +268,9 @@ static cudaError_t chol_batched(const std::vector<SubDev> &hm, const SubDev *dm,
         const int cnt = int(steps[st].size());
         k_potrf_diag<<<cnt, CHOL_STEP, 0, s>>>(d + off[st], dm, buf, status);
         if (nrb[st] > 0) k_trsm_panel<<<nrb[st], 128, 0, s>>>(d + off[st], cnt, dm, buf, dh + hrb[st]);
-        if (ntri[st] > 0) k_syrk_update<<<ntri[st], 256, SYRK_SMEM, s>>>(d + off[st], cnt, dm, buf, dh + htri[st]);
+        if (ntri[st] > 0)
+            k_syrk_update<<<std::min(ntri[st], 148), SYRK_THREADS, SYRK_SMEM, s>>>(d + off[st], cnt, ntri[st], dm, buf,
+                                                                                dh + htri[st], kserr);
     }
     return cudaGetLastError();
 }
@@ -483,7 +485,7 @@ int Engine::coarse(Problem &p, std::string &err) {
     CKC(cudaMemcpyAsync(dmF, mF.data(), ncl_ * sizeof(SubDev), cudaMemcpyHostToDevice, s_));
     CKC(cudaMemcpyAsync(dmS, mS.data(), ncl_ * sizeof(SubDev), cudaMemcpyHostToDevice, s_));
     CKC(copy_batched(cp, tmp, s_));
-    CKC(chol_batched(mF, dmF, dF, dst, tmp, s_));
+    CKC(chol_batched(mF, dmF, dF, dst, tmp, d_kserr_, s_));
     CKC(solve_batched(mF, dmF, dF, dW, colsW, tmp, d_kserr_, s_));               // [Z | Fi]
     std::vector<GemmDesc> gm;
     for (int c = 0; c < ncl_; ++c) {                                     // Sr = Gc^T Z + H H^T
@@ -498,7 +500,7 @@ int Engine::coarse(Problem &p, std::string &err) {
         CKC(gemm_batched(a, tmp, s_));
         CKC(gemm_batched(b, tmp, s_));
     }
-    CKC(chol_batched(mS, dmS, dS, dst + ncl_, tmp, s_));
+    CKC(chol_batched(mS, dmS, dS, dst + ncl_, tmp, d_kserr_, s_));
     CKC(solve_batched(mS, dmS, dS, dSi, colsS, tmp, d_kserr_, s_));              // Si = Sr^{-1}
     gm.clear();
     for (int c = 0; c < ncl_; ++c) {                                     // ZS = Z Si

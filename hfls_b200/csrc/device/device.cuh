@@ -39,9 +39,17 @@ __device__ __forceinline__ int tc_scale_exp(unsigned m_bits, float mult) {
 
 constexpr int TILE = 32;                  // packed tile edge
 constexpr int CHOL_STEP = 64;             // columns per batched Cholesky step (two factor panels)
-// dynamic shared memory of k_syrk_update: two 32-column panels of 64 rows for
-// each operand (row stride 68) and the 64 x 64 C block (column stride 65)
-constexpr int SYRK_SMEM = (4 * 32 * 68 + 64 * 65) * 8;
+// k_syrk_update: threads (eight product warps, four copy warps), two stages of
+// CHOL_STEP panel columns of 128 + 64 rows (strides 132 and 68), tiles of a
+// trailing matrix of `rows` rows (128-row blocks bi with column blocks of 64
+// up to the diagonal's)
+constexpr int SYRK_COPY_WARPS = 4;
+constexpr int SYRK_THREADS = 256 + 32 * SYRK_COPY_WARPS;
+constexpr int SYRK_SMEM = 2 * CHOL_STEP * (132 + 68) * 8;
+inline int syrk_tiles(int rows) {
+    const int nbr = (rows + 127) / 128;
+    return nbr * (nbr + 1) - (rows > 0 && (rows - 1) % 128 < 64 ? 1 : 0);
+}
 constexpr int TC_STAGES = 5;              // pipeline stages of the tensor-core product (2 CTAs per SM)
 constexpr int TC_THREADS = 320;           // threads of the tensor-core product: producer, MMA, 8 epilogue warps
 constexpr int TILE_ELEMS = TILE * TILE;
@@ -176,7 +184,7 @@ struct TcSet {
 
 // One step of the batched Cholesky for one subdomain: columns [k, k + nb),
 // nb <= CHOL_STEP, starting at a factor panel and covering at most two.
-// tri0 / rb0: first trailing 64x64 tile / first 128-row block of this entry
+// tri0 / rb0: first trailing 128x64 tile / first 128-row block of this entry
 // in the step's flattened SYRK / panel-solve grid (prefix sums over the step's
 // entries, so the grids have no idle CTAs whatever the subdomain sizes).
 struct StepDesc {

@@ -20,7 +20,7 @@ __global__ void k_assemble(const int *, int, const double *, const int *, const 
 __global__ void k_regularize(SubDev *, int, double *);
 __global__ void k_potrf_diag(const StepDesc *, const SubDev *, double *, int *);
 __global__ void k_trsm_panel(const StepDesc *, int, const SubDev *, double *, const int *);
-__global__ void k_syrk_update(const StepDesc *, int, const SubDev *, double *, const int *);
+__global__ void k_syrk_update(const StepDesc *, int, int, const SubDev *, double *, const int *, int *);
 __global__ void k_snapshot(const int *, const SubDev *, const double *, double *, long long);
 __global__ void k_make_slabs(const GemmBlock *, const SubDev *, const double *, float *, long long,
                              const unsigned *);
@@ -630,8 +630,8 @@ int Engine::factorize(Problem &p, std::string &err) {
         for (auto &v : steps) {
             int tri = 0, rb = 0;
             for (auto &x : v) {
-                const int rows = hs_[x.d].N - x.k - x.nb, nbr = (rows + 63) / 64;
-                x.tri0 = tri; tri += nbr * (nbr + 1) / 2;
+                const int rows = hs_[x.d].N - x.k - x.nb;
+                x.tri0 = tri; tri += syrk_tiles(rows);
                 x.rb0 = rb; rb += (rows + 127) / 128;
             }
             W.cnt.push_back(int(v.size()));
@@ -734,7 +734,8 @@ void Engine::factor_wave(int w, bool build, double *X) {
         k_potrf_diag<<<cnt, CHOL_STEP, 0, s_>>>(ds, d_subs_, d_K_, d_status_);
         if (W.nrb[s] > 0) k_trsm_panel<<<W.nrb[s], 128, 0, s_>>>(ds, cnt, d_subs_, d_K_, W.hints + W.hrb[s]);
         if (W.ntri[s] > 0)
-            k_syrk_update<<<W.ntri[s], 256, SYRK_SMEM, s_>>>(ds, cnt, d_subs_, d_K_, W.hints + W.htri[s]);
+            k_syrk_update<<<std::min(W.ntri[s], 148), SYRK_THREADS, SYRK_SMEM, s_>>>(ds, cnt, W.ntri[s], d_subs_, d_K_,
+                                                                              W.hints + W.htri[s], d_kserr_);
         if (build && dirichlet && W.nsnap[s] > 0)
             k_snapshot<<<dim3(W.nsnap[s], max_tiles_), 256, 0, s_>>>(W.snap + W.snap_off[s], d_subs_, d_K_, d_S_,
                                                                      st0);

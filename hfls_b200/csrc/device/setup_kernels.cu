@@ -20,6 +20,8 @@
 #include <cstdint>
 
 #include "device.cuh"
+#include "htfeti.h"
+#include "mbar.cuh"
 
 namespace htf {
 
@@ -273,18 +275,27 @@ __global__ void __launch_bounds__(128) k_trsm_panel(const StepDesc *__restrict__
         if (j < nb) Kbuf[(j < TILE ? c0 + (long long)j * ld0 : c1 + (long long)(j - TILE) * ld1) + row] = x[j];
 }
 
-// C(64x64 block, lower part of the trailing matrix) -= P_i P_j^T, P = the
-// step's panel rows; 32 columns of P at a time, one accumulator per panel,
-// C read and written once.  The products run on the FP64 tensor path
-// (mma.sync m8n8k4 .f64): warp w owns rows 32 (w / 4) .. +31 and columns
-// 16 (w % 4) .. +15 of the block, 4 x 2 tiles of 8 x 8, so per k-group of 4
-// a warp loads 6 operand fragments for 8 MMAs (the CUDA-core form loaded 8
-// values per 16 FMAs per thread and was bound by shared-memory loads).  A
-// row stride of 68 doubles keeps both fragment loads free of bank
-// conflicts.  All loads are cp.async into shared memory, issued at the start
-// in three groups (panel 0, panel 1, the C block), so panel 1 and C land
-// while panel 0 multiplies.  grid: the step's trailing tiles (flattened);
-// dynamic shared memory SYRK_SMEM.
+// C (128 x 64 tile of the lower part of the trailing matrix) -= P_i P_j^T, P =
+// the step's panel rows: 32 columns of P at a time, one sum per panel,
+// subtracted in turn, C read and written once.
+//
+// Persistent: one CTA per SM of eight product warps and four copy warps, which
+// run through the step's tiles (CTA c takes tiles c, c + CTAs, ..).  The copy
+// warps find the next tile and bring its panel rows (cp.async of 8 bytes: a
+// column starts at any double) into one of two shared-memory stages while the
+// product warps work on the other, C going straight to registers at the
+// start of a tile and back from there; a tile's table look-ups, copies and C
+// traffic thus hide behind the products of the tile before.  Products on the
+// FP64 tensor path (mma.sync m8n8k4 .f64): warp w owns rows 32 (w / 2) .. +31
+// and columns 32 (w % 2) .. +31, 4 x 4 tiles of 8 x 8, so a k-group of 4 is 8
+// fragment loads for 16 MMAs; row strides of 132 and 68 doubles keep them
+// free of bank conflicts.  C's loads are pinned to the start of the tile
+// (left to the compiler they sink to their use: 128 ms).  One CTA per 64 x 64
+// tile, with nothing in flight while it multiplied, reached 9.5 TFLOP/s on
+// 512 x 2 187 DOFs (189 ms in all), this 16.5 (108 ms); 64 uneven subdomains
+// of up to 5 577 DOFs 104 -> 59 ms.  The products alone would take 56 and 33
+// ms at the FP64 tensor rate (36 TFLOP/s); the rest is C through fragments of
+// 64 contiguous bytes.
 __device__ __forceinline__ void dmma_syrk(double &d0, double &d1, double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                  : "+d"(d0), "+d"(d1)
@@ -299,107 +310,162 @@ __device__ __forceinline__ void cp_async8(double *dst, const double *src, int sr
                  : "memory");
 }
 
-__global__ void __launch_bounds__(256) k_syrk_update(const StepDesc *__restrict__ st, int cnt,
-                                                     const SubDev *__restrict__ subs,
-                                                     double *__restrict__ Kbuf, const int *__restrict__ hint) {
-    constexpr int LDP = 68, LDC = 65;
-    extern __shared__ double syrk_sm[];
-    double(*Pa)[32][LDP] = reinterpret_cast<double(*)[32][LDP]>(syrk_sm);                 // [2][32][LDP]
-    double(*Pb)[32][LDP] = reinterpret_cast<double(*)[32][LDP]>(syrk_sm + 2 * 32 * LDP);  // [2][32][LDP]
-    double *Cs = syrk_sm + 4 * 32 * LDP;                                                    // [64 cols][LDC]
-    const int e = step_entry(st, cnt, int(blockIdx.x), [](const StepDesc &x) { return x.tri0; }, hint);
-    const StepDesc s = st[e];
-    const SubDev &sd = subs[s.d];
-    const int N = sd.N, k = s.k, nb = s.nb;
-    const int t0 = k + nb;                  // first trailing row/col
-    const int m = N - t0;
-    const int nbr = (m + 63) / 64;
-    const int tri = int(blockIdx.x) - s.tri0;
-    if (tri >= nbr * (nbr + 1) / 2) return;
-    int bi = (int)((sqrt(8.0 * tri + 1.0) - 1.0) * 0.5);
-    while ((bi + 1) * (bi + 2) / 2 <= tri) ++bi;
-    while (bi * (bi + 1) / 2 > tri) --bi;
-    const int bj = tri - bi * (bi + 1) / 2;
-    const int i0 = t0 + 64 * bi, j0 = t0 + 64 * bj;
+// *p, or zero: issued here, not where the value is used
+__device__ __forceinline__ double ld_now(const double *p, bool in) {
+    double v;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %2, 0;\n\t"
+        "mov.f64 %0, 0d0000000000000000;\n\t"
+        "@q ld.global.f64 %0, [%1];\n\t}"
+        : "=d"(v)
+        : "l"(p), "r"(int(in)));
+    return v;
+}
+
+constexpr int SYRK_LDA = 132, SYRK_LDB = 68;
+constexpr int SYRK_STAGE = CHOL_STEP * (SYRK_LDA + SYRK_LDB);       // doubles: A columns, then B columns
+
+struct SyrkTile {
+    int d, k, nb, i0, j0;                   // subdomain, step, first row and column of the tile; d < 0: no more
+};
+
+__global__ void __launch_bounds__(SYRK_THREADS, 1) k_syrk_update(const StepDesc *__restrict__ st, int cnt, int tiles,
+                                                                 const SubDev *__restrict__ subs, double *Kbuf,
+                                                                 const int *__restrict__ hint, int *__restrict__ err) {
+    extern __shared__ __align__(16) double syrk_sm[];                // two stages
+    __shared__ __align__(8) uint64_t full[2], empty[2];
+    __shared__ SyrkTile desc[2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane >> 2, t4 = lane & 3;
-    const int wr = 32 * (warp >> 2), wc = 16 * (warp & 3);
-    const int nq = (nb + TILE - 1) / TILE;
-    // groups 0, 1: the panels of the step's 32-column halves (zero outside)
-#pragma unroll
-    for (int q = 0; q < CHOL_STEP / TILE; ++q) {
-        if (q >= nq) break;
-        const int kc = TILE * q;
-        const int kn = min(TILE, nb - kc);
-        const double *P = Kbuf + kidx(sd, k + kc, k + kc);    // panel of columns k+kc..: entry (k+kc+i, k+kc+j) at P[i + j*ld]
-        const long long ld = kld(sd, k + kc);
-        for (int idx = threadIdx.x; idx < 32 * 64; idx += 256) {
-            const int r = idx % 64, kk = idx / 64;
-            const bool oka = kk < kn && i0 + r < N, okb = kk < kn && j0 + r < N;
-            cp_async8(&Pa[q][kk][r], oka ? P + (i0 + r - k - kc) + kk * ld : Kbuf, oka ? 8 : 0);
-            cp_async8(&Pb[q][kk][r], okb ? P + (j0 + r - k - kc) + kk * ld : Kbuf, okb ? 8 : 0);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    // last group: the lower part of the C block (rows >= columns, inside the
-    // matrix), needed only after the products
-    for (int idx = threadIdx.x; idx < 64 * 64; idx += 256) {
-        const int r = idx % 64, c = idx / 64;
-        const int row = i0 + r, col = j0 + c;
-        const bool ok = row < N && col < N && row >= col;
-        cp_async8(&Cs[c * LDC + r], ok ? Kbuf + kcol(sd, col) + row : Kbuf, ok ? 8 : 0);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    double acc[CHOL_STEP / TILE][4][2][2];
-#pragma unroll
-    for (int q = 0; q < CHOL_STEP / TILE; ++q)
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 2; ++b) acc[q][a][b][0] = acc[q][a][b][1] = 0.0;
-#pragma unroll
-    for (int q = 0; q < CHOL_STEP / TILE; ++q) {
-        if (q >= nq) break;
-        // panel q (and everything committed before it) has landed; the later
-        // panel and the C block may still be in flight
-        if (q + 1 < nq) asm volatile("cp.async.wait_group 2;" ::: "memory");
-        else asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();
-        const int kn = min(TILE, nb - TILE * q);
-        const int kgs = (kn + 3) >> 2;
-        for (int kg = 0; kg < kgs; ++kg) {
-            const int kr = 4 * kg + t4;
-            double av[4], bv[2];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) av[a] = Pa[q][kr][wr + 8 * a + g];
-#pragma unroll
-            for (int b = 0; b < 2; ++b) bv[b] = Pb[q][kr][wc + 8 * b + g];
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int b = 0; b < 2; ++b) dmma_syrk(acc[q][a][b][0], acc[q][a][b][1], av[a], bv[b]);
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < 2; ++q) {
+            mbar_init(&full[q], 32 * SYRK_COPY_WARPS + 1);     // the copy warps' lanes, the tile's description
+            mbar_init(&empty[q], 8);
         }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");    // the C block
     __syncthreads();
-#pragma unroll
-    for (int b = 0; b < 2; ++b)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int cl = wc + 8 * b + 2 * t4 + h, col = j0 + cl;
-            if (col >= N) continue;
-            double *C = Kbuf + kcol(sd, col);
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                const int rl = wr + 8 * a + g, row = i0 + rl;
-                if (row >= N || row < col) continue;
-                double c = Cs[cl * LDC + rl];
-#pragma unroll
-                for (int q = 0; q < CHOL_STEP / TILE; ++q)
-                    if (q < nq) c -= acc[q][a][b][h];
-                C[row] = c;
+    bool ok = true;
+    // registers: 12 warps of 168 at launch, then 8 of 216 and 4 of 72 (the same sum)
+    if (warp >= 8) {                        // copies: every SYRK_COPY_WARPS-th column
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+        int n = 0;
+        for (int t = blockIdx.x; ok; t += gridDim.x, ++n) {
+            const int q = n & 1;
+            SyrkTile T{-1, 0, 0, 0, 0};
+            if (t < tiles) {
+                const StepDesc s = st[step_entry(st, cnt, t, [](const StepDesc &x) { return x.tri0; }, hint)];
+                // row block bi (128 rows) has column blocks (64) 0 .. 2 bi + 1: bi (bi + 1) tiles before it
+                const int tri = t - s.tri0;
+                int bi = (int)((sqrt(4.0 * tri + 1.0) - 1.0) * 0.5);
+                while ((bi + 1) * (bi + 2) <= tri) ++bi;
+                while (bi * (bi + 1) > tri) --bi;
+                T = SyrkTile{s.d, s.k, s.nb, s.k + s.nb + 128 * bi, s.k + s.nb + 64 * (tri - bi * (bi + 1))};
             }
+            if (n >= 2) ok = mbar_wait(&empty[q], ((n >> 1) - 1) & 1);
+            if (!ok) break;
+            if (warp == 8 && lane == 0) desc[q] = T;
+            if (T.d >= 0) {
+                const SubDev &sd = subs[T.d];
+                const int N = sd.N;
+                double *A = syrk_sm + q * SYRK_STAGE, *B = A + CHOL_STEP * SYRK_LDA;
+                for (int kc = 0; kc < T.nb; kc += TILE) {
+                    // panel of columns k + kc ..: entry (row, k + kc + c) at P[row + c ld]
+                    const double *P = Kbuf + kcol(sd, T.k + kc);
+                    const long long ld = kld(sd, T.k + kc);
+                    const int kn = min(TILE, T.nb - kc);
+#pragma unroll 4
+                    for (int c = warp - 8; c < TILE; c += SYRK_COPY_WARPS) {
+                        const double *col = P + c * ld;
+#pragma unroll
+                        for (int r = 0; r < 128; r += 32) {
+                            const bool in = c < kn && T.i0 + r + lane < N;
+                            cp_async8(A + (kc + c) * SYRK_LDA + r + lane, in ? col + T.i0 + r + lane : Kbuf, in ? 8 : 0);
+                        }
+#pragma unroll
+                        for (int r = 0; r < 64; r += 32) {
+                            const bool in = c < kn && T.j0 + r + lane < N;
+                            cp_async8(B + (kc + c) * SYRK_LDB + r + lane, in ? col + T.j0 + r + lane : Kbuf, in ? 8 : 0);
+                        }
+                    }
+                }
+            }
+            if (warp == 8 && lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full[q])) : "memory");
+            // each lane's arrival comes once its copies into this stage have landed
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[q])) : "memory");
+            if (T.d < 0) break;
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+        const int g = lane >> 2, t4 = lane & 3;
+        const int wr = 32 * (warp >> 1), wc = 32 * (warp & 1);
+        for (int n = 0;; ++n) {
+            const int q = n & 1;
+            ok = mbar_wait(&full[q], (n >> 1) & 1);
+            if (!ok) break;
+            const SyrkTile T = desc[q];
+            if (T.d < 0) break;
+            const SubDev &sd = subs[T.d];
+            const int N = sd.N;
+            const double *A = syrk_sm + q * SYRK_STAGE, *B = A + CHOL_STEP * SYRK_LDA;
+            // this thread's C: rows i0 + wr + 8 a + g, columns j0 + wc + 8 b + 2 t4 + h (lower part, in range)
+            double *C[4][2];
+            double c[4][4][2];
+            int last[4][2];                 // rows row0 + 8 a of the column are stored for first <= row0 + 8 a < N
+            const int row0 = T.i0 + wr + g;
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int col = T.j0 + wc + 8 * b + 2 * t4 + h;
+                    C[b][h] = Kbuf + kcol(sd, min(col, N - 1)) + row0;
+                    last[b][h] = col < N ? col : N;
+#pragma unroll
+                    for (int a = 0; a < 4; ++a)
+                        c[a][b][h] = ld_now(C[b][h] + 8 * a, row0 + 8 * a >= last[b][h] && row0 + 8 * a < N);
+                }
+            for (int kc = 0; kc < T.nb; kc += TILE) {
+                double acc[4][4][2];
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+                const int kgs = (min(TILE, T.nb - kc) + 3) >> 2;
+#pragma unroll 2
+                for (int kg = 0; kg < kgs; ++kg) {
+                    const int kr = kc + 4 * kg + t4;
+                    double av[4], bv[4];
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) av[a] = A[kr * SYRK_LDA + wr + 8 * a + g];
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) bv[b] = B[kr * SYRK_LDB + wc + 8 * b + g];
+#pragma unroll
+                    for (int a = 0; a < 4; ++a)
+#pragma unroll
+                        for (int b = 0; b < 4; ++b) dmma_syrk(acc[a][b][0], acc[a][b][1], av[a], bv[b]);
+                }
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        c[a][b][0] -= acc[a][b][0];
+                        c[a][b][1] -= acc[a][b][1];
+                    }
+            }
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty[q])) : "memory");
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int a = 0; a < 4; ++a)
+                        if (row0 + 8 * a >= last[b][h] && row0 + 8 * a < N) C[b][h][8 * a] = c[a][b][h];
+        }
+    }
+    if (!ok && lane == 0) atomicExch(err, HTF_ETIMEDOUT);
 }
 
 // Copy the trailing nbp x nbp block into packed tiles, minus the fix diagonal.
