@@ -19,9 +19,9 @@
 // have read.
 //
 // Bound by the factor's bytes, read twice, or for few or small subdomains by
-// the chain of N / 32 blocks (2.7 us per block and direction).  Against one
+// the chain of N / 32 blocks (2 us per block and direction).  Against one
 // CTA per subdomain with a block-wide barrier per 32 rows, forward and
-// backward: 8 subdomains of 648 DOFs 1.18 -> 0.12 ms; 64 uneven ones of up to
+// backward: 8 subdomains of 648 DOFs 1.18 -> 0.09 ms; 64 uneven ones of up to
 // 5 577 57 -> 1.46 ms; 512 of 2 187 (10 GB of factor, read twice) 12.7 ->
 // 4.5 ms = 4.6 TB/s.
 #include <cuda_runtime.h>
@@ -248,23 +248,30 @@ cudaError_t ksolve_prepare(int optin) {
 }
 
 // CTAs per cluster for subdomains of blocks[i] 32-row blocks: the width with
-// the shortest estimated time, one CTA per SM.  A subdomain takes the longer
-// of its chain (KS_STEP_US per block and direction) and its factor at
-// KS_CTA_GBS per CTA and twice; the launch the longer of its longest
-// subdomain and the sum of CTA times over the SMs.
+// the shortest estimated time, one CTA per SM and no more CTAs than give
+// every block of the largest subdomain a warp.  A subdomain takes the longer
+// of its chain (KS_STEP_US per block and direction) and its factor, twice, at
+// KS_CTA_GBS per CTA, and a third of the other; the launch the longest of its
+// longest subdomain, the sum of CTA times over the SMs, and all factors at
+// KS_GBS.  Measured: 8 subdomains of 21 blocks 118 us with one CTA each, 86
+// with four; 64 uneven ones of up to 176 blocks 1.47 ms with four, 1.95 with
+// eight; 512 of 71 blocks 4.5 ms with one.
 int ksolve_ctas(const std::vector<int> &blocks) {
-    constexpr double KS_STEP_US = 1.5, KS_CTA_GBS = 60.0;
+    constexpr double KS_STEP_US = 2.0, KS_CTA_GBS = 55.0, KS_GBS = 5000.0;
+    const int most = blocks.empty() ? 1 : *std::max_element(blocks.begin(), blocks.end());
     int best = 1;
     double best_us = 0.0;
-    for (int c = 1; c <= 8; c *= 2) {
-        double sum = 0.0, longest = 0.0;
+    for (int c = 1; c <= 8 && (c == 1 || KS_WARPS * (c / 2) < most); c *= 2) {
+        double sum = 0.0, longest = 0.0, total = 0.0;
         for (int nb : blocks) {
             const double bytes = 8.0 * 32.0 * 32.0 * nb * (nb + 1.0);
-            const double us = std::max(2.0 * KS_STEP_US * nb, bytes / (c * KS_CTA_GBS * 1e3));
+            const double chain = 2.0 * KS_STEP_US * nb, stream = bytes / (c * KS_CTA_GBS * 1e3);
+            const double us = std::max(chain, stream) + 0.3 * std::min(chain, stream);
+            total += bytes;
             sum += c * us;
             longest = std::max(longest, us);
         }
-        const double us = std::max(longest, sum / 148.0);
+        const double us = std::max(std::max(longest, sum / 148.0), total / (KS_GBS * 1e3));
         if (c == 1 || us < 0.98 * best_us) {
             best = c;
             best_us = us;
