@@ -49,15 +49,19 @@ __global__ void k_msym_rows(const int2 *, const ClusterDev *, const double *, co
                             double *, double *, const PcpgState *);
 __global__ void k_msym_reduce(const int2 *, const ClusterDev *, const double *, const double *, double *,
                               const PcpgState *);
+__global__ void k_msym_small(const int2 *, const ClusterDev *, const double *, const int *, const int *, const double *,
+                             double *, const PcpgState *);
 __global__ void k_gf_apply(int, int, const double *, const int *, const double *, const double *, double *,
-                           const double *, double *, unsigned *, const PcpgState *);
+                           const double *, double *, unsigned *, const double *, const double *, const double *, int,
+                           double *, double *, PcpgState *);
 __global__ void k_coarse(const ClusterDev *, const double *, const double *, double *, const PcpgState *);
 __global__ void k_correct(const SubDev *, const ClusterDev *, const double *, const int *, const double *,
                           double *, const PcpgState *);
 __global__ void k_rows(int, const int *, const double *, const double *, const double *, double *,
                        const double *, double *, const PcpgState *);
 __global__ void k_gft_partial(const int *, const int *, const int *, const double *, const double *, double *, int,
-                              const int *, const double *, double *, double *, unsigned *, const PcpgState *);
+                              const int *, const double *, double *, double *, unsigned *, const double *,
+                              const double *, int, PcpgState *);
 __global__ void k_gf_mult(int, const int *, const double *, const double *, double *);
 __global__ void k_update_lam_g(int, const double *, int, const double *, const double *, double *, double *,
                                PcpgState *);
@@ -184,8 +188,16 @@ __global__ void k_gather_u(int ndof, const int *__restrict__ win, const double *
 // free one of the engine's buffers before the end of its life
 void Engine::release(void *p) { mem_.release(p); }
 
+// M's packed tiles up to which one kernel that reads them twice replaces two that read them once: at 8 to 300 tiles
+// it is worth 2 to 4 us of an iteration, at 4 224 tiles (512 subdomains) it takes 10 us more
+constexpr long long MSYM_SMALL_TILES = 1024;
+
 // s = M gc for every cluster (M = [Ac^{-1}] restricted, packed symmetric tiles), gc = the sums of t per coarse row
 void Engine::coarse_apply(const double *t, double *s, const PcpgState *st) {
+    if (msym_small_) {
+        launch_chain(k_msym_small, nmt_, 128, 0, s_, d_mt_, d_cl_, d_MT_, d_gptr_, d_gidx_, t, s, st);
+        return;
+    }
     launch_chain(k_msym_rows, nmt_, 128, 0, s_, d_mt_, d_cl_, d_MT_, d_gptr_, d_gidx_, t, d_mD_, d_mP_, st);
     launch_chain(k_msym_reduce, nmt_, 128, 0, s_, d_mt_, d_cl_, d_mD_, d_mP_, s, st);
 }
@@ -340,6 +352,7 @@ int Engine::upload_layout(Problem &p, std::string &err) {
     // the plain form's coarse solves read M as packed symmetric tiles (the dense M is freed after
     // set-up unless the batched mixed form needs it)
     nmt_ = int(mtl.size());
+    msym_small_ = MT_off <= MSYM_SMALL_TILES;
     d_mt_ = alloc<int2>(mtl.size(), err, rc);
     d_MT_ = alloc<double>(MT_off * TILE_ELEMS, err, rc);
     d_mP_ = alloc<double>(MT_off * TILE, err, rc);
@@ -1014,19 +1027,26 @@ void Engine::op_M(const double *x, double *z, PcpgState *st) {
 }
 
 void Engine::op_P(const double *x, double *Px, double *alpha_out, const double *dotv, double *partial,
-                  PcpgState *st) {
+                  PcpgState *st, bool step) {
     const size_t smem = 6 * ncl_ * sizeof(double);
+    const double *Fw = step ? d_Fw_ : nullptr;       // with the step x = g += rho Fw, lam += rho w (partials of w.Fw)
     launch_chain(k_gft_partial, nchunks_, 256, smem, s_, d_chunk_beg_, d_chunk_end_, d_crow_, d_cval_, x, d_gpart_, ncl_,
-                 d_cl_chunk_ptr_, d_invGtG_, d_a_, alpha_out, d_count_, st);
+                 d_cl_chunk_ptr_, d_invGtG_, d_a_, alpha_out, d_count_, Fw, d_partial_, npart_, st);
     launch_chain(k_gf_apply, npart_, 256, smem, s_, nlam_, ncl_, d_a_, d_gcl_, d_gval_, x, Px, dotv, partial, nullptr,
-                 st);
+                 d_w_, Fw, d_partial_, npart_, d_lam_, d_g_, st);
 }
+
+// every CTA that takes the step sums the npart_ partials itself: beyond STEP_IN_PROJECTOR of them (131 000 rows,
+// about 1 000 CTAs) that is more L2 traffic than the vectors, and a kernel of at most 1184 CTAs does it once
+constexpr int STEP_IN_PROJECTOR = 512;
 
 void Engine::iteration(PcpgState *st) {
     op_F(d_w_, d_Fw_, d_w_, d_partial_, st);
-    launch_chain(k_update_lam_g, std::min(npart_, 1184), 256, 0, s_, nlam_, d_partial_, npart_, d_w_, d_Fw_, d_lam_, d_g_,
-                 st);
-    op_P(d_g_, d_Pg_, d_alpha_, nullptr, nullptr, st);
+    const bool step = npart_ <= STEP_IN_PROJECTOR;
+    if (!step)
+        launch_chain(k_update_lam_g, std::min(npart_, 1184), 256, 0, s_, nlam_, d_partial_, npart_, d_w_, d_Fw_, d_lam_,
+                     d_g_, st);
+    op_P(d_g_, d_Pg_, d_alpha_, nullptr, nullptr, st, step);
     op_M(d_Pg_, d_z_, st);
     op_P(d_z_, d_Pz_, nullptr, d_g_, d_partial_, st);
     launch_chain(k_update_w, std::min(npart_, 1184), 256, 0, s_, nlam_, d_partial_, npart_, d_Pz_, d_w_, st, d_hist_,
@@ -1261,9 +1281,9 @@ int Engine::project_noalloc(const double *x, double *Px, cudaStream_t stream, st
     // that overlapped starts clean
     const size_t smem = 6 * ncl_ * sizeof(double);
     k_gft_partial<<<nchunks_, 256, smem, stream>>>(d_chunk_beg_, d_chunk_end_, d_crow_, d_cval_, x, scr, ncl_,
-                                                   d_cl_chunk_ptr_, d_invGtG_, scr, nullptr, counter, nullptr);
+                                                   d_cl_chunk_ptr_, d_invGtG_, scr, nullptr, counter, nullptr, nullptr, 0, nullptr);
     launch_chain(k_gf_apply, npart_, 256, smem, stream, nlam_, ncl_, scr, d_gcl_, d_gval_, x, Px, nullptr, nullptr,
-                 counter, nullptr);
+                 counter, nullptr, nullptr, nullptr, 0, nullptr, nullptr, nullptr);
     return check(cudaGetLastError(), "htf_projection_noalloc launch", err);
 }
 

@@ -140,7 +140,7 @@ private:
     void op_F(const double *w, double *Fw, const double *dotv, double *partial, PcpgState *st);
     void op_M(const double *x, double *z, PcpgState *st);
     void op_P(const double *x, double *Px, double *alpha_out, const double *dotv, double *partial,
-              PcpgState *st);
+              PcpgState *st, bool step = false);
     void iteration(PcpgState *st);
     void coarse_apply(const double *t, double *s, const PcpgState *st);   // s = M gc, gc summed from t
     void release(void *p);
@@ -195,6 +195,7 @@ private:
     double *d_MT_ = nullptr, *d_mP_ = nullptr, *d_mD_ = nullptr;   // packed symmetric M, its partial sums
     int2 *d_mt_ = nullptr;                     // (cluster, tile row) pairs of M
     int nmt_ = 0;
+    bool msym_small_ = false;                  // one kernel applies M
     int *d_bcr_ = nullptr, *d_bce_ptr_ = nullptr, *d_bce_pos_ = nullptr;
     double *d_bce_val_ = nullptr;
     int *d_slot_ptr_ = nullptr, *d_slot_ent_ = nullptr;

@@ -346,21 +346,36 @@ __device__ __forceinline__ double block_sum_fixed(const double *partial, int np,
 // Gf stored per cluster as a list of (row, 6 values) cut into chunks of up to
 // 1024 rows; per row as up to two (cluster, 6 values) entries.
 //
+// In the iteration x is the updated residual g + rho Fw (Cluster::pcpg,
+// Cluster.cpp:1426-1430): k_gft_partial forms it where it reads g, and
+// k_gf_apply, which visits every row once, writes g and lambda back.
+//
 // k_gft_partial: CTA ch sums its chunk's six products; the CTA that finishes
 // last (a counter, which it sets back to zero) adds the chunks of every
 // cluster, multiplies by (Gf^T Gf)^{-1} and writes a (and -a), both in a
 // fixed order whichever CTA that is.  a may be the partials' own array: all of
 // them have been read by then.
 // ---------------------------------------------------------------------------
+// rho = -gPz / wFw from the partials of w.Fw (256 threads; every CTA the same value)
+__device__ __forceinline__ double step_length(const double *partial, int np, double *red, const PcpgState *st,
+                                              double &wFw) {
+    const double gPz = st->gPz;
+    wFw = block_sum_fixed(partial, np, red);
+    const double rho = -gPz / wFw;
+    return (!(wFw > 0.0) || !isfinite(rho)) ? 0.0 : rho;
+}
+
 __global__ void __launch_bounds__(256) k_gft_partial(const int *__restrict__ chunk_beg,
                                                      const int *__restrict__ chunk_end,
                                                      const int *__restrict__ crow, const double *__restrict__ cval,
                                                      const double *x, double *partial, int ncl,
                                                      const int *__restrict__ cl_chunk_ptr,
                                                      const double *__restrict__ invGtG, double *a_out,
-                                                     double *alpha_out, unsigned *counter, const PcpgState *st) {
+                                                     double *alpha_out, unsigned *counter, const double *Fw,
+                                                     const double *wFw_part, int np, PcpgState *st) {
     extern __shared__ double gt[];                  // 6 ncl
     __shared__ double red[8][6];
+    __shared__ double red8[8];
     __shared__ bool last;
     pdl_next();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -382,10 +397,20 @@ __global__ void __launch_bounds__(256) k_gft_partial(const int *__restrict__ chu
     }
     pdl_wait();
     if (st && st->done) return;
+    double xr[4], fr[4], rho = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        xr[k] = row[k] >= 0 ? x[row[k]] : 0.0;
+        fr[k] = Fw && row[k] >= 0 ? Fw[row[k]] : 0.0;
+    }
+    if (Fw) {
+        double wFw;
+        rho = step_length(wFw_part, np, red8, st, wFw);
+    }
     double s[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const double xv = row[k] >= 0 ? x[row[k]] : 0.0;
+        const double xv = Fw ? xr[k] + rho * fr[k] : xr[k];
 #pragma unroll
         for (int q = 0; q < 6; ++q) s[q] += g[k][q] * xv;
     }
@@ -439,7 +464,9 @@ __global__ void __launch_bounds__(256) k_gft_partial(const int *__restrict__ chu
 __global__ void __launch_bounds__(256) k_gf_apply(int nlam, int ncl, const double *acoef,
                                                   const int *__restrict__ gcl, const double *__restrict__ gval,
                                                   const double *x, double *Px, const double *dotv, double *partial,
-                                                  unsigned *reset, const PcpgState *st) {
+                                                  unsigned *reset, const double *w, const double *Fw,
+                                                  const double *wFw_part, int np, double *lam, double *g_out,
+                                                  PcpgState *st) {
     extern __shared__ double sh[];
     double *a = sh;                  // 6*ncl
     __shared__ double red[8];
@@ -457,7 +484,21 @@ __global__ void __launch_bounds__(256) k_gf_apply(int nlam, int ncl, const doubl
     if (st && st->done) return;
     if (reset && blockIdx.x == 0 && threadIdx.x == 0) *reset = 0;
     for (int q = threadIdx.x; q < 6 * ncl; q += blockDim.x) a[q] = acoef[q];
-    const double xr = r < nlam ? x[r] : 0.0;
+    double xr = r < nlam ? x[r] : 0.0;
+    if (Fw) {                                        // lam += rho w ; g += rho Fw (x is g)
+        const double fw = r < nlam ? Fw[r] : 0.0, wr = r < nlam ? w[r] : 0.0, lr = r < nlam ? lam[r] : 0.0;
+        double wFw;
+        const double rho = step_length(wFw_part, np, red, st, wFw);
+        if (r < nlam) {
+            xr += rho * fw;
+            g_out[r] = xr;
+            lam[r] = lr + rho * wr;
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            st->wFw = wFw;
+            st->rho = rho;
+        }
+    }
     __syncthreads();
     double prod = 0.0;
     if (r < nlam) {
@@ -502,16 +543,15 @@ __global__ void k_gf_mult(int nlam, const int *__restrict__ gcl, const double *_
 // PCPG scalar / vector updates (Cluster::pcpg, Cluster.cpp:1422-1450)
 // ---------------------------------------------------------------------------
 // after Fw and the partials of w.Fw: rho = -gPz / wFw ; lam += rho w ; g += rho Fw
+// (problems of more rows than the projector updates on the way)
 __global__ void __launch_bounds__(256) k_update_lam_g(int n, const double *partial, int np, const double *w,
                                                       const double *Fw, double *lam, double *g, PcpgState *st) {
     __shared__ double red[8];
     pdl_next();
     pdl_wait();
     if (st->done) return;
-    const double gPz = st->gPz;
-    const double wFw = block_sum_fixed(partial, np, red);
-    double rho = -gPz / wFw;
-    if (!(wFw > 0.0) || !isfinite(rho)) rho = 0.0;
+    double wFw;
+    const double rho = step_length(partial, np, red, st, wFw);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         st->wFw = wFw;
         st->rho = rho;
@@ -767,6 +807,74 @@ __global__ void __launch_bounds__(128) k_msym_rows(const int2 *__restrict__ mt, 
     __syncthreads();
     if (warp == 0)
         D[((long long)c.mt_row_off + I) * TILE + lane] = ((part[0][lane] + part[1][lane]) + part[2][lane]) + part[3][lane];
+}
+
+// Both in one launch for a small M: CTA (cluster, J) reads the tiles of row J
+// and, transposed, of column J (every off-diagonal tile twice, the second
+// time from L2), with the sums of the two kernels in the same order.
+__global__ void __launch_bounds__(128) k_msym_small(const int2 *__restrict__ mt, const ClusterDev *__restrict__ cl,
+                                                    const double *__restrict__ T, const int *__restrict__ gptr,
+                                                    const int *__restrict__ gidx, const double *t, double *s,
+                                                    const PcpgState *st) {
+    __shared__ double part[4][TILE];
+    __shared__ double xs[4][TILE];
+    pdl_next();
+    const int2 b = mt[blockIdx.x];
+    const ClusterDev c = cl[b.x];
+    const int J = b.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double v[32];
+    int e0 = 0, e1 = 0, i0 = 0, i1 = 0;
+    // tile (A, B), A >= B, and the t entries behind the coarse right-hand side of block X
+    auto load = [&](int A, int B, int X) {
+        const double *tp = T + (c.MT_off + (long long)A * (A + 1) / 2 + B) * TILE_ELEMS;
+#pragma unroll
+        for (int r = 0; r < 32; ++r) v[r] = tp[r * TILE + lane];
+        e0 = e1 = 0;
+        const int q = TILE * X + lane;
+        if (q < c.ngc) {
+            e0 = gptr[c.gc_off + q];
+            e1 = gptr[c.gc_off + q + 1];
+        }
+        i0 = e0 < e1 ? gidx[e0] : 0;
+        i1 = e0 + 1 < e1 ? gidx[e0 + 1] : 0;
+    };
+    auto rhs = [&] {
+        double g = e0 < e1 ? t[i0] : 0.0;
+        if (e0 + 1 < e1) g += t[i1];
+        for (int e = e0 + 2; e < e1; ++e) g += t[gidx[e]];
+        return g;
+    };
+    if (warp <= J) load(J, warp, warp);
+    pdl_wait();
+    if (st && st->done) return;
+    double dir = 0.0;
+    for (int B = warp; B <= J; B += 4) {
+        const double xB = rhs();
+        double p[32];
+#pragma unroll
+        for (int r = 0; r < 32; ++r) p[r] = v[r] * xB;
+        if (B + 4 <= J) load(J, B + 4, B + 4);
+        reduce_scatter32(p, lane);
+        dir += p[0];
+    }
+    part[warp][lane] = dir;
+    __syncthreads();
+    double y = warp == 0 ? ((part[0][lane] + part[1][lane]) + part[2][lane]) + part[3][lane] : 0.0;
+    __syncthreads();
+    for (int I = J + 1 + warp; I < c.mt; I += 4) {
+        load(I, J, I);
+        xs[warp][lane] = rhs();
+        __syncwarp();
+        double col = 0.0;
+#pragma unroll
+        for (int r = 0; r < 32; ++r) col += v[r] * xs[warp][r];
+        __syncwarp();
+        y += col;
+    }
+    part[warp][lane] = y;
+    __syncthreads();
+    if (warp == 0 && TILE * J + lane < c.ngc)
+        s[c.gc_off + TILE * J + lane] = ((part[0][lane] + part[1][lane]) + part[2][lane]) + part[3][lane];
 }
 
 __global__ void __launch_bounds__(128) k_msym_reduce(const int2 *__restrict__ mt, const ClusterDev *__restrict__ cl,
