@@ -213,17 +213,18 @@ struct DevTmp {                        // device scratch freed when the coarse s
     }
 };
 
+int cdivc(long long a, long long b) { return int((a + b - 1) / b); }
+
 // step tables of the batched right-looking Cholesky of the given matrices
 void chol_steps(const std::vector<SubDev> &m, std::vector<std::vector<StepDesc>> &steps) {
     steps.clear();
     for (int d = 0; d < int(m.size()); ++d)
         for (int k = 0, s = 0; k < m[d].N; k += CHOL_STEP, ++s) {
             if (int(steps.size()) <= s) steps.resize(s + 1);
-            steps[s].push_back({d, k, std::min(CHOL_STEP, m[d].N - k), 0, 0});
+            const int nb = std::min(CHOL_STEP, m[d].N - k), n = cdivc(m[d].N, CHOL_STEP);
+            steps[s].push_back({d, k, nb, step_pair(s, n, std::min(CHOL_STEP, m[d].N - k - nb), m[d].N), 0, 0});
         }
 }
-
-int cdivc(long long a, long long b) { return int((a + b - 1) / b); }
 
 }  // namespace
 
@@ -239,7 +240,7 @@ static cudaError_t chol_batched(const std::vector<SubDev> &hm, const SubDev *dm,
         int tri = 0, rb = 0;
         for (auto &x : v) {
             const int rows = hm[x.d].N - x.k - x.nb;
-            x.tri0 = tri; tri += syrk_tiles(rows);
+            x.tri0 = tri; tri += syrk_tiles(rows, x.pair);
             x.rb0 = rb; rb += (rows + 127) / 128;
         }
         ntri.push_back(tri);

@@ -635,7 +635,13 @@ int Engine::factorize(Problem &p, std::string &err) {
             int interior_steps = int(blocks.size());
             for (int k = h.nr; k < h.N; k += CHOL_STEP) blocks.push_back({k, std::min(CHOL_STEP, h.N - k)});
             if (steps.size() < blocks.size()) { steps.resize(blocks.size()); snap_after.resize(blocks.size()); }
-            for (size_t s = 0; s < blocks.size(); ++s) steps[s].push_back({d, blocks[s].first, blocks[s].second, 0, 0});
+            // pairs within the interior and within the b set
+            const int nint = interior_steps, nbset = int(blocks.size()) - nint;
+            for (int s = 0; s < int(blocks.size()); ++s) {
+                const int i = s < nint ? s : s - nint, n = s < nint ? nint : nbset;
+                steps[s].push_back({d, blocks[s].first, blocks[s].second,
+                                    step_pair(i, n, i + 1 < n ? blocks[s + 1].second : 0, h.N), 0, 0});
+            }
             if (interior_steps == 0) snap_first.push_back(d);
             else snap_after[interior_steps - 1].push_back(d);
         }
@@ -644,7 +650,7 @@ int Engine::factorize(Problem &p, std::string &err) {
             int tri = 0, rb = 0;
             for (auto &x : v) {
                 const int rows = hs_[x.d].N - x.k - x.nb;
-                x.tri0 = tri; tri += syrk_tiles(rows);
+                x.tri0 = tri; tri += syrk_tiles(rows, x.pair);
                 x.rb0 = rb; rb += (rows + 127) / 128;
             }
             W.cnt.push_back(int(v.size()));

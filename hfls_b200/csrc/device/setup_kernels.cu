@@ -329,7 +329,9 @@ __global__ void __launch_bounds__(128) k_trsm_panel(const StepDesc *__restrict__
 
 // C (128 x 64 tile of the lower part of the trailing matrix) -= P_i P_j^T, P =
 // the step's panel rows: 32 columns of P at a time, one sum per panel,
-// subtracted in turn, C read and written once.
+// subtracted in turn, C read and written once.  Steps come in pairs
+// (StepDesc::pair): after the first only the second's columns are updated,
+// after the second the rest with the panels of both.
 //
 // Persistent: one CTA per SM of eight product warps and four copy warps, which
 // run through the step's tiles (CTA c takes tiles c, c + CTAs, ..).  The copy
@@ -344,10 +346,10 @@ __global__ void __launch_bounds__(128) k_trsm_panel(const StepDesc *__restrict__
 // free of bank conflicts.  C's loads are pinned to the start of the tile
 // (left to the compiler they sink to their use: 128 ms).  One CTA per 64 x 64
 // tile, with nothing in flight while it multiplied, reached 9.5 TFLOP/s on
-// 512 x 2 187 DOFs (189 ms in all), this 16.5 (108 ms); 64 uneven subdomains
-// of up to 5 577 DOFs 104 -> 59 ms.  The products alone would take 56 and 33
-// ms at the FP64 tensor rate (36 TFLOP/s); the rest is C through fragments of
-// 64 contiguous bytes.
+// 512 x 2 187 DOFs (189 ms in all), this 19 (94 ms); 64 uneven subdomains of
+// up to 5 577 DOFs 104 -> 50 ms.  The products alone would take 56 and 33 ms
+// at the FP64 tensor rate (36 TFLOP/s); the rest is C through fragments of 64
+// contiguous bytes.
 __device__ __forceinline__ void dmma_syrk(double &d0, double &d1, double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                  : "+d"(d0), "+d"(d1)
@@ -379,7 +381,9 @@ constexpr int SYRK_LDA = 132, SYRK_LDB = 68;
 constexpr int SYRK_STAGE = CHOL_STEP * (SYRK_LDA + SYRK_LDB);       // doubles: A columns, then B columns
 
 struct SyrkTile {
-    int d, k, nb, i0, j0;                   // subdomain, step, first row and column of the tile; d < 0: no more
+    int d, k, nb;                           // subdomain (< 0: no more), panel columns of this stage
+    int i0, j0, jend;                       // first row and column of the tile, end of the columns to update
+    int part;                               // bit 0: the tile's first stage, bit 1: its last
 };
 
 __global__ void __launch_bounds__(SYRK_THREADS, 1) k_syrk_update(const StepDesc *__restrict__ st, int cnt, int tiles,
@@ -400,18 +404,31 @@ __global__ void __launch_bounds__(SYRK_THREADS, 1) k_syrk_update(const StepDesc 
     // registers: 12 warps of 168 at launch, then 8 of 216 and 4 of 72 (the same sum)
     if (warp >= 8) {                        // copies: every SYRK_COPY_WARPS-th column
         asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-        int n = 0;
-        for (int t = blockIdx.x; ok; t += gridDim.x, ++n) {
+        int n = 0, half = 0;
+        StepDesc s{};
+        for (int t = blockIdx.x; ok; t += half ? 0 : gridDim.x, ++n) {
             const int q = n & 1;
-            SyrkTile T{-1, 0, 0, 0, 0};
+            SyrkTile T{-1, 0, 0, 0, 0, 0, 0};
             if (t < tiles) {
-                const StepDesc s = st[step_entry(st, cnt, t, [](const StepDesc &x) { return x.tri0; }, hint)];
-                // row block bi (128 rows) has column blocks (64) 0 .. 2 bi + 1: bi (bi + 1) tiles before it
-                const int tri = t - s.tri0;
-                int bi = (int)((sqrt(4.0 * tri + 1.0) - 1.0) * 0.5);
-                while ((bi + 1) * (bi + 2) <= tri) ++bi;
-                while (bi * (bi + 1) > tri) --bi;
-                T = SyrkTile{s.d, s.k, s.nb, s.k + s.nb + 128 * bi, s.k + s.nb + 64 * (tri - bi * (bi + 1))};
+                if (half == 0) s = st[step_entry(st, cnt, t, [](const StepDesc &x) { return x.tri0; }, hint)];
+                const int tri = t - s.tri0, t0 = s.k + s.nb;
+                int bi = tri, bj = 0;                    // first of a pair: column block 0 of every row block
+                if (s.pair <= 0) {
+                    // row block bi (128 rows) has column blocks (64) 0 .. 2 bi + 1: bi (bi + 1) tiles before it
+                    bi = (int)((sqrt(4.0 * tri + 1.0) - 1.0) * 0.5);
+                    while ((bi + 1) * (bi + 2) <= tri) ++bi;
+                    while (bi * (bi + 1) > tri) --bi;
+                    bj = tri - bi * (bi + 1);
+                }
+                T = SyrkTile{s.d, s.k, s.nb, t0 + 128 * bi, t0 + 64 * bj, s.pair > 0 ? t0 + s.pair : subs[s.d].N, 3};
+                if (s.pair < 0) {                        // the panels of both steps, one stage each
+                    if (half == 0) {
+                        T.k = s.k - CHOL_STEP;
+                        T.nb = CHOL_STEP;
+                    }
+                    T.part = half == 0 ? 1 : 2;
+                    half ^= 1;
+                }
             }
             if (n >= 2) ok = mbar_wait(&empty[q], ((n >> 1) - 1) & 1);
             if (!ok) break;
@@ -452,31 +469,34 @@ __global__ void __launch_bounds__(SYRK_THREADS, 1) k_syrk_update(const StepDesc 
         asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
         const int g = lane >> 2, t4 = lane & 3;
         const int wr = 32 * (warp >> 1), wc = 32 * (warp & 1);
+        // this thread's C: rows i0 + wr + 8 a + g, columns j0 + wc + 8 b + 2 t4 + h (lower part, in range)
+        double *C[4][2];
+        double c[4][4][2];
+        int last[4][2];                     // rows row0 + 8 a of the column are stored for last <= row0 + 8 a < N
+        int row0 = 0, N = 0;
         for (int n = 0;; ++n) {
             const int q = n & 1;
             ok = mbar_wait(&full[q], (n >> 1) & 1);
             if (!ok) break;
             const SyrkTile T = desc[q];
             if (T.d < 0) break;
-            const SubDev &sd = subs[T.d];
-            const int N = sd.N;
             const double *A = syrk_sm + q * SYRK_STAGE, *B = A + CHOL_STEP * SYRK_LDA;
-            // this thread's C: rows i0 + wr + 8 a + g, columns j0 + wc + 8 b + 2 t4 + h (lower part, in range)
-            double *C[4][2];
-            double c[4][4][2];
-            int last[4][2];                 // rows row0 + 8 a of the column are stored for first <= row0 + 8 a < N
-            const int row0 = T.i0 + wr + g;
+            if (T.part & 1) {
+                const SubDev &sd = subs[T.d];
+                N = sd.N;
+                row0 = T.i0 + wr + g;
 #pragma unroll
-            for (int b = 0; b < 4; ++b)
+                for (int b = 0; b < 4; ++b)
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int col = T.j0 + wc + 8 * b + 2 * t4 + h;
-                    C[b][h] = Kbuf + kcol(sd, min(col, N - 1)) + row0;
-                    last[b][h] = col < N ? col : N;
+                    for (int h = 0; h < 2; ++h) {
+                        const int col = T.j0 + wc + 8 * b + 2 * t4 + h;
+                        C[b][h] = Kbuf + kcol(sd, min(col, N - 1)) + row0;
+                        last[b][h] = col < T.jend ? col : N;
 #pragma unroll
-                    for (int a = 0; a < 4; ++a)
-                        c[a][b][h] = ld_now(C[b][h] + 8 * a, row0 + 8 * a >= last[b][h] && row0 + 8 * a < N);
-                }
+                        for (int a = 0; a < 4; ++a)
+                            c[a][b][h] = ld_now(C[b][h] + 8 * a, row0 + 8 * a >= last[b][h] && row0 + 8 * a < N);
+                    }
+            }
             for (int kc = 0; kc < T.nb; kc += TILE) {
                 double acc[4][4][2];
 #pragma unroll
@@ -508,6 +528,7 @@ __global__ void __launch_bounds__(SYRK_THREADS, 1) k_syrk_update(const StepDesc 
             __syncwarp();
             if (lane == 0)
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty[q])) : "memory");
+            if (!(T.part & 2)) continue;
 #pragma unroll
             for (int b = 0; b < 4; ++b)
 #pragma unroll
