@@ -179,7 +179,7 @@ struct TcSet {
     const float *Xs;                      // FP16-pair X slabs (k x 32 words per 32 b-space slots)
     double *yb;                           // b-space output, RHS-interleaved
     const unsigned *amaxF, *amaxS;        // largest |F_i|, |S_i| per subdomain (FP32 bits): scale of A
-    const unsigned *xmax;                 // largest |w_j| of the gathered batch vector (FP32 bits)
+    const unsigned *xmax, *xmaxS;         // largest |w_j| of the batch vector gathered for F, for S (FP32 bits)
     float xbound;                         // |x_b| <= xbound * max|w_j|: scale of X
 };
 

@@ -103,15 +103,18 @@ private:
     void tc_apply(int which);
     void f_pre(const double *w);
     void coarse_batch();
-    void f_post(double *Fw, const double *dotv, double *partial);
+    void f_post(double *Fw, const double *dotv, double *partial, const double *dot2v = nullptr,
+                double *partial2 = nullptr);
     void m_pre(const double *x);
-    void gather_x(const double *w, const double *weight, double *xb);   // x_b and the X slabs
+    void column_maxima(const double *w, int which);
+    void gather_x(const double *w, int which, double *xb);              // x_b and the X slabs
     void m_post(double *z);
     int fp64_residual_batch(const std::vector<int> &sel, const std::vector<int> &reset, std::string &err);
     void profile_batch_gather(const double *w);
     void op_F_batch(const double *w, double *Fw, const double *dotv, double *partial);
     void op_M_batch(const double *x, double *z);
-    void op_P_batch(const double *x, double *Px, double *alpha_out, const double *dotv, double *partial);
+    void op_P_batch(const double *x, double *Px, double *alpha_out, const double *dotv, double *partial,
+                    unsigned *xmax = nullptr);
     template <typename... P, typename... A>
     void link(void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args);
     void iteration_batch();
@@ -242,7 +245,7 @@ private:
     int *d_slot_sub_ = nullptr, *d_tcerr_ = nullptr;
     double *b_lam_ = nullptr, *b_g_ = nullptr, *b_w_ = nullptr, *b_Fw_ = nullptr, *b_Pg_ = nullptr, *b_z_ = nullptr,
            *b_Pz_ = nullptr, *b_d_ = nullptr, *b_xb_ = nullptr, *b_yb_ = nullptr, *b_t_ = nullptr, *b_gc_ = nullptr,
-           *b_s_ = nullptr, *b_part_ = nullptr, *b_gpart_ = nullptr, *b_wFw_ = nullptr, *b_gPz_ = nullptr, *b_gw_ = nullptr, *b_gt_ = nullptr, *b_acoef_ = nullptr,
+           *b_s_ = nullptr, *b_part_ = nullptr, *b_part2_ = nullptr, *b_gpart_ = nullptr, *b_wFw_ = nullptr, *b_gPz_ = nullptr, *b_gw_ = nullptr, *b_gt_ = nullptr, *b_acoef_ = nullptr,
            *b_alpha_ = nullptr, *b_tmp_ = nullptr;
     double *b_fullA_ = nullptr, *b_fullB_ = nullptr;   // full vectors of the batch (nfull x K)
     double *b_srec_ = nullptr;                         // coarse solutions of the reconstruction (ngc x K)

@@ -43,18 +43,17 @@ template <int K>
 __global__ void k_correct_multi(const SubDev *, const ClusterDev *, const double *, const int *, const double *,
                                 double *);
 __global__ void k_rows_multi(int, int, const int *, const double *, const double *, const double *, double *,
-                             const double *, double *);
+                             const double *, double *, const double *, double *);
 __global__ void k_gft_partial_multi(int, const int *, const int *, const int *, const double *, const double *,
                                     double *);
 __global__ void k_gt_sum_multi(int, const int *, const double *, double *);
 __global__ void k_gf_coef_multi(int, int, const double *, const double *, double *, double *);
 __global__ void k_gf_apply_multi(int, int, const double *, const int *, const double *, const double *, double *,
-                                 const double *, double *);
-__global__ void k_colsum(const double *, int, int, double *);
+                                 const double *, double *, unsigned *);
+__global__ void k_colsum(const double *, int, int, double *, const double *, double *, unsigned *);
 __global__ void k_update_lam_g_multi(int, int, const double *, const double *, const double *, const double *, double *,
                                      double *, PcpgState *);
-__global__ void k_dot_multi(int, int, const double *, const double *, double *);
-__global__ void k_update_w_multi(int, int, const double *, const double *, double *, const PcpgState *);
+__global__ void k_update_w_multi(int, int, const double *, const double *, double *, const PcpgState *, unsigned *);
 __global__ void k_finish_multi(int, const double *, const double *, PcpgState *, double *);
 template <int K>
 __global__ void k_msym_rows_multi(const int2 *, const ClusterDev *, const double *, const double *, double *);
@@ -160,7 +159,7 @@ int Engine::setup_batch(int K, std::string &err) {
         }
     if ((rc = plan_slabs(K, err))) return rc;
     d_Xs_ = alloc<float>((size_t)nslots_ * K, err, rc);
-    d_xmax_ = alloc<unsigned>(K, err, rc);
+    d_xmax_ = alloc<unsigned>(2 * K, err, rc);        // of w (F product), of P g (S product)
     d_slot_sub_ = alloc<int>(nslots_, err, rc);
     d_tcerr_ = alloc<int>(1, err, rc);
     d_tcset_ = alloc<TcSet>(1, err, rc);
@@ -228,7 +227,7 @@ int Engine::alloc_batch(int K, std::string &err) {
     b_xb_ = alloc<double>((size_t)nslots_ * K, err, rc); b_yb_ = alloc<double>((size_t)nslots_ * K, err, rc);
     b_t_ = alloc<double>((size_t)ntot * vt_nch_ * K, err, rc);     // V^T x_b partials per 128-row chunk
     b_gc_ = alloc<double>((size_t)ngc_total_ * K, err, rc); b_s_ = alloc<double>((size_t)ngc_total_ * K, err, rc);
-    b_part_ = alloc<double>((size_t)bnpart_ * K, err, rc);
+    b_part_ = alloc<double>((size_t)bnpart_ * K, err, rc); b_part2_ = alloc<double>((size_t)bnpart_ * K, err, rc);
     b_gpart_ = alloc<double>((size_t)nchunks_ * 6 * K, err, rc);
     b_wFw_ = alloc<double>(K, err, rc); b_gPz_ = alloc<double>(K, err, rc);
     b_gw_ = alloc<double>(K, err, rc);
@@ -254,21 +253,30 @@ int Engine::alloc_batch(int K, std::string &err) {
 // the coarse correction of the F product runs after it (k_correct_multi in
 // f_post), so the product's epilogue gets no coarse solution
 TcSet Engine::tc_set() const {
-    return TcSet{d_AF_, d_AS_, d_Xs_, b_yb_, d_amaxF_, d_amaxS_, d_xmax_, xbound_};
+    return TcSet{d_AF_, d_AS_, d_Xs_, b_yb_, d_amaxF_, d_amaxS_, d_xmax_, d_xmax_ + bK_, xbound_};
 }
 
-// x_b = Bf^T w (weighted when weight != nullptr; into xb when xb != nullptr)
-// and the X slabs of the tensor-core product, scaled from w's column maxima
-void Engine::gather_x(const double *w, const double *weight, double *xb) {
+// column maxima of a batch vector, the scale of its X slabs: of w for F (which = 0), of P g for S (1).  The
+// iteration's own kernels keep them for the vectors they write; this is for vectors made elsewhere
+void Engine::column_maxima(const double *w, int which) {
     const int K = bK_;
-    cudaMemsetAsync(d_xmax_, 0, K * sizeof(unsigned), s_);
-    k_colmax<<<std::max(1, std::min(cdivb((long long)nlam_ * K, 256), 1184)), 256, 0, s_>>>(nlam_, K, w, d_xmax_);
-    link(k_gather_multi, nslots_ / 32, 256, 0, nslots_, K, d_slot_ptr_, d_slot_ent_, w, weight, xb, d_Xs_, d_xmax_,
-                                                 xbound_);
+    cudaMemsetAsync(d_xmax_ + which * K, 0, K * sizeof(unsigned), s_);
+    k_colmax<<<std::max(1, std::min(cdivb((long long)nlam_ * K, 256), 1184)), 256, 0, s_>>>(nlam_, K, w,
+                                                                                              d_xmax_ + which * K);
+}
+
+// x_b = Bf^T w (for S weighted; into xb when xb != nullptr) and the X slabs of the tensor-core product, scaled from
+// w's column maxima
+void Engine::gather_x(const double *w, int which, double *xb) {
+    link(k_gather_multi, nslots_ / 32, 256, 0, nslots_, bK_, d_slot_ptr_, d_slot_ent_, w, which ? d_weight_ : nullptr,
+         xb, d_Xs_, d_xmax_ + which * bK_, xbound_);
 }
 
 // X slabs of a batch vector (for timing the tensor-core product alone)
-void Engine::profile_batch_gather(const double *w) { gather_x(w, nullptr, b_xb_); }
+void Engine::profile_batch_gather(const double *w) {
+    column_maxima(w, 0);
+    gather_x(w, 0, b_xb_);
+}
 
 // one tensor-core launch over the given blocks / operand sets (which: 0 = F,
 // 1 = S; the coarse correction of F follows in k_correct_multi)
@@ -289,7 +297,7 @@ void Engine::tc_apply(int which) {
 // F w = Bf [F_d x_b - V_d M_c V_d^T x_b]: the coarse solve before the
 // tensor-core product, whose epilogue applies the correction
 void Engine::f_pre(const double *w) {
-    gather_x(w, nullptr, b_xb_);
+    gather_x(w, 0, b_xb_);
     coarse_batch();
 }
 
@@ -319,38 +327,43 @@ void Engine::coarse_batch() {
     else link(k_coarse_multi<16>, dim3(ncl_, cdivb(maxg, 32)), 128, 0, d_cl_, d_M_, b_gc_, b_s_);
 }
 
-void Engine::f_post(double *Fw, const double *dotv, double *partial) {
+void Engine::f_post(double *Fw, const double *dotv, double *partial, const double *dot2v, double *partial2) {
     const dim3 gc(nsub_, cdivb(max_nbp_, 128));
     if (bK_ == 32) link(k_correct_multi<32>, gc, 256, 0, d_subs_, d_cl_, d_V_, d_bcr_, b_s_, b_yb_);
     else link(k_correct_multi<16>, gc, 256, 0, d_subs_, d_cl_, d_V_, d_bcr_, b_s_, b_yb_);
-    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, nullptr, Fw, dotv, partial);
+    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, nullptr, Fw, dotv, partial, dot2v,
+         partial2);
 }
 
 // the preconditioner uses the same FP16-pair products as F
-void Engine::m_pre(const double *x) { gather_x(x, d_weight_, nullptr); }
+void Engine::m_pre(const double *x) { gather_x(x, 1, nullptr); }
 
 void Engine::m_post(double *z) {
-    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, d_weight_, z, nullptr, nullptr);
+    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, d_weight_, z, nullptr, nullptr, nullptr,
+         nullptr);
 }
 
 void Engine::op_F_batch(const double *w, double *Fw, const double *dotv, double *partial) {
+    column_maxima(w, 0);
     f_pre(w);
     tc_apply(0);
     f_post(Fw, dotv, partial);
 }
 
 void Engine::op_M_batch(const double *x, double *z) {
+    column_maxima(x, 1);
     m_pre(x);
     tc_apply(1);
     m_post(z);
 }
 
-void Engine::op_P_batch(const double *x, double *Px, double *alpha_out, const double *dotv, double *partial) {
+void Engine::op_P_batch(const double *x, double *Px, double *alpha_out, const double *dotv, double *partial,
+                        unsigned *xmax) {
     const int K = bK_;
     link(k_gft_partial_multi, nchunks_, 256, GFT_SMEM, K, d_chunk_beg_, d_chunk_end_, d_crow_, d_cval_, x, b_gpart_);
     link(k_gt_sum_multi, 6 * ncl_, K, 0, K, d_cl_chunk_ptr_, b_gpart_, b_gt_);
     link(k_gf_coef_multi, 6 * ncl_, K, 0, K, ncl_, d_invGtG_, b_gt_, b_acoef_, alpha_out);
-    link(k_gf_apply_multi, bnpart_, 256, 0, nlam_, K, b_acoef_, d_gcl_, d_gval_, x, Px, dotv, partial);
+    link(k_gf_apply_multi, bnpart_, 256, 0, nlam_, K, b_acoef_, d_gcl_, d_gval_, x, Px, dotv, partial, xmax);
 }
 
 // one batched iteration = iter_a | F product | iter_b | S product | iter_c
@@ -359,22 +372,21 @@ void Engine::iter_a() { f_pre(b_w_); }
 void Engine::iter_b() {
     const int K = bK_;
     const int nk = cdivb((long long)nlam_ * K, 256);
-    f_post(b_Fw_, b_w_, b_part_);
-    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_wFw_);
-    link(k_dot_multi, bnpart_, 256, 0, nlam_, K, b_g_, b_w_, b_part_);
-    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gw_);
+    // w'Fw and g'w; the maxima of this iteration's w and of the last P g have been used: set to zero
+    f_post(b_Fw_, b_w_, b_part_, b_g_, b_part2_);
+    link(k_colsum, 2 * K, 256, 0, b_part_, bnpart_, K, b_wFw_, b_part2_, b_gw_, d_xmax_);
     link(k_update_lam_g_multi, nk, 256, 0, nlam_, K, b_wFw_, b_gw_, b_w_, b_Fw_, b_lam_, b_g_, b_st_);
-    op_P_batch(b_g_, b_Pg_, nullptr, nullptr, nullptr);
+    op_P_batch(b_g_, b_Pg_, nullptr, nullptr, nullptr, d_xmax_ + K);
     m_pre(b_Pg_);
 }
 
 void Engine::iter_c() {
     const int K = bK_;
-    const int nk = cdivb((long long)nlam_ * K, 256);
     m_post(b_z_);
     op_P_batch(b_z_, b_Pz_, nullptr, b_g_, b_part_);
-    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_);
-    link(k_update_w_multi, nk, 256, 0, nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_);
+    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_, nullptr, nullptr, nullptr);
+    link(k_update_w_multi, std::min(cdivb((long long)nlam_ * K, 256), 1184), 256, 0, nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_,
+         d_xmax_);
     link(k_finish_multi, 1, 32, 0, K, b_wFw_, b_gPz_, b_st_, nullptr);
 }
 
@@ -445,7 +457,8 @@ int Engine::fp64_residual_batch(const std::vector<int> &sel, const std::vector<i
                                                  nullptr, 0.f);
     coarse_batch();
     symv_multi(d_F_, b_s_);
-    link(k_rows_multi, bnpart_, 256, 0, nlam_, K, d_rslot_, d_rsign_, b_yb_, nullptr, b_tmp_, nullptr, nullptr);
+    link(k_rows_multi, bnpart_, 256, 0, nlam_, K, d_rslot_, d_rsign_, b_yb_, nullptr, b_tmp_, nullptr, nullptr, nullptr,
+         nullptr);
     k_axpby<<<cdivb(nk, 256), 256, 0, s_>>>(int(nk), -1.0, b_d_, 1.0, b_tmp_);
     op_P_batch(b_tmp_, b_Pg_, b_alpha2_, nullptr, nullptr);
     // z = M P g, P z, g'Pz
@@ -453,12 +466,13 @@ int Engine::fp64_residual_batch(const std::vector<int> &sel, const std::vector<i
         link(k_gather_multi, nslots_ / 32, 256, 0, nslots_, K, d_slot_ptr_, d_slot_ent_, b_Pg_, d_weight_, b_xb_,
                                                      nullptr, nullptr, 0.f);
         symv_multi(d_S_, nullptr);
-        link(k_rows_multi, bnpart_, 256, 0, nlam_, K, d_rslot_, d_rsign_, b_yb_, d_weight_, b_z_, nullptr, nullptr);
+        link(k_rows_multi, bnpart_, 256, 0, nlam_, K, d_rslot_, d_rsign_, b_yb_, d_weight_, b_z_, nullptr, nullptr, nullptr,
+         nullptr);
     } else {
         op_M_batch(b_Pg_, b_z_);      // S_i only as tensor-core slabs: the tensor-core product
     }
     op_P_batch(b_z_, b_Pz_, nullptr, b_tmp_, b_part_);
-    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_);
+    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_, nullptr, nullptr, nullptr);
     // the selected columns back into the recurrence
     std::vector<int> masks(2 * K, 0);
     for (int j = 0; j < K; ++j) {
@@ -468,6 +482,7 @@ int Engine::fp64_residual_batch(const std::vector<int> &sel, const std::vector<i
     CKB(cudaMemcpyAsync(d_mask_, masks.data(), 2 * K * sizeof(int), cudaMemcpyHostToDevice, s_));
     k_cols_copy<<<cdivb(nk, 256), 256, 0, s_>>>(nlam_, K, d_mask_, b_tmp_, b_g_);
     k_cols_copy<<<cdivb(nk, 256), 256, 0, s_>>>(nlam_, K, d_mask_ + K, b_Pz_, b_w_);
+    column_maxima(b_w_, 0);
     k_alpha_cols<<<1, 256, 0, s_>>>(6 * ncl_, K, d_mask_, b_alpha2_, b_alpha_);
     CKB(cudaGetLastError());
     launches_ += 19 + 8;
@@ -778,7 +793,7 @@ bool Engine::ready_batch64(int nrhs) {
     }
     const double need = 8.0 * K *
                         (9.0 * nlam_ + 2.0 * nslots_ + 2.0 * nfull_ + double(tn) * nch + 3.0 * ngc_total_ +
-                         6.0 * nchunks_ + 1184.0 + double(std::max(opt_.max_iter, 0)) + 1.0);
+                         6.0 * nchunks_ + 2.0 * 1184.0 + double(std::max(opt_.max_iter, 0)) + 1.0);
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || need > 0.25 * double(fr)) {
         cudaGetLastError();
@@ -810,13 +825,13 @@ void Engine::iteration_batch64() {
     const int K = bK_;
     const int nk = cdivb((long long)nlam_ * K, 256);
     op_F_batch64(b_w_, b_Fw_, b_w_, b_part_);
-    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_wFw_);
+    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_wFw_, nullptr, nullptr, nullptr);
     link(k_update_lam_g_multi, nk, 256, 0, nlam_, K, b_wFw_, nullptr, b_w_, b_Fw_, b_lam_, b_g_, b_st_);
     op_P_batch(b_g_, b_Pg_, b_alpha2_, nullptr, nullptr);
     op_M_batch64(b_Pg_, b_z_);
     op_P_batch(b_z_, b_Pz_, nullptr, b_g_, b_part_);
-    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_);
-    link(k_update_w_multi, nk, 256, 0, nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_);
+    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_, nullptr, nullptr, nullptr);
+    link(k_update_w_multi, std::min(nk, 1184), 256, 0, nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_, nullptr);
     link(k_finish_multi, 1, 32, 0, K, b_wFw_, b_gPz_, b_st_, b_hist_);
 }
 
@@ -825,14 +840,16 @@ void Engine::op_F_batch64(const double *w, double *Fw, const double *dotv, doubl
                                                  nullptr, 0.f);
     coarse_batch();
     symv_multi(d_F_, b_s_);
-    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, nullptr, Fw, dotv, partial);
+    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, nullptr, Fw, dotv, partial, nullptr,
+         nullptr);
 }
 
 void Engine::op_M_batch64(const double *x, double *z) {
     link(k_gather_multi, nslots_ / 32, 256, 0, nslots_, bK_, d_slot_ptr_, d_slot_ent_, x, d_weight_, b_xb_, nullptr,
                                                  nullptr, 0.f);
     symv_multi(d_S_, nullptr);
-    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, d_weight_, z, nullptr, nullptr);
+    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, d_weight_, z, nullptr, nullptr, nullptr,
+         nullptr);
 }
 
 // load cases [r0, r0 + kc) together: per-column results in run_.st, displacements in d_u_
@@ -864,7 +881,7 @@ int Engine::solve_chunk64(int r0, int kc, double &ms, std::string &err) {
     op_P_batch(b_g_, b_Pg_, b_alpha2_, nullptr, nullptr);
     op_M_batch64(b_Pg_, b_z_);
     op_P_batch(b_z_, b_Pz_, nullptr, b_g_, b_part_);
-    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_);
+    link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_, nullptr, nullptr, nullptr);
     CKB(cudaMemcpyAsync(b_w_, b_Pz_, nk * sizeof(double), cudaMemcpyDeviceToDevice, s_));
     launches_ += 18;
     std::vector<double> gPz(K);

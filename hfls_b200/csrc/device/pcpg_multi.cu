@@ -387,37 +387,47 @@ template __global__ void k_correct_multi<16>(const SubDev *, const ClusterDev *,
 template __global__ void k_correct_multi<32>(const SubDev *, const ClusterDev *, const double *, const int *,
                                              const double *, double *);
 
+// dot2v (with dotv): also the partials of dot2v . dotv into partial2
 __global__ void k_rows_multi(int nlam, int K, const int *__restrict__ rslot, const double *__restrict__ rsign,
-                             const double *yb, const double *__restrict__ weight,
-                             double *out, const double *dotv,
-                             double *partial) {
+                             const double *yb, const double *__restrict__ weight, double *out, const double *dotv,
+                             double *partial, const double *dot2v, double *partial2) {
     pdl_next();
     pdl_wait();
     const int rows_per_block = 256 / K;
     const int lr = threadIdx.x / K, j = threadIdx.x % K;
     const int stride = gridDim.x * rows_per_block;
-    double prod = 0.0;
+    double prod = 0.0, prod2 = 0.0;
     if (lr < rows_per_block)
         for (int r0 = blockIdx.x * rows_per_block; r0 < nlam; r0 += 2 * stride) {
             const int ra = r0 + lr, rb = r0 + stride + lr;
             const bool ha = ra < nlam, hb = rb < nlam;
-            double va = 0.0, vb = 0.0, da = 0.0, db = 0.0;
+            double va = 0.0, vb = 0.0, da = 0.0, db = 0.0, ga = 0.0, gb = 0.0;
             if (ha) va = row_value(ra, K, j, rslot, rsign, yb, weight);
             if (hb) vb = row_value(rb, K, j, rslot, rsign, yb, weight);
             if (dotv) {
                 if (ha) da = dotv[(size_t)ra * K + j];
                 if (hb) db = dotv[(size_t)rb * K + j];
             }
+            if (dot2v) {
+                if (ha) ga = dot2v[(size_t)ra * K + j];
+                if (hb) gb = dot2v[(size_t)rb * K + j];
+            }
             if (ha) {
                 out[(size_t)ra * K + j] = va;
                 if (dotv) prod += va * da;
+                if (dot2v) prod2 += ga * da;
             }
             if (hb) {
                 out[(size_t)rb * K + j] = vb;
                 if (dotv) prod += vb * db;
+                if (dot2v) prod2 += gb * db;
             }
         }
     if (partial) block_col_partial(prod, K, partial);
+    if (dot2v) {
+        __syncthreads();
+        block_col_partial(prod2, K, partial2);
+    }
 }
 
 // Gf^T x per chunk and column: partial[ch][q][j].  The chunk's row indices
@@ -516,17 +526,28 @@ __global__ void k_gf_coef_multi(int K, int ncl, const double *__restrict__ invGt
     if (alpha_out) alpha_out[(size_t)q * K + j] = -s;
 }
 
+// largest |v| of every column over the CTA's threads (thread t: column t % K) into xmax (FP32 bits, atomicMax)
+__device__ __forceinline__ void col_max(double v, int K, unsigned *xmax) {
+    __shared__ float red_max[256];
+    red_max[threadIdx.x] = (float)fabs(v);
+    __syncthreads();
+    if ((int)threadIdx.x < K) {
+        float m = red_max[threadIdx.x];
+        for (int t = threadIdx.x + K; t < (int)blockDim.x; t += K) m = fmaxf(m, red_max[t]);
+        if (m > 0.f) atomicMax(xmax + threadIdx.x, __float_as_uint(m));
+    }
+}
+
 // Px = x - Gf a; partial dot with dotv per (block, j); blocks stride over
 // row groups like k_rows_multi
 __global__ void k_gf_apply_multi(int nlam, int K, const double *a, const int *__restrict__ gcl,
                                  const double *__restrict__ gval, const double *x,
-                                 double *Px, const double *dotv,
-                                 double *partial) {
+                                 double *Px, const double *dotv, double *partial, unsigned *xmax) {
     pdl_next();
     pdl_wait();
     const int rows_per_block = 256 / K;
     const int lr = threadIdx.x / K, j = threadIdx.x % K;
-    double prod = 0.0;
+    double prod = 0.0, m = 0.0;
     for (int r0 = blockIdx.x * rows_per_block; r0 < nlam; r0 += gridDim.x * rows_per_block) {
         const int r = r0 + lr;
         if (lr < rows_per_block && r < nlam) {
@@ -540,10 +561,12 @@ __global__ void k_gf_apply_multi(int nlam, int K, const double *a, const int *__
             }
             const double pv = x[(size_t)r * K + j] - v;
             Px[(size_t)r * K + j] = pv;
+            m = fmax(m, fabs(pv));
             if (dotv) prod += pv * dotv[(size_t)r * K + j];
         }
     }
     if (partial) block_col_partial(prod, K, partial);
+    if (xmax) col_max(m, K, xmax);
 }
 
 // sum of partials of column j (fixed order), one CTA per column
@@ -562,12 +585,17 @@ __device__ double col_sum(const double *partial, int np, int K, int j) {
     return r;
 }
 
-// per column: scalar = sum of partials -> out[j]
-__global__ void k_colsum(const double *partial, int np, int K, double *out) {
+// per column: scalar = sum of partials -> out[j]; CTAs K .. 2 K - 1: of partial2 -> out2[j]; zero (2 K values, the
+// column maxima) is set to zero on the way
+__global__ void k_colsum(const double *partial, int np, int K, double *out, const double *partial2, double *out2,
+                         unsigned *zero) {
     pdl_next();
     pdl_wait();
-    const double s = col_sum(partial, np, K, blockIdx.x);
-    if (threadIdx.x == 0) out[blockIdx.x] = s;
+    const int j = blockIdx.x % K;
+    const bool second = blockIdx.x >= K;
+    const double s = col_sum(second ? partial2 : partial, np, K, j);
+    if (threadIdx.x == 0) (second ? out2 : out)[j] = s;
+    if (zero && blockIdx.x == 0 && threadIdx.x < 2 * K) zero[threadIdx.x] = 0;
 }
 
 // rho_j = -gPz_j / wFw_j ; lam += rho w ; g += rho Fw  (skips finished columns)
@@ -590,31 +618,26 @@ __global__ void k_update_lam_g_multi(int n, int K, const double *wFw, const doub
     g[id] += rho * Fw[id];
 }
 
-// partial[blk][j] = sum over the rows of block blk of a[r][j] * b[r][j]
-// (row groups of 256 / K rows, strided like k_rows_multi)
-__global__ void k_dot_multi(int nlam, int K, const double *a, const double *b,
-                            double *partial) {
+// w = Pz + gamma w (skips finished columns); with xmax also the column maxima of |w|, the scale of the next gather
+__global__ void __launch_bounds__(256) k_update_w_multi(int n, int K, const double *gPz_new, const double *Pz,
+                                                        double *w, const PcpgState *st, unsigned *xmax) {
     pdl_next();
     pdl_wait();
-    const int rows_per_block = 256 / K;
-    const int lr = threadIdx.x / K, j = threadIdx.x % K;
-    double prod = 0.0;
-    for (int r0 = blockIdx.x * rows_per_block; r0 < nlam; r0 += gridDim.x * rows_per_block) {
-        const int r = r0 + lr;
-        if (lr < rows_per_block && r < nlam) prod += a[(size_t)r * K + j] * b[(size_t)r * K + j];
+    const long long stride = (long long)gridDim.x * blockDim.x;      // a multiple of K
+    const long long id0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int j = int(id0 % K);
+    const bool run = !st[j].done;
+    const double gam = run ? gPz_new[j] / st[j].gPz : 0.0;
+    double m = 0.0;
+    for (long long id = id0; id < (long long)n * K; id += stride) {
+        double v = w[id];
+        if (run) {
+            v = Pz[id] + gam * v;
+            w[id] = v;
+        }
+        m = fmax(m, fabs(v));
     }
-    block_col_partial(prod, K, partial);
-}
-
-__global__ void k_update_w_multi(int n, int K, const double *gPz_new, const double *Pz,
-                                 double *w, const PcpgState *st) {
-    pdl_next();
-    pdl_wait();
-    const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (id >= (long long)n * K) return;
-    const int j = int(id % K);
-    if (st[j].done) return;
-    w[id] = Pz[id] + (gPz_new[j] / st[j].gPz) * w[id];
+    if (xmax) col_max(m, K, xmax);
 }
 
 // hist (FP64 form): relative residual of column j after iteration it at hist[it * K + j]

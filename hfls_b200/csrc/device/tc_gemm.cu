@@ -281,9 +281,10 @@ __global__ void __launch_bounds__(TC_THREADS, 2) k_tc_gemm(const GemmBlock *__re
             }
             // undo the scales: 2^-(EA + EX_j)
             const unsigned *amax = which == 0 ? ts.amaxF : ts.amaxS;
+            const unsigned *xmax = which == 0 ? ts.xmax : ts.xmaxS;
             const int ea = tc_scale_exp(amax[g.d], 1.0f);
 #pragma unroll
-            for (int j = 0; j < KH; ++j) acc[j] = ldexp(acc[j], -(ea + tc_scale_exp(ts.xmax[h * KH + j], ts.xbound)));
+            for (int j = 0; j < KH; ++j) acc[j] = ldexp(acc[j], -(ea + tc_scale_exp(xmax[h * KH + j], ts.xbound)));
             // the warp's 32 rows x KH columns through shared memory (row stride KH + 1
             // doubles; the stage buffers are idle: every copy landed before the last
             // MMA completed), stored as 32 segments of KH contiguous doubles
