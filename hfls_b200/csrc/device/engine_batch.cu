@@ -81,7 +81,6 @@ __global__ void k_add_R(const SubDev *, const ClusterDev *, const double *, cons
                         const double *, double *);
 __global__ void k_gather_u(int, const int *, const double *, double *);
 
-constexpr int GFT_SMEM = 1024 * (6 * 8 + 4);        // k_gft_partial_multi: one chunk's rows and Gf values
 
 static inline int cdivb(long long a, long long b) { return int((a + b - 1) / b); }
 
@@ -207,7 +206,6 @@ int Engine::setup_batch(int K, std::string &err) {
 // vectors of a batch of K load cases (mixed and FP64 form)
 int Engine::alloc_batch(int K, std::string &err) {
     int rc = HTF_OK;
-    CKB(cudaFuncSetAttribute(k_gft_partial_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, GFT_SMEM));
     // batch vectors
     const size_t nl = (size_t)nlam_ * K;
     int ntot = 0;
@@ -228,7 +226,7 @@ int Engine::alloc_batch(int K, std::string &err) {
     b_t_ = alloc<double>((size_t)ntot * vt_nch_ * K, err, rc);     // V^T x_b partials per 128-row chunk
     b_gc_ = alloc<double>((size_t)ngc_total_ * K, err, rc); b_s_ = alloc<double>((size_t)ngc_total_ * K, err, rc);
     b_part_ = alloc<double>((size_t)bnpart_ * K, err, rc); b_part2_ = alloc<double>((size_t)bnpart_ * K, err, rc);
-    b_gpart_ = alloc<double>((size_t)nchunks_ * 6 * K, err, rc);
+    b_gpart_ = alloc<double>((size_t)nchunks_ * 4 * 6 * K, err, rc);
     b_wFw_ = alloc<double>(K, err, rc); b_gPz_ = alloc<double>(K, err, rc);
     b_gw_ = alloc<double>(K, err, rc);
     b_gt_ = alloc<double>((size_t)6 * ncl_ * K, err, rc); b_acoef_ = alloc<double>((size_t)6 * ncl_ * K, err, rc);
@@ -331,7 +329,7 @@ void Engine::f_post(double *Fw, const double *dotv, double *partial, const doubl
     const dim3 gc(nsub_, cdivb(max_nbp_, 128));
     if (bK_ == 32) link(k_correct_multi<32>, gc, 256, 0, d_subs_, d_cl_, d_V_, d_bcr_, b_s_, b_yb_);
     else link(k_correct_multi<16>, gc, 256, 0, d_subs_, d_cl_, d_V_, d_bcr_, b_s_, b_yb_);
-    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, nullptr, Fw, dotv, partial, dot2v,
+    link(k_rows_multi, bnpart_, 128, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, nullptr, Fw, dotv, partial, dot2v,
          partial2);
 }
 
@@ -339,7 +337,7 @@ void Engine::f_post(double *Fw, const double *dotv, double *partial, const doubl
 void Engine::m_pre(const double *x) { gather_x(x, 1, nullptr); }
 
 void Engine::m_post(double *z) {
-    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, d_weight_, z, nullptr, nullptr, nullptr,
+    link(k_rows_multi, bnpart_, 128, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, d_weight_, z, nullptr, nullptr, nullptr,
          nullptr);
 }
 
@@ -360,10 +358,10 @@ void Engine::op_M_batch(const double *x, double *z) {
 void Engine::op_P_batch(const double *x, double *Px, double *alpha_out, const double *dotv, double *partial,
                         unsigned *xmax) {
     const int K = bK_;
-    link(k_gft_partial_multi, nchunks_, 256, GFT_SMEM, K, d_chunk_beg_, d_chunk_end_, d_crow_, d_cval_, x, b_gpart_);
-    link(k_gt_sum_multi, 6 * ncl_, K, 0, K, d_cl_chunk_ptr_, b_gpart_, b_gt_);
-    link(k_gf_coef_multi, 6 * ncl_, K, 0, K, ncl_, d_invGtG_, b_gt_, b_acoef_, alpha_out);
-    link(k_gf_apply_multi, bnpart_, 256, 0, nlam_, K, b_acoef_, d_gcl_, d_gval_, x, Px, dotv, partial, xmax);
+    link(k_gft_partial_multi, 4 * nchunks_, 64, 0, K, d_chunk_beg_, d_chunk_end_, d_crow_, d_cval_, x, b_gpart_);
+    link(k_gt_sum_multi, 6 * ncl_, 256, 0, K, d_cl_chunk_ptr_, b_gpart_, b_gt_);
+    link(k_gf_coef_multi, 6 * ncl_, 256, 0, K, ncl_, d_invGtG_, b_gt_, b_acoef_, alpha_out);
+    link(k_gf_apply_multi, bnpart_, 128, 0, nlam_, K, b_acoef_, d_gcl_, d_gval_, x, Px, dotv, partial, xmax);
 }
 
 // one batched iteration = iter_a | F product | iter_b | S product | iter_c
@@ -375,7 +373,7 @@ void Engine::iter_b() {
     // w'Fw and g'w; the maxima of this iteration's w and of the last P g have been used: set to zero
     f_post(b_Fw_, b_w_, b_part_, b_g_, b_part2_);
     link(k_colsum, 2 * K, 256, 0, b_part_, bnpart_, K, b_wFw_, b_part2_, b_gw_, d_xmax_);
-    link(k_update_lam_g_multi, nk, 256, 0, nlam_, K, b_wFw_, b_gw_, b_w_, b_Fw_, b_lam_, b_g_, b_st_);
+    link(k_update_lam_g_multi, nk, 128, 0, nlam_, K, b_wFw_, b_gw_, b_w_, b_Fw_, b_lam_, b_g_, b_st_);
     op_P_batch(b_g_, b_Pg_, nullptr, nullptr, nullptr, d_xmax_ + K);
     m_pre(b_Pg_);
 }
@@ -385,7 +383,7 @@ void Engine::iter_c() {
     m_post(b_z_);
     op_P_batch(b_z_, b_Pz_, nullptr, b_g_, b_part_);
     link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_, nullptr, nullptr, nullptr);
-    link(k_update_w_multi, std::min(cdivb((long long)nlam_ * K, 256), 1184), 256, 0, nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_,
+    link(k_update_w_multi, std::min(cdivb((long long)nlam_ * K, 256), 1184), 128, 0, nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_,
          d_xmax_);
     link(k_finish_multi, 1, 32, 0, K, b_wFw_, b_gPz_, b_st_, nullptr);
 }
@@ -457,7 +455,7 @@ int Engine::fp64_residual_batch(const std::vector<int> &sel, const std::vector<i
                                                  nullptr, 0.f);
     coarse_batch();
     symv_multi(d_F_, b_s_);
-    link(k_rows_multi, bnpart_, 256, 0, nlam_, K, d_rslot_, d_rsign_, b_yb_, nullptr, b_tmp_, nullptr, nullptr, nullptr,
+    link(k_rows_multi, bnpart_, 128, 0, nlam_, K, d_rslot_, d_rsign_, b_yb_, nullptr, b_tmp_, nullptr, nullptr, nullptr,
          nullptr);
     k_axpby<<<cdivb(nk, 256), 256, 0, s_>>>(int(nk), -1.0, b_d_, 1.0, b_tmp_);
     op_P_batch(b_tmp_, b_Pg_, b_alpha2_, nullptr, nullptr);
@@ -466,7 +464,7 @@ int Engine::fp64_residual_batch(const std::vector<int> &sel, const std::vector<i
         link(k_gather_multi, nslots_ / 32, 256, 0, nslots_, K, d_slot_ptr_, d_slot_ent_, b_Pg_, d_weight_, b_xb_,
                                                      nullptr, nullptr, 0.f);
         symv_multi(d_S_, nullptr);
-        link(k_rows_multi, bnpart_, 256, 0, nlam_, K, d_rslot_, d_rsign_, b_yb_, d_weight_, b_z_, nullptr, nullptr, nullptr,
+        link(k_rows_multi, bnpart_, 128, 0, nlam_, K, d_rslot_, d_rsign_, b_yb_, d_weight_, b_z_, nullptr, nullptr, nullptr,
          nullptr);
     } else {
         op_M_batch(b_Pg_, b_z_);      // S_i only as tensor-core slabs: the tensor-core product
@@ -826,12 +824,12 @@ void Engine::iteration_batch64() {
     const int nk = cdivb((long long)nlam_ * K, 256);
     op_F_batch64(b_w_, b_Fw_, b_w_, b_part_);
     link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_wFw_, nullptr, nullptr, nullptr);
-    link(k_update_lam_g_multi, nk, 256, 0, nlam_, K, b_wFw_, nullptr, b_w_, b_Fw_, b_lam_, b_g_, b_st_);
+    link(k_update_lam_g_multi, nk, 128, 0, nlam_, K, b_wFw_, nullptr, b_w_, b_Fw_, b_lam_, b_g_, b_st_);
     op_P_batch(b_g_, b_Pg_, b_alpha2_, nullptr, nullptr);
     op_M_batch64(b_Pg_, b_z_);
     op_P_batch(b_z_, b_Pz_, nullptr, b_g_, b_part_);
     link(k_colsum, K, 256, 0, b_part_, bnpart_, K, b_gPz_, nullptr, nullptr, nullptr);
-    link(k_update_w_multi, std::min(nk, 1184), 256, 0, nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_, nullptr);
+    link(k_update_w_multi, std::min(nk, 1184), 128, 0, nlam_, K, b_gPz_, b_Pz_, b_w_, b_st_, nullptr);
     link(k_finish_multi, 1, 32, 0, K, b_wFw_, b_gPz_, b_st_, b_hist_);
 }
 
@@ -840,7 +838,7 @@ void Engine::op_F_batch64(const double *w, double *Fw, const double *dotv, doubl
                                                  nullptr, 0.f);
     coarse_batch();
     symv_multi(d_F_, b_s_);
-    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, nullptr, Fw, dotv, partial, nullptr,
+    link(k_rows_multi, bnpart_, 128, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, nullptr, Fw, dotv, partial, nullptr,
          nullptr);
 }
 
@@ -848,7 +846,7 @@ void Engine::op_M_batch64(const double *x, double *z) {
     link(k_gather_multi, nslots_ / 32, 256, 0, nslots_, bK_, d_slot_ptr_, d_slot_ent_, x, d_weight_, b_xb_, nullptr,
                                                  nullptr, 0.f);
     symv_multi(d_S_, nullptr);
-    link(k_rows_multi, bnpart_, 256, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, d_weight_, z, nullptr, nullptr, nullptr,
+    link(k_rows_multi, bnpart_, 128, 0, nlam_, bK_, d_rslot_, d_rsign_, b_yb_, d_weight_, z, nullptr, nullptr, nullptr,
          nullptr);
 }
 

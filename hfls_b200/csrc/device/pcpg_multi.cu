@@ -27,44 +27,81 @@ __device__ __forceinline__ void dmma_8x8x4(double &d0, double &d1, double a, dou
 // then the lo plane, SWIZZLE_64B K-major.  One CTA per 32 consecutive slots
 // (one K slab of one subdomain: b offsets and padded sizes are multiples of
 // 32); the values go through shared memory so both outputs are written
-// coalesced.
-__global__ void k_gather_multi(int nslots, int K, const int *__restrict__ ptr, const int *__restrict__ ent,
-                               const double *w, const double *__restrict__ weight,
-                               double *xb, float *__restrict__ Xs, const unsigned *xmax,
-                               float xbound) {
-    pdl_next();
-    pdl_wait();
+// coalesced.  Two columns per thread and two slots per conversion (64 uneven
+// subdomains, 32 columns, 1 964 CTAs, about 45 MB in L2): 17.1 -> 13.6 us.
+__global__ void __launch_bounds__(256) k_gather_multi(int nslots, int K, const int *__restrict__ ptr,
+                                                      const int *__restrict__ ent, const double *w,
+                                                      const double *__restrict__ weight, double *xb,
+                                                      float *__restrict__ Xs, const unsigned *xmax, float xbound) {
     __shared__ double vs[32 * 33];
-    __shared__ int ex[32];
+    __shared__ double sc[32];
     const int i0 = blockIdx.x * 32;
-    for (int o = threadIdx.x; o < 32 * K; o += blockDim.x) {
-        const int il = o / K, j = o % K, i = i0 + il;
-        double v = 0.0;
-        if (i < nslots)
-            for (int e = ptr[i]; e < ptr[i + 1]; ++e) {
-                const int q = ent[e];
-                const int lam = q >> 1;
-                double a = w[(size_t)lam * K + j];
-                if (weight) a *= weight[lam];
-                v += (q & 1) ? -a : a;
+    pdl_next();
+    const int K2 = K / 2, j2 = threadIdx.x % K2;    // a thread makes two columns of one or two slots
+    int e0[2], e1[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int i = i0 + (int(threadIdx.x) + 256 * u) / K2;
+        const bool here = 256 * u < 32 * K2 && i < nslots;
+        e0[u] = here ? ptr[i] : 0;
+        e1[u] = here ? ptr[i + 1] : 0;
+    }
+    pdl_wait();
+    const double2 *w2 = reinterpret_cast<const double2 *>(w) + j2;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        if (256 * u >= 32 * K2) break;
+        const int il = (int(threadIdx.x) + 256 * u) / K2, i = i0 + il;
+        // a face slot has one entry, an edge slot three: their loads are in flight together
+        int q[3];
+        double2 v = make_double2(0.0, 0.0), a[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) q[k] = e0[u] + k < e1[u] ? ent[e0[u] + k] : -1;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            a[k] = q[k] >= 0 ? w2[(size_t)(q[k] >> 1) * K2] : make_double2(0.0, 0.0);
+            if (weight && q[k] >= 0) {
+                const double wt = weight[q[k] >> 1];
+                a[k].x *= wt;
+                a[k].y *= wt;
             }
-        if (xb && i < nslots) xb[(size_t)i * K + j] = v;
-        vs[il * 33 + j] = v;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (q[k] >= 0) {
+                v.x += (q[k] & 1) ? -a[k].x : a[k].x;
+                v.y += (q[k] & 1) ? -a[k].y : a[k].y;
+            }
+        for (int e = e0[u] + 3; e < e1[u]; ++e) {
+            const int qe = ent[e], lam = qe >> 1;
+            double2 ae = w2[(size_t)lam * K2];
+            if (weight) {
+                ae.x *= weight[lam];
+                ae.y *= weight[lam];
+            }
+            v.x += (qe & 1) ? -ae.x : ae.x;
+            v.y += (qe & 1) ? -ae.y : ae.y;
+        }
+        if (xb && i < nslots) reinterpret_cast<double2 *>(xb)[(size_t)i * K2 + j2] = v;
+        vs[il * 33 + 2 * j2] = v.x;
+        vs[il * 33 + 2 * j2 + 1] = v.y;
     }
     if (!Xs) return;
-    if (threadIdx.x < K) ex[threadIdx.x] = tc_scale_exp(xmax[threadIdx.x], xbound);
+    // 2^EX_j, a normal FP64 number (EX_j comes from an FP32 value)
+    if (threadIdx.x < K) sc[threadIdx.x] = __hiloint2double((1023 + tc_scale_exp(xmax[threadIdx.x], xbound)) << 20, 0);
     __syncthreads();
-    // row j (load case) of each plane holds the 32 slots of this chunk, 64 bytes
-    __half *hi = reinterpret_cast<__half *>(Xs + (size_t)i0 * K);
-    __half *lo = hi + 32 * K;
-    for (int o = threadIdx.x; o < 32 * K; o += blockDim.x) {
-        const int j = o / 32, c = o % 32;
-        const double v = ldexp(vs[c * 33 + j], ex[j]);
-        const __half vh = __double2half(v);
-        const uint32_t b = uint32_t(j * 64 + c * 2);
-        const uint32_t bs = b ^ (((b >> 7) & 3u) << 4);
-        hi[bs / 2] = vh;
-        lo[bs / 2] = __double2half(v - (double)__half2float(vh));
+    // row j (load case) of each plane holds the 32 slots of this chunk, 64 bytes; a thread makes two slots of it
+    __half2 *hi = reinterpret_cast<__half2 *>(Xs + (size_t)i0 * K);
+    __half2 *lo = hi + 16 * K;
+    for (int o = threadIdx.x; o < 16 * K; o += blockDim.x) {
+        const int row = o / 16, c = 2 * (o % 16);
+        const double v0 = vs[c * 33 + row] * sc[row], v1 = vs[(c + 1) * 33 + row] * sc[row];
+        const __half h0 = __double2half(v0), h1 = __double2half(v1);
+        const uint32_t b = uint32_t(row * 64 + c * 2);
+        const uint32_t bs = (b ^ (((b >> 7) & 3u) << 4)) / 4;
+        hi[bs] = __halves2half2(h0, h1);
+        lo[bs] = __halves2half2(__double2half(v0 - (double)__half2float(h0)),
+                                __double2half(v1 - (double)__half2float(h1)));
     }
 }
 
@@ -167,13 +204,26 @@ HTF_VT(32, 64)
 __global__ void k_gc_multi(int ngc_total, int K, int nch, const int *__restrict__ gptr, const int *__restrict__ gidx,
                            const double *tpart, double *gc) {
     pdl_next();
-    pdl_wait();
     const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (id >= (long long)ngc_total * K) return;
+    const bool here = id < (long long)ngc_total * K;
     const int q = int(id / K), j = int(id % K);
+    const int e0 = here ? gptr[q] : 0, e1 = here ? gptr[q + 1] : 0;
+    int t = e0 < e1 ? gidx[e0] : 0;                 // the entry after this one is read ahead
+    pdl_wait();
+    if (!here) return;
     double s = 0.0;
-    for (int e = gptr[q]; e < gptr[q + 1]; ++e)
-        for (int ch = 0; ch < nch; ++ch) s += tpart[((size_t)gidx[e] * nch + ch) * K + j];
+    constexpr int U = 8;                            // chunks in flight
+    for (int e = e0; e < e1; ++e) {
+        const double *tp = tpart + (size_t)t * nch * K + j;
+        if (e + 1 < e1) t = gidx[e + 1];
+        for (int c0 = 0; c0 < nch; c0 += U) {
+            double v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = c0 + u < nch ? tp[(size_t)(c0 + u) * K] : 0.0;
+#pragma unroll
+            for (int u = 0; u < U; ++u) s += v[u];
+        }
+    }
     gc[(size_t)q * K + j] = s;
 }
 
@@ -256,34 +306,56 @@ __global__ void __launch_bounds__(128) k_coarse_multi(const ClusterDev *__restri
 template __global__ void k_coarse_multi<16>(const ClusterDev *, const double *, const double *, double *);
 template __global__ void k_coarse_multi<32>(const ClusterDev *, const double *, const double *, double *);
 
-// per-block, per-column tree sum of prod over the block's rows (256 / K rows,
-// threads j, j+K, ...) -> partial[block][j]
-__device__ __forceinline__ void block_col_partial(double prod, int K, double *partial) {
-    __shared__ double red[256];
-    const int rows_per_block = 256 / K;
-    const int lr = threadIdx.x / K, j = threadIdx.x % K;
-    red[threadIdx.x] = prod;
+// The row kernels below (k_rows_multi, k_gf_apply_multi, the updates) run 128
+// threads, thread (lr, j2) the columns 2 j2 and 2 j2 + 1 of the rows
+// lr, lr + 256 / K, ...: 16-byte accesses, half the instructions per byte of
+// one column per thread, by which these kernels (vectors in L2) are bound.  One
+// column per thread -> two, alone: 64 uneven subdomains, 32 columns:
+// k_gf_apply_multi 14.7 -> 10.4 us, updates 11.0 -> 9.3 and 10.6 -> 8.3,
+// k_rows_multi 10.1 -> 10.7; 32 uneven subdomains, 8 load cases in 16 columns:
+// 6.3 -> 5.0, 5.5 -> 4.6, 5.3 -> 5.1, 5.2 -> 4.4 us.
+
+// per-block, per-column tree sum of prod over the block's 256 / K rows -> partial[block][j]
+__device__ __forceinline__ void block_col_partial(double2 prod, int K, double *partial) {
+    __shared__ double2 red[128];
+    const int K2 = K / 2, lr = threadIdx.x / K2, tid = threadIdx.x;
+    red[tid] = prod;
     __syncthreads();
-    for (int o = rows_per_block / 2; o > 0; o >>= 1) {
-        if (lr < o) red[threadIdx.x] += red[threadIdx.x + o * K];
+    for (int o = 128 / K; o > 0; o >>= 1) {
+        if (lr < o) {
+            red[tid].x += red[tid + o * K2].x;
+            red[tid].y += red[tid + o * K2].y;
+        }
         __syncthreads();
     }
-    if (lr == 0) partial[(size_t)blockIdx.x * K + j] = red[j];
+    if (lr == 0) reinterpret_cast<double2 *>(partial)[(size_t)blockIdx.x * K2 + tid] = red[tid];
 }
 
 // out[r][j] = wt[r] * sum_k sign * y[slot][j]; partial dot with dotv per
 // (block, j).  Blocks stride over groups of 256 / K rows (fixed assignment,
 // so the partials and their sums are the same on every run); each thread
 // has the loads of two of its rows in flight and adds them in row order.
-__device__ __forceinline__ double row_value(int r, int K, int j, const int *__restrict__ rslot,
-                                            const double *__restrict__ rsign, const double *yb,
-                                            const double *__restrict__ weight) {
+__device__ __forceinline__ double2 row_value(int r, int K2, const int *__restrict__ rslot,
+                                             const double *__restrict__ rsign, const double2 *yb,
+                                             const double *__restrict__ weight) {
     const int2 sl = reinterpret_cast<const int2 *>(rslot)[r];
     const double2 sg = reinterpret_cast<const double2 *>(rsign)[r];
-    double v = 0.0;
-    if (sl.x >= 0) v += sg.x * yb[(size_t)sl.x * K + j];
-    if (sl.y >= 0) v += sg.y * yb[(size_t)sl.y * K + j];
-    if (weight) v *= weight[r];
+    const double wt = weight ? weight[r] : 1.0;
+    const double2 zero = make_double2(0.0, 0.0);
+    const double2 y0 = sl.x >= 0 ? yb[(size_t)sl.x * K2] : zero, y1 = sl.y >= 0 ? yb[(size_t)sl.y * K2] : zero;
+    double2 v = zero;
+    if (sl.x >= 0) {
+        v.x += sg.x * y0.x;
+        v.y += sg.x * y0.y;
+    }
+    if (sl.y >= 0) {
+        v.x += sg.y * y1.x;
+        v.y += sg.y * y1.y;
+    }
+    if (weight) {
+        v.x *= wt;
+        v.y *= wt;
+    }
     return v;
 }
 
@@ -388,41 +460,47 @@ template __global__ void k_correct_multi<32>(const SubDev *, const ClusterDev *,
                                              const double *, double *);
 
 // dot2v (with dotv): also the partials of dot2v . dotv into partial2
-__global__ void k_rows_multi(int nlam, int K, const int *__restrict__ rslot, const double *__restrict__ rsign,
-                             const double *yb, const double *__restrict__ weight, double *out, const double *dotv,
-                             double *partial, const double *dot2v, double *partial2) {
+__global__ void __launch_bounds__(128) k_rows_multi(int nlam, int K, const int *__restrict__ rslot,
+                                                    const double *__restrict__ rsign, const double *yb,
+                                                    const double *__restrict__ weight, double *out,
+                                                    const double *dotv, double *partial, const double *dot2v,
+                                                    double *partial2) {
     pdl_next();
     pdl_wait();
-    const int rows_per_block = 256 / K;
-    const int lr = threadIdx.x / K, j = threadIdx.x % K;
+    const int rows_per_block = 256 / K, K2 = K / 2;
+    const int lr = threadIdx.x / K2, j2 = threadIdx.x % K2;
     const int stride = gridDim.x * rows_per_block;
-    double prod = 0.0, prod2 = 0.0;
-    if (lr < rows_per_block)
-        for (int r0 = blockIdx.x * rows_per_block; r0 < nlam; r0 += 2 * stride) {
-            const int ra = r0 + lr, rb = r0 + stride + lr;
-            const bool ha = ra < nlam, hb = rb < nlam;
-            double va = 0.0, vb = 0.0, da = 0.0, db = 0.0, ga = 0.0, gb = 0.0;
-            if (ha) va = row_value(ra, K, j, rslot, rsign, yb, weight);
-            if (hb) vb = row_value(rb, K, j, rslot, rsign, yb, weight);
+    const double2 *y2 = reinterpret_cast<const double2 *>(yb) + j2;
+    const double2 *d2 = reinterpret_cast<const double2 *>(dotv) + j2;
+    const double2 *g2 = reinterpret_cast<const double2 *>(dot2v) + j2;
+    double2 *o2 = reinterpret_cast<double2 *>(out) + j2;
+    const double2 zero = make_double2(0.0, 0.0);
+    double2 prod = zero, prod2 = zero;
+    for (int r0 = blockIdx.x * rows_per_block; r0 < nlam; r0 += 2 * stride) {
+        double2 v[2], d[2], g[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int r = r0 + k * stride + lr;
+            const bool here = r < nlam;
+            v[k] = here ? row_value(r, K2, rslot, rsign, y2, weight) : zero;
+            d[k] = here && dotv ? d2[(size_t)r * K2] : zero;
+            g[k] = here && dot2v ? g2[(size_t)r * K2] : zero;
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int r = r0 + k * stride + lr;
+            if (r >= nlam) continue;
+            o2[(size_t)r * K2] = v[k];
             if (dotv) {
-                if (ha) da = dotv[(size_t)ra * K + j];
-                if (hb) db = dotv[(size_t)rb * K + j];
+                prod.x += v[k].x * d[k].x;
+                prod.y += v[k].y * d[k].y;
             }
             if (dot2v) {
-                if (ha) ga = dot2v[(size_t)ra * K + j];
-                if (hb) gb = dot2v[(size_t)rb * K + j];
-            }
-            if (ha) {
-                out[(size_t)ra * K + j] = va;
-                if (dotv) prod += va * da;
-                if (dot2v) prod2 += ga * da;
-            }
-            if (hb) {
-                out[(size_t)rb * K + j] = vb;
-                if (dotv) prod += vb * db;
-                if (dot2v) prod2 += gb * db;
+                prod2.x += g[k].x * d[k].x;
+                prod2.y += g[k].y * d[k].y;
             }
         }
+    }
     if (partial) block_col_partial(prod, K, partial);
     if (dot2v) {
         __syncthreads();
@@ -430,139 +508,190 @@ __global__ void k_rows_multi(int nlam, int K, const int *__restrict__ rslot, con
     }
 }
 
-// Gf^T x per chunk and column: partial[ch][q][j].  The chunk's row indices
-// and Gf values (up to 1024 entries) are staged in shared memory at once;
-// thread (lr, j) walks every (256/K)-th entry with sixteen x loads in flight,
-// adding its entries in the order lr, lr + 256/K, ...; the 6 sums are then
-// reduced over lr in one pass through shared memory.  Bound by the latency of
-// the x loads, a row of K values each.
-constexpr int GFT_CHUNK = 1024;                    // most entries of a chunk
-__global__ void __launch_bounds__(256) k_gft_partial_multi(int K, const int *__restrict__ chunk_beg,
-                                                           const int *__restrict__ chunk_end,
-                                                           const int *__restrict__ crow,
-                                                           const double *__restrict__ cval,
-                                                           const double *x,
-                                                           double *partial) {
-    extern __shared__ double gft_sm[];
-    double *cs = gft_sm;                            // [6 GFT_CHUNK]; then [6][256] sums
-    int *rs = reinterpret_cast<int *>(gft_sm + 6 * GFT_CHUNK);
-    const int ch = blockIdx.x;
-    const int j = threadIdx.x % K, nl = 256 / K, lr = threadIdx.x / K;
-    const int beg = chunk_beg[ch], n = chunk_end[ch] - beg;
+// Gf^T x per chunk and column.  Of the 256 / K interleaved sums of a chunk
+// (entries lr, lr + 256/K, ...) CTA (chunk, p) makes those with lr % 4 == p:
+// its rows and Gf values (up to 256 entries) are staged in shared memory before
+// the wait, thread (lr / 4, j) walks its entries with 32 x loads in flight, and
+// the sums are added as a tree; k_gt_sum_multi adds the four parts the same
+// way.  Bound by the latency of the x loads, a row of K values each: 60 chunks
+// are 240 CTAs in four parts.  64 uneven subdomains, 32 columns (60 chunks),
+// alone: 15.8 us with one CTA per chunk, 9.8 us in parts.
+constexpr int GFT_PART = 1024 / 4;                 // most entries of a part of a chunk
+__global__ void __launch_bounds__(64) k_gft_partial_multi(int K, const int *__restrict__ chunk_beg,
+                                                          const int *__restrict__ chunk_end,
+                                                          const int *__restrict__ crow,
+                                                          const double *__restrict__ cval,
+                                                          const double *x,
+                                                          double *partial) {
+    __shared__ double2 cs[3 * GFT_PART];            // then [6][64] sums
+    __shared__ int rs[GFT_PART];
+    const int ch = blockIdx.x / 4, p = blockIdx.x % 4, tid = threadIdx.x;
+    const int j = tid % K, nl = 64 / K, lr = tid / K;
+    const int beg = chunk_beg[ch] + p, n = (chunk_end[ch] - beg + 3) / 4;
     pdl_next();
-    const double2 *cv2 = reinterpret_cast<const double2 *>(cval + 6 * (size_t)beg);
+    const double2 *cv = reinterpret_cast<const double2 *>(cval);
 #pragma unroll
-    for (int u = 0; u < GFT_CHUNK / 256; ++u) {
-        const int o = int(threadIdx.x) + 256 * u;
-        if (o < n) rs[o] = crow[beg + o];
+    for (int u = 0; u < GFT_PART / 64; ++u) {       // missing entries: zeros
+        const int o = tid + 64 * u;
+        rs[o] = o < n ? crow[beg + 4 * o] : -1;
     }
 #pragma unroll
-    for (int u = 0; u < 3 * GFT_CHUNK / 256; ++u) {
-        const int o = int(threadIdx.x) + 256 * u;
-        if (o < 3 * n) reinterpret_cast<double2 *>(cs)[o] = cv2[o];
+    for (int u = 0; u < 3 * GFT_PART / 64; ++u) {
+        const int o = tid + 64 * u, e = o / 3;
+        cs[o] = e < n ? cv[3 * (size_t)(beg + 4 * e) + o % 3] : make_double2(0.0, 0.0);
     }
     pdl_wait();
     __syncthreads();
     double s[6] = {0, 0, 0, 0, 0, 0};
-    constexpr int U = 16;
-    int e = lr;
-    for (; e + (U - 1) * nl < n; e += U * nl) {
+    constexpr int U = 32;                           // of at most 128 (K = 32) or 64 entries per thread
+    for (int e0 = lr; e0 < n; e0 += U * nl) {
         double xv[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) xv[u] = x[(size_t)rs[e + u * nl] * K + j];
+        for (int u = 0; u < U; ++u) {
+            const int r = rs[e0 + u * nl];
+            xv[u] = r >= 0 ? x[(size_t)r * K + j] : 0.0;
+        }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const double *cv = cs + 6 * (e + u * nl);
+            const double2 *c = cs + 3 * (e0 + u * nl);
 #pragma unroll
-            for (int q = 0; q < 6; ++q) s[q] += cv[q] * xv[u];
+            for (int q = 0; q < 3; ++q) {
+                s[2 * q] += c[q].x * xv[u];
+                s[2 * q + 1] += c[q].y * xv[u];
+            }
         }
     }
-    for (; e < n; e += nl) {
-        const double xv = x[(size_t)rs[e] * K + j];
-#pragma unroll
-        for (int q = 0; q < 6; ++q) s[q] += cs[6 * e + q] * xv;
-    }
     __syncthreads();                                // the staged values are consumed
-    double *red = cs;
+    double *red = reinterpret_cast<double *>(cs);
 #pragma unroll
-    for (int q = 0; q < 6; ++q) red[q * 256 + threadIdx.x] = s[q];
+    for (int q = 0; q < 6; ++q) red[q * 64 + tid] = s[q];
     __syncthreads();
     for (int o = nl / 2; o > 0; o >>= 1) {
         if (lr < o)
 #pragma unroll
-            for (int q = 0; q < 6; ++q) red[q * 256 + threadIdx.x] += red[q * 256 + threadIdx.x + o * K];
+            for (int q = 0; q < 6; ++q) red[q * 64 + tid] += red[q * 64 + tid + o * K];
         __syncthreads();
     }
     if (lr == 0)
 #pragma unroll
-        for (int q = 0; q < 6; ++q) partial[((size_t)ch * 6 + q) * K + j] = red[q * 256 + j];
+        for (int q = 0; q < 6; ++q) partial[((size_t)blockIdx.x * 6 + q) * K + j] = red[q * 64 + j];
 }
 
 // gt[c][i][j] = sum of the chunk partials of cluster c (in chunk order); CTA
-// (cluster, mode i), thread j
-__global__ void k_gt_sum_multi(int K, const int *__restrict__ cl_chunk_ptr, const double *gpart,
-                               double *gt) {
+// (cluster, mode i): 32 chunks at a time are read by all threads (four parts
+// each, as a tree) and added in order by thread j
+__global__ void __launch_bounds__(256) k_gt_sum_multi(int K, const int *__restrict__ cl_chunk_ptr,
+                                                      const double *gpart, double *gt) {
+    __shared__ double v[32 * 32];
     pdl_next();
+    const int c = blockIdx.x / 6, i = blockIdx.x % 6, j = threadIdx.x % K, lr = threadIdx.x / K, nl = 256 / K;
+    const int beg = cl_chunk_ptr[c], end = cl_chunk_ptr[c + 1];
     pdl_wait();
-    const int c = blockIdx.x / 6, i = blockIdx.x % 6, j = threadIdx.x;
     double s = 0.0;
-#pragma unroll 8
-    for (int chk = cl_chunk_ptr[c]; chk < cl_chunk_ptr[c + 1]; ++chk) s += gpart[((size_t)chk * 6 + i) * K + j];
-    gt[(size_t)blockIdx.x * K + j] = s;
+    for (int c0 = beg; c0 < end; c0 += 32) {
+        const int n = min(32, end - c0);
+#pragma unroll 4
+        for (int o = lr; o < n; o += nl) {
+            const double *g = gpart + ((size_t)(c0 + o) * 24 + i) * K + j;
+            v[o * K + j] = (g[0] + g[12 * K]) + (g[6 * K] + g[18 * K]);
+        }
+        __syncthreads();
+        if (lr == 0)
+            for (int o = 0; o < n; ++o) s += v[o * K + j];
+        __syncthreads();
+    }
+    if (lr == 0) gt[(size_t)blockIdx.x * K + j] = s;
 }
 
 // a = (Gf^T Gf)^{-1} gt per column (gt = Gf^T x from k_gt_sum_multi), CTA per
-// row, thread per column; alpha_out = -a when requested.  (All rows in one
-// CTA: 23.7 us for 8 clusters and 32 load cases, 2.9 us here.)
-__global__ void k_gf_coef_multi(int K, int ncl, const double *__restrict__ invGtG, const double *gt,
-                                double *a, double *alpha_out) {
+// row: 64 entries of gt at a time are read by all threads and multiplied in
+// order by thread j; alpha_out = -a when requested.  8 clusters, 32 load cases,
+// alone: all rows in one CTA 23.7 us, one warp per row with its loads in
+// rounds of 16 8.7 us, 4.5 us here.
+__global__ void __launch_bounds__(256) k_gf_coef_multi(int K, int ncl, const double *__restrict__ invGtG,
+                                                       const double *gt, double *a, double *alpha_out) {
+    __shared__ double gs[64 * 32], is[64];
     pdl_next();
-    pdl_wait();
     const int m = 6 * ncl, q = blockIdx.x, j = threadIdx.x;
+    if (j < min(64, m)) is[j] = invGtG[q + (size_t)j * m];
+    pdl_wait();
     double s = 0.0;
-#pragma unroll 16
-    for (int p = 0; p < m; ++p) s += invGtG[q + (size_t)p * m] * gt[(size_t)p * K + j];
+    for (int p0 = 0; p0 < m; p0 += 64) {
+        const int n = min(64, m - p0);
+        if (p0 && j < n) is[j] = invGtG[q + (size_t)(p0 + j) * m];
+#pragma unroll 8
+        for (int o = j; o < n * K; o += 256) gs[o] = gt[(size_t)p0 * K + o];
+        __syncthreads();
+        if (j < K)
+#pragma unroll 8
+            for (int p = 0; p < n; ++p) s += is[p] * gs[p * K + j];
+        __syncthreads();
+    }
+    if (j >= K) return;
     a[(size_t)q * K + j] = s;
     if (alpha_out) alpha_out[(size_t)q * K + j] = -s;
 }
 
-// largest |v| of every column over the CTA's threads (thread t: column t % K) into xmax (FP32 bits, atomicMax)
-__device__ __forceinline__ void col_max(double v, int K, unsigned *xmax) {
+// largest values m of the columns over the CTA's 128 threads into xmax (FP32 bits, atomicMax)
+__device__ __forceinline__ void col_max(double2 m, int K, unsigned *xmax) {
     __shared__ float red_max[256];
-    red_max[threadIdx.x] = (float)fabs(v);
+    red_max[2 * threadIdx.x] = (float)m.x;
+    red_max[2 * threadIdx.x + 1] = (float)m.y;
     __syncthreads();
     if ((int)threadIdx.x < K) {
-        float m = red_max[threadIdx.x];
-        for (int t = threadIdx.x + K; t < (int)blockDim.x; t += K) m = fmaxf(m, red_max[t]);
-        if (m > 0.f) atomicMax(xmax + threadIdx.x, __float_as_uint(m));
+        float v = red_max[threadIdx.x];
+        for (int t = threadIdx.x + K; t < 256; t += K) v = fmaxf(v, red_max[t]);
+        if (v > 0.f) atomicMax(xmax + threadIdx.x, __float_as_uint(v));
     }
 }
 
 // Px = x - Gf a; partial dot with dotv per (block, j); blocks stride over
-// row groups like k_rows_multi
-__global__ void k_gf_apply_multi(int nlam, int K, const double *a, const int *__restrict__ gcl,
-                                 const double *__restrict__ gval, const double *x,
-                                 double *Px, const double *dotv, double *partial, unsigned *xmax) {
+// row groups like k_rows_multi.  A row's clusters are read one step ahead, so
+// that a step is one round of loads.
+__global__ void __launch_bounds__(128) k_gf_apply_multi(int nlam, int K, const double *a, const int *__restrict__ gcl,
+                                                        const double *__restrict__ gval, const double *x,
+                                                        double *Px, const double *dotv, double *partial,
+                                                        unsigned *xmax) {
     pdl_next();
+    const int K2 = K / 2, lr = threadIdx.x / K2, j2 = threadIdx.x % K2;
+    const int2 *cl = reinterpret_cast<const int2 *>(gcl);
+    const double2 *x2 = reinterpret_cast<const double2 *>(x) + j2, *d2 = reinterpret_cast<const double2 *>(dotv) + j2;
+    const double2 *a2 = reinterpret_cast<const double2 *>(a) + j2;
+    double2 *p2 = reinterpret_cast<double2 *>(Px) + j2;
+    const int stride = gridDim.x * (256 / K);
+    int r = blockIdx.x * (256 / K) + lr;
+    int2 c = make_int2(-1, -1);
+    if (r < nlam) c = cl[r];
     pdl_wait();
-    const int rows_per_block = 256 / K;
-    const int lr = threadIdx.x / K, j = threadIdx.x % K;
-    double prod = 0.0, m = 0.0;
-    for (int r0 = blockIdx.x * rows_per_block; r0 < nlam; r0 += gridDim.x * rows_per_block) {
-        const int r = r0 + lr;
-        if (lr < rows_per_block && r < nlam) {
-            double v = 0.0;
-            for (int k = 0; k < 2; ++k) {
-                const int c = gcl[2 * r + k];
-                if (c < 0) continue;
-                const double *g = gval + 6 * (size_t)(2 * r + k);
+    const double2 zero = make_double2(0.0, 0.0);
+    double2 prod = zero, m = zero;
+    for (; r < nlam; r += stride) {
+        const int2 now = c;
+        const double2 xv = x2[(size_t)r * K2], dv = dotv ? d2[(size_t)r * K2] : zero;
+        if (r + stride < nlam) c = cl[r + stride];
+        double2 v = zero;
 #pragma unroll
-                for (int q = 0; q < 6; ++q) v += g[q] * a[(6 * c + q) * K + j];
+        for (int k = 0; k < 2; ++k) {
+            const int ck = k ? now.y : now.x;
+            if (ck < 0) continue;
+            const double2 *g = reinterpret_cast<const double2 *>(gval) + 3 * (size_t)(2 * r + k);
+            const double2 *ac = a2 + 6 * ck * K2;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const double2 gq = g[q], a0 = ac[2 * q * K2], a1 = ac[(2 * q + 1) * K2];
+                v.x += gq.x * a0.x;
+                v.y += gq.x * a0.y;
+                v.x += gq.y * a1.x;
+                v.y += gq.y * a1.y;
             }
-            const double pv = x[(size_t)r * K + j] - v;
-            Px[(size_t)r * K + j] = pv;
-            m = fmax(m, fabs(pv));
-            if (dotv) prod += pv * dotv[(size_t)r * K + j];
+        }
+        const double2 pv = make_double2(xv.x - v.x, xv.y - v.y);
+        p2[(size_t)r * K2] = pv;
+        m.x = fmax(m.x, fabs(pv.x));
+        m.y = fmax(m.y, fabs(pv.y));
+        if (dotv) {
+            prod.x += pv.x * dv.x;
+            prod.y += pv.y * dv.y;
         }
     }
     if (partial) block_col_partial(prod, K, partial);
@@ -599,43 +728,70 @@ __global__ void k_colsum(const double *partial, int np, int K, double *out, cons
 }
 
 // rho_j = -gPz_j / wFw_j ; lam += rho w ; g += rho Fw  (skips finished columns)
-__global__ void k_update_lam_g_multi(int n, int K, const double *wFw, const double *gw,
-                                     const double *w, const double *Fw,
-                                     double *lam, double *g, PcpgState *st) {
+__global__ void __launch_bounds__(128) k_update_lam_g_multi(int n, int K, const double *wFw, const double *gw,
+                                                            const double *w, const double *Fw,
+                                                            double *lam, double *g, PcpgState *st) {
     pdl_next();
     pdl_wait();
-    const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (id >= (long long)n * K) return;
-    const int j = int(id % K);
-    if (st[j].done) return;
-    // mixed form: step length -g'w / w'Fw, equal to -g'Pz / w'Fw in exact
-    // arithmetic and still the exact line minimum along w after the residual
-    // g has been replaced by the FP64 one; FP64 form (no gw): -g'Pz / w'Fw
-    const double d = wFw[j];
-    double rho = -(gw ? gw[j] : st[j].gPz) / d;
-    if (!(d > 0.0) || !isfinite(rho)) rho = 0.0;
-    lam[id] += rho * w[id];
-    g[id] += rho * Fw[id];
+    const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;      // pair of columns
+    if (id >= (long long)n * (K / 2)) return;
+    const int j = 2 * int(id % (K / 2));
+    const bool run[2] = {!st[j].done, !st[j + 1].done};
+    if (!run[0] && !run[1]) return;
+    const double2 wv = reinterpret_cast<const double2 *>(w)[id], fv = reinterpret_cast<const double2 *>(Fw)[id];
+    double2 lv = reinterpret_cast<double2 *>(lam)[id], gv = reinterpret_cast<double2 *>(g)[id];
+    double rho[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        // mixed form: step length -g'w / w'Fw, equal to -g'Pz / w'Fw in exact
+        // arithmetic and still the exact line minimum along w after the residual
+        // g has been replaced by the FP64 one; FP64 form (no gw): -g'Pz / w'Fw
+        const double d = wFw[j + k];
+        rho[k] = -(gw ? gw[j + k] : st[j + k].gPz) / d;
+        if (!(d > 0.0) || !isfinite(rho[k])) rho[k] = 0.0;
+    }
+    if (run[0]) {
+        lv.x += rho[0] * wv.x;
+        gv.x += rho[0] * fv.x;
+    }
+    if (run[1]) {
+        lv.y += rho[1] * wv.y;
+        gv.y += rho[1] * fv.y;
+    }
+    reinterpret_cast<double2 *>(lam)[id] = lv;
+    reinterpret_cast<double2 *>(g)[id] = gv;
 }
 
 // w = Pz + gamma w (skips finished columns); with xmax also the column maxima of |w|, the scale of the next gather
-__global__ void __launch_bounds__(256) k_update_w_multi(int n, int K, const double *gPz_new, const double *Pz,
+__global__ void __launch_bounds__(128) k_update_w_multi(int n, int K, const double *gPz_new, const double *Pz,
                                                         double *w, const PcpgState *st, unsigned *xmax) {
     pdl_next();
     pdl_wait();
-    const long long stride = (long long)gridDim.x * blockDim.x;      // a multiple of K
-    const long long id0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const int j = int(id0 % K);
-    const bool run = !st[j].done;
-    const double gam = run ? gPz_new[j] / st[j].gPz : 0.0;
-    double m = 0.0;
-    for (long long id = id0; id < (long long)n * K; id += stride) {
-        double v = w[id];
-        if (run) {
-            v = Pz[id] + gam * v;
-            w[id] = v;
+    const int stride = gridDim.x * 128, end = n * (K / 2);          // the stride is a multiple of K / 2
+    const int id0 = blockIdx.x * 128 + threadIdx.x;
+    const int j = 2 * (id0 % (K / 2));
+    const bool run0 = !st[j].done, run1 = !st[j + 1].done;
+    const double gam0 = run0 ? gPz_new[j] / st[j].gPz : 0.0, gam1 = run1 ? gPz_new[j + 1] / st[j + 1].gPz : 0.0;
+    double2 *w2 = reinterpret_cast<double2 *>(w);
+    const double2 *z2 = reinterpret_cast<const double2 *>(Pz);
+    const double2 zero = make_double2(0.0, 0.0);
+    double2 m = zero;
+    for (long long id = id0; id < end; id += 2 * stride) {
+        double2 v[2], z[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const bool here = id + u * stride < end;
+            v[u] = here ? w2[id + u * stride] : zero;
+            z[u] = here ? z2[id + u * stride] : zero;
         }
-        m = fmax(m, fabs(v));
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            if (run0) v[u].x = z[u].x + gam0 * v[u].x;
+            if (run1) v[u].y = z[u].y + gam1 * v[u].y;
+            if ((run0 || run1) && id + u * stride < end) w2[id + u * stride] = v[u];
+            m.x = fmax(m.x, fabs(v[u].x));
+            m.y = fmax(m.y, fabs(v[u].y));
+        }
     }
     if (xmax) col_max(m, K, xmax);
 }
