@@ -70,12 +70,23 @@ __global__ void k_init_state(const double *, int, PcpgState *, double, int);
 __global__ void k_axpby(int, double, const double *, double, double *);
 
 // ---- glue kernels on full (permuted local) vectors ----------------------
+// CTA row blockIdx.y is a load case of several done in one launch, its vectors
+// at strides nfull (full vectors), nt (t), ng (coarse vectors) and na (alpha).
+// Bound by latency: a subdomain is one CTA, so the loads of eight terms are in
+// flight before they are added in order, and the load cases of a chunk, 2 to 5
+// launches each before, run side by side.  64 uneven subdomains, 32 load cases:
+// k_bc_rt 64 x 19 us, k_correct 32 x 18 -> 6 us, k_sub_bct 32 x 12 and k_add_R
+// 32 x 9 us; a solve 57.7 -> 55.1 ms.
+
 // t_d = [Bc_b z_b ; -R^T y]  (y full, z full)
 __global__ void k_bc_rt(const SubDev *__restrict__ subs, const int *__restrict__ bce_ptr,
                         const int *__restrict__ bce_pos, const double *__restrict__ bce_val,
                         const double *__restrict__ Rbuf, const double *__restrict__ z,
-                        const double *__restrict__ y, double *__restrict__ t) {
+                        const double *__restrict__ y, double *__restrict__ t, long long nfull, long long nt) {
     const SubDev &sd = subs[blockIdx.x];
+    z += blockIdx.y * nfull;
+    y += blockIdx.y * nfull;
+    t += blockIdx.y * nt;
     const int lane = threadIdx.x % 32, warp = threadIdx.x / 32, nw = blockDim.x / 32;
     const double *zb = z + sd.nfull_off + sd.nr;
     for (int q = threadIdx.x; q < sd.c; q += blockDim.x) {
@@ -87,6 +98,7 @@ __global__ void k_bc_rt(const SubDev *__restrict__ subs, const int *__restrict__
         const double *R = Rbuf + sd.R_off + (size_t)j * sd.N;
         const double *yy = y + sd.nfull_off;
         double s = 0.0;
+#pragma unroll 8
         for (int i = lane; i < sd.N; i += 32) s += R[i] * yy[i];
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) t[sd.t_off + sd.c + j] = -s;
@@ -109,9 +121,11 @@ __global__ void k_full_minus_b(const SubDev *__restrict__ subs, const double *__
 __global__ void k_sub_bct(const SubDev *__restrict__ subs, const ClusterDev *__restrict__ cl,
                           const int *__restrict__ bcr, const int *__restrict__ bce_ptr,
                           const int *__restrict__ bce_pos, const double *__restrict__ bce_val,
-                          const double *__restrict__ s, double *__restrict__ y) {
+                          const double *__restrict__ s, double *__restrict__ y, long long nfull, long long ng) {
     const SubDev &sd = subs[blockIdx.x];
     if (threadIdx.x != 0) return;      // few entries; sequential keeps the order fixed
+    s += blockIdx.y * ng;
+    y += blockIdx.y * nfull;
     const ClusterDev &c = cl[sd.cluster];
     for (int q = 0; q < sd.c; ++q) {
         const double lc = s[c.gc_off + bcr[sd.bcr_off + q]];
@@ -123,8 +137,12 @@ __global__ void k_sub_bct(const SubDev *__restrict__ subs, const ClusterDev *__r
 // u_full += R_d (alpha_c,d - H_d alpha_f,cluster)
 __global__ void k_add_R(const SubDev *__restrict__ subs, const ClusterDev *__restrict__ cl,
                         const double *__restrict__ Rbuf, const double *__restrict__ Hbuf,
-                        const double *__restrict__ s, const double *__restrict__ alpha_f, double *__restrict__ u) {
+                        const double *__restrict__ s, const double *__restrict__ alpha_f, double *__restrict__ u,
+                        long long nfull, long long ng, long long na) {
     __shared__ double coef[6];
+    s += blockIdx.y * ng;
+    alpha_f += blockIdx.y * na;
+    u += blockIdx.y * nfull;
     const SubDev &sd = subs[blockIdx.x];
     const ClusterDev &c = cl[sd.cluster];
     if (threadIdx.x < 6) {
@@ -177,7 +195,10 @@ __global__ void k_build_f(int nfull, int ndof, int nrhs, const double *__restric
 }
 
 // u[g] = uloc[win[g]]
-__global__ void k_gather_u(int ndof, const int *__restrict__ win, const double *__restrict__ uloc, double *__restrict__ u) {
+__global__ void k_gather_u(int ndof, const int *__restrict__ win, const double *__restrict__ uloc,
+                           double *__restrict__ u, long long nfull) {
+    uloc += blockIdx.y * nfull;
+    u += blockIdx.y * (long long)ndof;
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ndof) return;
     const int s = win[g];
@@ -487,6 +508,7 @@ int Engine::upload_layout(Problem &p, std::string &err) {
         d_tb_ = alloc<double>(nslots_, err, rc);
         if (!rc) CK(cudaMemcpyAsync(d_lblk_, lb.data(), lb.size() * sizeof(int2), cudaMemcpyHostToDevice, s_));
     }
+    nt_total_ = int(t_off);
     d_t_ = alloc<double>(t_off, err, rc);
     d_gc_ = alloc<double>(ngc_total_, err, rc);
     d_s_ = alloc<double>(ngc_total_, err, rc);
@@ -1083,20 +1105,23 @@ void Engine::ksolve(double *v) {
 
 // x = K_HT^+ f, d = Bf x, lambda0 = Gf (GfTGf)^{-1} Rf^T f  (Cluster.cpp:1385-1394, 967-1040);
 // with x_solved the triangular solves K_reg^{-1} f were done already (for
-// several load cases at once) and x_solved holds them
-void Engine::init_rhs(const double *f, const double *x_solved) {
+// several load cases at once) and x_solved holds them, t what k_bc_rt makes of them
+void Engine::init_rhs(const double *f, const double *x_solved, const double *t) {
     const double *x = x_solved;
     if (!x) {
         cudaMemcpyAsync(d_full_, f, nfull_ * sizeof(double), cudaMemcpyDeviceToDevice, s_);
         ksolve(d_full_);
         x = d_full_;
     }
-    k_bc_rt<<<nsub_, 256, 0, s_>>>(d_subs_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_R_, x, f, d_t_);
-    coarse_apply(d_t_, d_s_, nullptr);
+    if (!t) {
+        k_bc_rt<<<nsub_, 256, 0, s_>>>(d_subs_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_R_, x, f, d_t_, 0, 0);
+        t = d_t_;
+    }
+    coarse_apply(t, d_s_, nullptr);
     k_full_to_b<<<nsub_, 256, 0, s_>>>(d_subs_, x, d_yb_);
-    k_correct<<<nsub_, 256, 0, s_>>>(d_subs_, d_cl_, d_V_, d_bcr_, d_s_, d_yb_, nullptr);
+    k_correct<<<dim3(nsub_, cdiv(max_nbp_, 256)), 256, 0, s_>>>(d_subs_, d_cl_, d_V_, d_bcr_, d_s_, d_yb_, nullptr);
     k_rows<<<npart_, 256, 0, s_>>>(nlam_, d_rslot_, d_rsign_, d_yb_, nullptr, d_d_, nullptr, nullptr, nullptr);
-    k_e_vec<<<cdiv(6 * ncl_, 128), 128, 0, s_>>>(ncl_, d_csp_, d_cs_, d_subs_, d_H_, d_t_, d_gc_);
+    k_e_vec<<<cdiv(6 * ncl_, 128), 128, 0, s_>>>(ncl_, d_csp_, d_cs_, d_subs_, d_H_, t, d_gc_);
     k_small_gemv<<<1, 256, 0, s_>>>(6 * ncl_, d_invGtG_, d_gc_, d_a_);
     k_gf_mult<<<npart_, 256, 0, s_>>>(nlam_, d_gcl_, d_gval_, d_a_, d_lam_);
 }
@@ -1119,12 +1144,13 @@ void Engine::reconstruct(const double *f, double *u_dev) {
     k_full_minus_b<<<nsub_, 256, 0, s_>>>(d_subs_, d_xb_, d_full_);
     cudaMemcpyAsync(d_full2_, d_full_, nfull_ * sizeof(double), cudaMemcpyDeviceToDevice, s_);
     ksolve(d_full2_);
-    k_bc_rt<<<nsub_, 256, 0, s_>>>(d_subs_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_R_, d_full2_, d_full_, d_t_);
+    k_bc_rt<<<nsub_, 256, 0, s_>>>(d_subs_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_R_, d_full2_, d_full_, d_t_,
+                                   0, 0);
     coarse_apply(d_t_, d_s_, nullptr);
-    k_sub_bct<<<nsub_, 32, 0, s_>>>(d_subs_, d_cl_, d_bcr_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_s_, d_full_);
+    k_sub_bct<<<nsub_, 32, 0, s_>>>(d_subs_, d_cl_, d_bcr_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_s_, d_full_, 0, 0);
     ksolve(d_full_);
-    k_add_R<<<nsub_, 256, 0, s_>>>(d_subs_, d_cl_, d_R_, d_H_, d_s_, d_alpha_, d_full_);
-    if (u_dev) k_gather_u<<<cdiv(ndof_, 256), 256, 0, s_>>>(ndof_, d_win_, d_full_, u_dev);
+    k_add_R<<<nsub_, 256, 0, s_>>>(d_subs_, d_cl_, d_R_, d_H_, d_s_, d_alpha_, d_full_, 0, 0, 0);
+    if (u_dev) k_gather_u<<<cdiv(ndof_, 256), 256, 0, s_>>>(ndof_, d_win_, d_full_, u_dev, 0);
 }
 
 // one load case: Cluster::pcpg (Cluster.cpp:1363-1458) + printVTK (1648-1678)

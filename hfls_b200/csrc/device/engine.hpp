@@ -95,7 +95,7 @@ public:
 
 private:
     template <typename T> T *alloc(size_t n, std::string &err, int &rc);
-    void init_rhs(const double *f, const double *x_solved = nullptr);   // d = Bf K_HT^+ f, lambda0
+    void init_rhs(const double *f, const double *x_solved = nullptr, const double *t = nullptr);   // d = Bf K_HT^+ f, lambda0
     void ksolve(double *v);                               // v = K_reg^{-1} v, one column of nfull
     void trsm_multi(double *v, int nrhs);                 // v_j = K_reg^{-1} v_j, nrhs <= 32 columns of nfull
     void reconstruct(const double *f, double *u_dev);     // u from lambda, alpha

@@ -72,14 +72,14 @@ __global__ void k_gather_b(int, const int *, const int *, const double *, const 
                            const PcpgState *);
 __global__ void k_full_minus_b(const SubDev *, const double *, double *);
 __global__ void k_bc_rt(const SubDev *, const int *, const int *, const double *, const double *, const double *,
-                        const double *, double *);
+                        const double *, double *, long long, long long);
 __global__ void k_gc(int, const int *, const int *, const double *, double *, const PcpgState *);
 __global__ void k_coarse(const ClusterDev *, const double *, const double *, double *, const PcpgState *);
 __global__ void k_sub_bct(const SubDev *, const ClusterDev *, const int *, const int *, const int *, const double *,
-                          const double *, double *);
+                          const double *, double *, long long, long long);
 __global__ void k_add_R(const SubDev *, const ClusterDev *, const double *, const double *, const double *,
-                        const double *, double *);
-__global__ void k_gather_u(int, const int *, const double *, double *);
+                        const double *, double *, long long, long long, long long);
+__global__ void k_gather_u(int, const int *, const double *, double *, long long);
 
 
 static inline int cdivb(long long a, long long b) { return int((a + b - 1) / b); }
@@ -523,12 +523,14 @@ int Engine::batch_rhs(int r0, int kc, std::string &err) {
     CKB(cudaMemcpyAsync(b_fullB_, d_f_ + (size_t)r0 * nfull_, (size_t)kc * nfull_ * sizeof(double),
                         cudaMemcpyDeviceToDevice, s_));
     trsm_multi(b_fullB_, kc);
-    launches_ += 1;
+    k_bc_rt<<<dim3(nsub_, kc), 256, 0, s_>>>(d_subs_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_R_, b_fullB_,
+                                             d_f_ + (size_t)r0 * nfull_, b_t_, nfull_, nt_total_);
+    launches_ += 2;
     for (int j = 0; j < kc; ++j) {
-        init_rhs(d_f_ + (size_t)(r0 + j) * nfull_, b_fullB_ + (size_t)j * nfull_);
+        init_rhs(d_f_ + (size_t)(r0 + j) * nfull_, b_fullB_ + (size_t)j * nfull_, b_t_ + (size_t)j * nt_total_);
         k_col_set<<<npart_, 256, 0, s_>>>(nlam_, K, j, d_d_, b_d_);
         k_col_set<<<npart_, 256, 0, s_>>>(nlam_, K, j, d_lam_, b_lam_);
-        launches_ += 25;
+        launches_ += 24;
     }
     return HTF_OK;
 }
@@ -629,28 +631,25 @@ int Engine::batch_reconstruct(int r0, int kc, std::string &err) {
     }
     CKB(cudaMemcpyAsync(b_fullB_, b_fullA_, (size_t)kc * nfull_ * sizeof(double), cudaMemcpyDeviceToDevice, s_));
     trsm_multi(b_fullB_, kc);
+    k_bc_rt<<<dim3(nsub_, kc), 256, 0, s_>>>(d_subs_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_R_, b_fullB_, b_fullA_,
+                                             b_t_, nfull_, nt_total_);
     for (int j = 0; j < kc; ++j) {
-        double *fa = b_fullA_ + (size_t)j * nfull_;
-        k_bc_rt<<<nsub_, 256, 0, s_>>>(d_subs_, d_bce_ptr_, d_bce_pos_, d_bce_val_, d_R_, b_fullB_ + (size_t)j * nfull_,
-                                       fa, d_t_);
+        const double *t = b_t_ + (size_t)j * nt_total_;
         if (d_M_) {
-            k_gc<<<cdivb(ngc_total_, 256), 256, 0, s_>>>(ngc_total_, d_gptr_, d_gidx_, d_t_, d_gc_, nullptr);
+            k_gc<<<cdivb(ngc_total_, 256), 256, 0, s_>>>(ngc_total_, d_gptr_, d_gidx_, t, d_gc_, nullptr);
             k_coarse<<<dim3(ncl_, cdivb(maxg, 8)), 256, 0, s_>>>(d_cl_, d_M_, d_gc_, b_srec_ + (size_t)j * ngc_total_,
                                                                 nullptr);
         } else {
-            coarse_apply(d_t_, b_srec_ + (size_t)j * ngc_total_, nullptr);
+            coarse_apply(t, b_srec_ + (size_t)j * ngc_total_, nullptr);
         }
-        k_sub_bct<<<nsub_, 32, 0, s_>>>(d_subs_, d_cl_, d_bcr_, d_bce_ptr_, d_bce_pos_, d_bce_val_,
-                                        b_srec_ + (size_t)j * ngc_total_, fa);
     }
+    k_sub_bct<<<dim3(nsub_, kc), 32, 0, s_>>>(d_subs_, d_cl_, d_bcr_, d_bce_ptr_, d_bce_pos_, d_bce_val_, b_srec_,
+                                              b_fullA_, nfull_, ngc_total_);
     trsm_multi(b_fullA_, kc);
-    for (int j = 0; j < kc; ++j) {
-        double *fa = b_fullA_ + (size_t)j * nfull_;
-        k_add_R<<<nsub_, 256, 0, s_>>>(d_subs_, d_cl_, d_R_, d_H_, b_srec_ + (size_t)j * ngc_total_,
-                                       b_alpha_ + (size_t)j * 6 * ncl_, fa);
-        k_gather_u<<<cdivb(ndof_, 256), 256, 0, s_>>>(ndof_, d_win_, fa, d_u_ + (size_t)(r0 + j) * ndof_);
-    }
-    launches_ += 2 + 9 * kc;
+    k_add_R<<<dim3(nsub_, kc), 256, 0, s_>>>(d_subs_, d_cl_, d_R_, d_H_, b_srec_, b_alpha_, b_fullA_, nfull_,
+                                             ngc_total_, 6 * ncl_);
+    k_gather_u<<<dim3(cdivb(ndof_, 256), kc), 256, 0, s_>>>(ndof_, d_win_, b_fullA_, d_u_ + (size_t)r0 * ndof_, nfull_);
+    launches_ += 6 + 5 * kc;
     return HTF_OK;
 }
 

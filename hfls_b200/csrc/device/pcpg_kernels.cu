@@ -294,8 +294,9 @@ __global__ void k_correct(const SubDev *__restrict__ subs, const ClusterDev *__r
     __syncthreads();
     const double *V = Vbuf + sd.V_off;
     double *y = yb + sd.xb_off;
-    for (int i = threadIdx.x; i < sd.nb; i += blockDim.x) {
+    for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < sd.nb; i += gridDim.y * blockDim.x) {
         double a = y[i];
+#pragma unroll 8
         for (int q = 0; q < nc; ++q) a -= V[i + (size_t)q * sd.nbp] * sd_s[q];
         y[i] = a;
     }
