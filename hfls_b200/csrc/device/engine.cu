@@ -39,6 +39,7 @@ __global__ void k_gather_b(int, const int *, const int *, const double *, const 
                            const PcpgState *);
 __global__ void k_symv_units(const SymvUnit *, const SubDev *, const double *, const double *, const double *, double *,
                              double *, const PcpgState *);
+template <bool CORRECT>
 __global__ void k_reduce_correct(const SubDev *, const int *, const long long *, const double *, const ClusterDev *,
                                  const double *, const int *, const double *, double *, const PcpgState *);
 __global__ void k_lbt_x(const int2 *, const SubDev *, const double *, const double *, double *, const PcpgState *);
@@ -1035,7 +1036,7 @@ void Engine::op_F(const double *w, double *Fw, const double *dotv, double *parti
     launch_chain(k_symv_units, nunits_ + nvunits_, SYMV_WARPS * 32, symv_smem_, s_, d_units_, d_subs_, d_F_, d_V_, d_xb_,
                  d_ypart_, d_t_, st);
     coarse_apply(d_t_, d_s_, st);
-    launch_chain(k_reduce_correct, dim3(nsub_, cdiv(max_nbp_, 64)), 256, 0, s_, d_subs_, d_rbptr_, d_rboff_, d_ypart_,
+    launch_chain(k_reduce_correct<true>, dim3(nsub_, cdiv(max_nbp_, 64)), 256, 0, s_, d_subs_, d_rbptr_, d_rboff_, d_ypart_,
                  d_cl_, d_V_, d_bcr_, d_s_, d_yb_, st);
     launch_chain(k_rows, npart_, 256, 0, s_, nlam_, d_rslot_, d_rsign_, d_yb_, nullptr, Fw, dotv, partial, st);
 }
@@ -1048,7 +1049,7 @@ void Engine::op_M(const double *x, double *z, PcpgState *st) {
     } else {
         launch_chain(k_symv_units, nunits_, SYMV_WARPS * 32, symv_smem_, s_, d_units_, d_subs_, d_S_, d_V_, d_xb_,
                      d_ypart_, d_t_, st);
-        launch_chain(k_reduce_correct, dim3(nsub_, cdiv(max_nbp_, 64)), 256, 0, s_, d_subs_, d_rbptr_, d_rboff_,
+        launch_chain(k_reduce_correct<false>, dim3(nsub_, cdiv(max_nbp_, 64)), 256, 0, s_, d_subs_, d_rbptr_, d_rboff_,
                      d_ypart_, d_cl_, d_V_, d_bcr_, nullptr, d_yb_, st);
     }
     launch_chain(k_rows, npart_, 256, 0, s_, nlam_, d_rslot_, d_rsign_, d_yb_, d_weight_, z, nullptr, nullptr, st);

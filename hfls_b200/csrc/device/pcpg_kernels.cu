@@ -199,12 +199,19 @@ __global__ void __launch_bounds__(SYMV_WARPS * 32) k_symv_units(const SymvUnit *
     }
 }
 
-// y_b = sum of the unit partials [- V_d s_d when s != null].  CTA
+// y_b = sum of the unit partials [- V_d s_d with CORRECT].  CTA
 // (subdomain, 64 b rows) of four groups of 64 threads: thread (group k, row)
 // adds the partials k, k + 4, .. of the row's block (rboff: where each
 // unit's 32 partial rows of the block start in ypart, in unit order) and the
 // columns k, k + 4, .. of V; the groups are added in order.  V's first
 // RC_PRE columns of a thread and the lists are loaded before the wait.
+// Bound by latency (a large subdomain has some 50 partials a row).  Without the
+// correction a warp, whose 32 rows share their block's list, reads up to 32
+// offsets at once, before the wait, and keeps eight partials in flight: S_i of
+// the 512-subdomain cube 34 -> 28 us, of 4 096 uneven subdomains 346 -> 292.
+// With V's columns in flight too that costs the registers of a CTA per SM (55
+// -> 58 and 540 -> 598 us), so F_i reads each offset before its partial.
+template <bool CORRECT>
 __global__ void __launch_bounds__(256) k_reduce_correct(const SubDev *__restrict__ subs,
                                                         const int *__restrict__ rbptr,
                                                         const long long *__restrict__ rboff, const double *ypart,
@@ -212,43 +219,71 @@ __global__ void __launch_bounds__(256) k_reduce_correct(const SubDev *__restrict
                                                         const double *__restrict__ Vbuf,
                                                         const int *__restrict__ bcrows, const double *s, double *yb,
                                                         const PcpgState *st) {
-    constexpr int RC_PRE = 8;
-    __shared__ double sd_s[256];
+    constexpr int RC_PRE = 8, U = 8;
+    __shared__ double sd_s[CORRECT ? 256 : 1];
     __shared__ double part[3][64];
     pdl_next();
     const SubDev &sd = subs[blockIdx.x];
-    const int grp = threadIdx.x >> 6, lr = threadIdx.x & 63, i = blockIdx.y * 64 + lr;
+    const int grp = threadIdx.x >> 6, lr = threadIdx.x & 63, i = blockIdx.y * 64 + lr, lane = threadIdx.x & 31;
     if (blockIdx.y * 64 >= sd.nbp) return;
-    const bool in = i < sd.nbp;             // nbp is a multiple of 32, not of 64
-    const int nc = s ? sd.c + 6 : 0;
+    const bool in = i < sd.nbp;             // nbp is a multiple of 32, not of 64: the same for a warp
+    const int nc = CORRECT ? sd.c + 6 : 0;
     const double *V = Vbuf + sd.V_off + i;
     const size_t nbp = sd.nbp;
     const int q0 = in ? rbptr[sd.rb_off + i / TILE] : 0, q1 = in ? rbptr[sd.rb_off + i / TILE + 1] : 0;
+    long long off = !CORRECT && q0 + grp + 4 * lane < q1 ? rboff[q0 + grp + 4 * lane] : 0;
     double vr[RC_PRE];
-#pragma unroll
-    for (int u = 0; u < RC_PRE; ++u) vr[u] = (in && grp + 4 * u < nc) ? V[(grp + 4 * u) * nbp] : 0.0;
     int pos = -1;
-    if (int(threadIdx.x) < nc)
-        pos = cl[sd.cluster].gc_off +
-              (int(threadIdx.x) < sd.c ? bcrows[sd.bcr_off + threadIdx.x] : sd.alpha_pos + (int(threadIdx.x) - sd.c));
+    if (CORRECT) {
+#pragma unroll
+        for (int u = 0; u < RC_PRE; ++u) vr[u] = (in && grp + 4 * u < nc) ? V[(grp + 4 * u) * nbp] : 0.0;
+        if (int(threadIdx.x) < nc)
+            pos = cl[sd.cluster].gc_off +
+                  (int(threadIdx.x) < sd.c ? bcrows[sd.bcr_off + threadIdx.x] : sd.alpha_pos + (int(threadIdx.x) - sd.c));
+    }
     pdl_wait();
     if (st && st->done) return;
-    if (pos >= 0) sd_s[threadIdx.x] = s[pos];           // c + 6 <= 256
+    if (CORRECT && pos >= 0) sd_s[threadIdx.x] = s[pos];           // c + 6 <= 256
     double a = 0.0;
+    if (CORRECT) {
 #pragma unroll 4
-    for (int q = q0 + grp; q < q1; q += 4) a += ypart[rboff[q] + (lr & 31)];
-    __syncthreads();
-    double b = 0.0;
+        for (int q = q0 + grp; q < q1; q += 4) a += ypart[rboff[q] + lane];
+    } else {
+        for (int q = q0 + grp; q < q1; q += 4 * 32) {              // 32 partials of this group at a time
+            if (q != q0 + grp) off = q + 4 * lane < q1 ? rboff[q + 4 * lane] : 0;
+            const int n = min(32, (q1 - q + 3) / 4);
+            for (int k = 0; k < n; k += U) {
+                double v[U];
 #pragma unroll
-    for (int u = 0; u < RC_PRE; ++u) b += (grp + 4 * u < nc) ? vr[u] * sd_s[grp + 4 * u] : 0.0;
-    if (in)
+                for (int u = 0; u < U; ++u) {
+                    const long long o = __shfl_sync(FULL, off, (k + u) & 31);
+                    v[u] = k + u < n ? ypart[o + lane] : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) a += v[u];
+            }
+        }
+    }
+    if (CORRECT) {
+        __syncthreads();
+        double b = 0.0;
+#pragma unroll
+        for (int u = 0; u < RC_PRE; ++u) b += (grp + 4 * u < nc) ? vr[u] * sd_s[grp + 4 * u] : 0.0;
+        if (in)
 #pragma unroll 4
-        for (int q = grp + 4 * RC_PRE; q < nc; q += 4) b += V[q * nbp] * sd_s[q];
-    a -= b;
+            for (int q = grp + 4 * RC_PRE; q < nc; q += 4) b += V[q * nbp] * sd_s[q];
+        a -= b;
+    }
     if (grp) part[grp - 1][lr] = a;
     __syncthreads();
     if (grp == 0 && in) yb[sd.xb_off + i] = ((a + part[0][lr]) + part[1][lr]) + part[2][lr];
 }
+template __global__ void k_reduce_correct<false>(const SubDev *, const int *, const long long *, const double *,
+                                                 const ClusterDev *, const double *, const int *, const double *,
+                                                 double *, const PcpgState *);
+template __global__ void k_reduce_correct<true>(const SubDev *, const int *, const long long *, const double *,
+                                                const ClusterDev *, const double *, const int *, const double *,
+                                                double *, const PcpgState *);
 
 // gc[q] = sum of the t entries listed for q (fixed order)
 __global__ void k_gc(int ngc_total, const int *__restrict__ gptr, const int *__restrict__ gidx,
