@@ -367,33 +367,34 @@ __device__ __forceinline__ double2 row_value(int r, int K2, const int *__restric
 // chunk), a 128 x K by (c + 6) x K product: s_d staged in shared memory
 // ((c + 6) K <= 2048 doubles, checked at set-up), V in chunks of 16 columns
 // (coalesced column reads); thread (row group, case group) keeps 128 K / 256
-// outputs in registers (rows rg + RG i, cases jg + JG c: conflict-free
-// shared-memory reads), summed over the columns in order.
+// outputs in registers (rows rg + RG i, case pairs jg + JG c: conflict-free
+// 16-byte shared-memory reads), summed over the columns in order.  y is read
+// only for the subtraction, so that three CTAs fit an SM: the mixed iteration
+// of 32 load cases 1744 -> 1688 us (512-subdomain cube), 271 -> 268 (64 uneven
+// subdomains, this kernel 22 -> 20 us for 5 us of FP64 operations).
 template <int K>
-__global__ void __launch_bounds__(256, 2) k_correct_multi(const SubDev *__restrict__ subs,
+__global__ void __launch_bounds__(256, 3) k_correct_multi(const SubDev *__restrict__ subs,
                                                        const ClusterDev *__restrict__ cl,
                                                        const double *__restrict__ V, const int *__restrict__ bcr,
                                                        const double *s, double *yb) {
     constexpr int QC = 16;                            // V columns per shared-memory chunk
-    constexpr int JG = K / 4;                         // case groups (4 cases per thread)
+    constexpr int JG = K / 4;                         // case groups (two pairs of cases per thread)
     constexpr int RG = 256 / JG;                      // row groups
     constexpr int RPT = 128 / RG;                     // rows per thread
-    __shared__ double ss[2048];
+    __shared__ double2 ss[1024];
     __shared__ double vs[QC][128];
+    __shared__ int ps[2048 / K];
     const SubDev &sd = subs[blockIdx.x];
     const int r0 = blockIdx.y * 128;
     if (r0 >= sd.nb) return;
     const int nc = sd.c + 6;
-    const int gc_off = cl[sd.cluster].gc_off;
     pdl_next();
     const int rend = min(128, sd.nb - r0);
     const int jg = threadIdx.x % JG, rg = threadIdx.x / JG;
     const double *Vd = V + sd.V_off + r0;
-    double acc[RPT][4];
+    double2 acc[RPT][2];
 #pragma unroll
-    for (int i = 0; i < RPT; ++i)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[i][c] = 0.0;
+    for (int i = 0; i < RPT; ++i) acc[i][0] = acc[i][1] = make_double2(0.0, 0.0);
     // the next V chunk is loaded into registers while the current one multiplies
     constexpr int VPT = QC * 128 / 256;               // V values per thread and chunk
     double vr[VPT];
@@ -405,21 +406,15 @@ __global__ void __launch_bounds__(256, 2) k_correct_multi(const SubDev *__restri
         }
     };
     fetch(0);
+    if (int(threadIdx.x) < nc)                        // (c + 6) K <= 2048
+        ps[threadIdx.x] = cl[sd.cluster].gc_off + (int(threadIdx.x) < sd.c ? bcr[sd.bcr_off + threadIdx.x]
+                                                                           : sd.alpha_pos + int(threadIdx.x) - sd.c);
+    __syncthreads();
     pdl_wait();
-    for (int o = threadIdx.x; o < nc * K; o += blockDim.x) {
-        const int q = o / K, j = o % K;
-        const int pos = q < sd.c ? bcr[sd.bcr_off + q] : sd.alpha_pos + (q - sd.c);
-        ss[o] = s[((size_t)gc_off + pos) * K + j];
-    }
-    // this thread's y entries, read now so their latency overlaps the products
-    double yv[RPT][4];
-#pragma unroll
-    for (int i = 0; i < RPT; ++i) {
-        const int row = rg + RG * i;
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            yv[i][c] = row < rend ? yb[((size_t)sd.xb_off + r0 + row) * K + jg + JG * c] : 0.0;
-    }
+    const double2 *s2 = reinterpret_cast<const double2 *>(s);
+#pragma unroll 4
+    for (int o = threadIdx.x; o < nc * (K / 2); o += 256) ss[o] = s2[(size_t)ps[o / (K / 2)] * (K / 2) + o % (K / 2)];
+    double2 *y2 = reinterpret_cast<double2 *>(yb) + ((size_t)sd.xb_off + r0) * (K / 2) + jg;
     for (int q0 = 0; q0 < nc; q0 += QC) {
         const int qn = min(QC, nc - q0);
         __syncthreads();                              // s_d staged, the previous chunk consumed
@@ -430,28 +425,28 @@ __global__ void __launch_bounds__(256, 2) k_correct_multi(const SubDev *__restri
         }
         __syncthreads();
         if (q0 + QC < nc) fetch(q0 + QC);
+#pragma unroll 2
         for (int q = 0; q < qn; ++q) {
-            const double *sq = ss + (q0 + q) * K + jg;
-            double sv[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) sv[c] = sq[JG * c];
+            const double2 *sq = ss + (q0 + q) * (K / 2) + jg;
+            const double2 s0 = sq[0], s1 = sq[JG];
 #pragma unroll
             for (int i = 0; i < RPT; ++i) {
                 const double v = vs[q][rg + RG * i];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[i][c] += v * sv[c];
+                acc[i][0].x += v * s0.x;
+                acc[i][0].y += v * s0.y;
+                acc[i][1].x += v * s1.x;
+                acc[i][1].y += v * s1.y;
             }
         }
     }
 #pragma unroll
-    for (int i = 0; i < RPT; ++i) {
-        const int row = rg + RG * i;
-        if (row < rend) {
-            double *y = yb + ((size_t)sd.xb_off + r0 + row) * K + jg;
+    for (int i = 0; i < RPT; ++i)
+        if (rg + RG * i < rend)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) y[JG * c] = yv[i][c] - acc[i][c];
-        }
-    }
+            for (int c = 0; c < 2; ++c) {
+                double2 &y = y2[(rg + RG * i) * (K / 2) + JG * c];
+                y = make_double2(y.x - acc[i][c].x, y.y - acc[i][c].y);
+            }
 }
 
 template __global__ void k_correct_multi<16>(const SubDev *, const ClusterDev *, const double *, const int *,
