@@ -220,11 +220,13 @@ int Engine::alloc_units(std::string &err) {
     std::vector<int> cands(1, SYMV_DEFAULT_TILES);
     if (opt_.autotune) cands.assign(std::begin(CANDIDATES), std::end(CANDIDATES));
     // A schedule's unit sizes are upper bounds: a problem of few tiles is cut into at least SYMV_MIN_UNITS units
-    // (four CTAs per SM), down to 4 tiles each, one per warp.  Measured per iteration: 528 tiles (8 subdomains) 59
-    // us with units of 48 tiles, 41 us with 4; 7 900 tiles (32 subdomains) 88 us with 48, 78 with 12, 82 with 4;
+    // (four CTAs per SM), down to one tile each.  Measured per iteration: 528 tiles (8 subdomains) 59 us with units
+    // of 48 tiles, 41 with 5 to 8, 39 with 1 to 4; 7 900 tiles (32 subdomains) 88 us with 48, 78 with 12, 82 with 4;
     // from 29 000 tiles on the bound is above 48 and the schedule's own sizes hold (43 000 tiles: 252 us with 32 or
-    // 48, 262 with 16).
-    unit_cap_ = int(std::max<long long>(4, std::min<long long>(ntiles_ / SYMV_MIN_UNITS, 1 << 20)));
+    // 48, 262 with 16).  One tile at least, not four: a solve of the 8 subdomains takes 2.22 ms instead of 2.11, but
+    // with four the E-contrast problem of __graft_entry__.smoke stops at 151 iterations, one beyond its bar of 148 +-
+    // 2, with one at 149 (with loads moved by 1e-17 the counts are 147 to 153 either way, mean 149.6 and 150.1).
+    unit_cap_ = int(std::max<long long>(1, std::min<long long>(ntiles_ / SYMV_MIN_UNITS, 1 << 20)));
     // every unit's row window is at most 32 (ut + 1) rows of 5 doubles: the
     // largest candidate (96 tiles) needs 124 KB, within the 227 KB opt-in limit
     long long bu[SYMV_BUCKETS][8] = {}, by[SYMV_BUCKETS][8] = {};
