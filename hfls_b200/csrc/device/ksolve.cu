@@ -15,8 +15,8 @@
 // the inverse of the diagonal block instead is shorter but not backward
 // stable: K_reg is singular up to its six fix DOFs, and the residual it
 // leaves moved an E-contrast-100 solve by 4 iterations.)  All results stay in
-// shared memory, so no buffer is reused and no warp waits for another to
-// have read.
+// shared memory, x_b in the place of y_b: between the passes the cluster meets
+// once, so that within a pass no warp waits for another to have read.
 //
 // Bound by the factor's bytes, read twice, or for few or small subdomains by
 // the chain of N / 32 blocks (2 us per block and direction).  Against one
@@ -60,6 +60,22 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// first phase of a barrier whose arrivals come from any CTA of the cluster; false on time-out
+__device__ __forceinline__ bool bar_wait_cluster(uint64_t *bar) {
+    uint32_t done = 0;
+    for (unsigned it = 0; it < TC_WAIT_LIMIT; ++it) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0, %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(smem_u32(bar)), "r"(TC_WAIT_HINT_NS)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
 }
 
 // lane l's value to slot[l] of every CTA of the cluster, counted on their bar
@@ -146,7 +162,7 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) k_ksolve(const SubDev *__res
             for (int j = 0; j < 32; ++j) l[j] = j < wk ? col[j * ld] : 0.0;
         };
         auto apply = [&](const double (&l)[32], int k) {
-            ok = ok && mbar_wait(&fwd[k], 0);
+            ok = ok && bar_wait_cluster(&fwd[k]);
             const double2 *yk = reinterpret_cast<const double2 *>(xs + 32 * k);
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
@@ -175,16 +191,19 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) k_ksolve(const SubDev *__res
         }
         if (ok) send_block(xs + 32 * b, &fwd[b], lane, y, C);
     }
-    // backward: x_b = L_bb^{-T} (y_b - sum_{k > b} L_kb^T x_k); a result x_k overwrites y_k's slot once
-    // every y is known, when no forward step reads it any more
+    // x_b goes to the slots of y_b, and asynchronous stores have no order among themselves: no x is sent before
+    // every y has landed in every CTA of the cluster (in a CTA that owns no later block nothing else waits for
+    // y_b), by when no forward step reads one any more either
+    for (int b = threadIdx.x; b < nblk && ok; b += blockDim.x) ok = bar_wait_cluster(&fwd[b]);
+    ok = __all_sync(0xffffffffu, ok);
+    cluster_sync_all();
+    // backward: x_b = L_bb^{-T} (y_b - sum_{k > b} L_kb^T x_k)
     const int mine = first < nblk ? (nblk - 1 - first) / step : -1;
-    if (ok && mine >= 0) ok = mbar_wait(&fwd[nblk - 1], 0);
     for (int i = mine; i >= 0 && ok; --i) {
         const int b = first + i * step, c0 = start(b), wb = width(b);
         const double rd = load_diag(b);
         const double *col0 = K + kcol(sd, c0);
         const long long ld = kld(sd, c0);
-        if (!mbar_wait(&fwd[b], 0)) { ok = false; break; }
         double z = xs[32 * b + lane], p[32], lA[32], lB[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) p[j] = 0.0;
@@ -200,7 +219,7 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) k_ksolve(const SubDev *__res
 #pragma unroll
                 for (int j = 0; j < 32; ++j) p[j] = 0.0;
             }
-            ok = ok && mbar_wait(&bwd[k], 0);
+            ok = ok && bar_wait_cluster(&bwd[k]);
             const double xk = xs[32 * k + lane];                       // zero past the block's rows
 #pragma unroll
             for (int j = 0; j < 32; ++j) p[j] += l[j] * xk;
@@ -227,7 +246,7 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) k_ksolve(const SubDev *__res
     }
     // no CTA leaves while results are on their way to it
     if (warp == 0 && ok)
-        for (int b = 0; b < nblk && ok; ++b) ok = mbar_wait(&bwd[b], 0);
+        for (int b = 0; b < nblk && ok; ++b) ok = bar_wait_cluster(&bwd[b]);
     if (!ok && lane == 0) atomicExch(err, HTF_ETIMEDOUT);
     cluster_sync_all();
 }
@@ -333,21 +352,6 @@ __device__ __forceinline__ bool bar_poll(uint64_t *bar) {
         : "r"(smem_u32(bar))
         : "memory");
     return done;
-}
-
-__device__ __forceinline__ bool bar_wait_cluster(uint64_t *bar) {
-    uint32_t done = 0;
-    for (unsigned it = 0; it < TC_WAIT_LIMIT; ++it) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0, %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(smem_u32(bar)), "r"(TC_WAIT_HINT_NS)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
 }
 
 // the CTA's global writes before the last __syncthreads are visible to whoever sees bar complete
