@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <utility>
 #include <vector>
 
 namespace htf {
@@ -46,6 +47,12 @@ public:
                 bufs_.erase(bufs_.begin() + i);
                 return;
             }
+    }
+
+    void swap(DevArena &o) {
+        bufs_.swap(o.bufs_);
+        std::swap(next_, o.next_);
+        std::swap(left_, o.left_);
     }
 
     size_t bytes() const {

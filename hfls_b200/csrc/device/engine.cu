@@ -229,6 +229,8 @@ Engine::~Engine() {
     if (s_ && s_ != own_s_) cudaStreamSynchronize(s_);
     if (graph_) cudaGraphExecDestroy(graph_);
     if (bgraph_) cudaGraphExecDestroy(bgraph_);
+    for (cudaGraphExec_t g : bgraph64_)
+        if (g) cudaGraphExecDestroy(g);
     if (run_e0_) cudaEventDestroy(run_e0_);
     if (run_e1_) cudaEventDestroy(run_e1_);
     mem_.clear();
@@ -1252,9 +1254,11 @@ int Engine::solve(Problem &p, int nrhs, const double *f_nodal, double *u, htf_st
     k_build_f<<<cdiv(nfull_, 256), 256, 0, s_>>>(nfull_, ndof_, nrhs, d_fbody_, d_own_, f_nodal ? d_fn_ : nullptr, d_f_);
     CK(cudaGetLastError());
     double total_ms = 0.0;
+    const int together = width64(nrhs);
     for (int r = 0; r < nrhs;) {
-        // the remaining load cases together, or one (the last few, or a problem the batched form does not take)
-        const int kc = ready_batch64(nrhs - r) ? std::min(nrhs - r, bK_) : 1;
+        // up to `together` of the remaining load cases, or one (the last few, or a problem the batched form does not
+        // take)
+        const int kc = nrhs - r >= B64_MIN && together > 0 ? std::min(nrhs - r, together) : 1;
         int it = 0;
         double n0 = 0, rel = 0, ms = 0;
         if (kc > 1) rc = solve_chunk64(r, kc, ms, err);

@@ -45,7 +45,27 @@ struct BatchRun {
 constexpr int MIXED_STALL_LIMIT = 10;
 constexpr int MIXED_STALL_ITERATIONS = 500;
 
-class Engine {
+constexpr int B64_MIN = 3;                     // load cases of the FP64 form from which on they are solved together
+
+// vectors and scratch of a batch of load cases, K columns interleaved (mixed and FP64 form); they hold any K up to
+// the one they were allocated for
+struct BatchVectors {
+    int bnpart_ = 0, vt_nch_ = 1, vt_qn_ = 64;
+    double *b_lam_ = nullptr, *b_g_ = nullptr, *b_w_ = nullptr, *b_Fw_ = nullptr, *b_Pg_ = nullptr, *b_z_ = nullptr,
+           *b_Pz_ = nullptr, *b_d_ = nullptr, *b_xb_ = nullptr, *b_yb_ = nullptr, *b_t_ = nullptr, *b_gc_ = nullptr,
+           *b_s_ = nullptr, *b_part_ = nullptr, *b_part2_ = nullptr, *b_gpart_ = nullptr, *b_wFw_ = nullptr, *b_gPz_ = nullptr, *b_gw_ = nullptr, *b_gt_ = nullptr, *b_acoef_ = nullptr,
+           *b_alpha_ = nullptr, *b_tmp_ = nullptr;
+    double *b_fullA_ = nullptr, *b_fullB_ = nullptr;   // full vectors of the batch (nfull x K)
+    double *b_srec_ = nullptr;                         // coarse solutions of the reconstruction (ngc x K)
+    double *b_alpha2_ = nullptr;                       // alpha of the FP64 residuals, K-interleaved
+    int *d_mask_ = nullptr;                            // selected / reset columns of an FP64 residual batch
+    void *d_rowblk_ = nullptr;                         // (subdomain, 32-row block) list of the FP64 multi-RHS SYMV
+    int nrowblk_ = 0;
+    PcpgState *b_st_ = nullptr;
+    double *b_hist_ = nullptr;                         // FP64 form: relative residuals, [iteration][column]
+};
+
+class Engine : private BatchVectors {
 public:
     explicit Engine(const Options &o) : opt_(o) {}
     ~Engine();
@@ -63,7 +83,6 @@ public:
     int plan_slabs(int K, std::string &err);       // tensor-core blocks and slab buffers
     int solve_batch(Problem &p, int nrhs, const double *f_nodal, double *u, htf_stats *stats, std::string &err);
     int apply_batch(int op, const double *x, double *y, int nrhs, std::string &err);
-    bool batch_ready() const { return bK_ > 0; }
     // steps of a batched solve, for callers that interleave several problems
     int batch_loads(int nrhs, const double *f_nodal, std::string &err);
     int batch_begin(int r0, int kc, std::string &err);
@@ -122,7 +141,9 @@ private:
     int batch_reconstruct(int r0, int kc, std::string &err);
     void symv_multi(const double *tiles, const double *scoarse);
     // FP64 form, several load cases at once (engine_batch.cu)
-    bool ready_batch64(int nrhs);
+    int width64(int nrhs);                                // most columns for nrhs load cases, 0: one at a time
+    bool grow_batch64(int K);
+    void set_width64(int K);
     void op_F_batch64(const double *w, double *Fw, const double *dotv, double *partial);
     void op_M_batch64(const double *x, double *z);
     void iteration_batch64();
@@ -232,7 +253,7 @@ private:
     int unit_cap_ = 1 << 20;                     // and their bound for problems of few tiles
     bool tuned_ = false;
     // batched mixed-precision form
-    int bK_ = 0, nblocks_ = 0, bnpart_ = 0, bnpartP_ = 0;
+    int bK_ = 0, nblocks_ = 0;
     float *d_AF_ = nullptr, *d_AS_ = nullptr, *d_Xs_ = nullptr;
     unsigned *d_amaxF_ = nullptr, *d_amaxS_ = nullptr;   // scales of the FP16-pair slabs (largest |A| per subdomain)
     unsigned *d_xmax_ = nullptr;                         // scale of the X slabs (largest |w_j| per column)
@@ -243,22 +264,12 @@ private:
     BatchRun run_;
     cudaEvent_t run_e0_ = nullptr, run_e1_ = nullptr;
     int *d_slot_sub_ = nullptr, *d_tcerr_ = nullptr;
-    double *b_lam_ = nullptr, *b_g_ = nullptr, *b_w_ = nullptr, *b_Fw_ = nullptr, *b_Pg_ = nullptr, *b_z_ = nullptr,
-           *b_Pz_ = nullptr, *b_d_ = nullptr, *b_xb_ = nullptr, *b_yb_ = nullptr, *b_t_ = nullptr, *b_gc_ = nullptr,
-           *b_s_ = nullptr, *b_part_ = nullptr, *b_part2_ = nullptr, *b_gpart_ = nullptr, *b_wFw_ = nullptr, *b_gPz_ = nullptr, *b_gw_ = nullptr, *b_gt_ = nullptr, *b_acoef_ = nullptr,
-           *b_alpha_ = nullptr, *b_tmp_ = nullptr;
-    double *b_fullA_ = nullptr, *b_fullB_ = nullptr;   // full vectors of the batch (nfull x K)
-    double *b_srec_ = nullptr;                         // coarse solutions of the reconstruction (ngc x K)
-    double *b_alpha2_ = nullptr;                       // alpha of the FP64 residuals, K-interleaved
-    int *d_mask_ = nullptr;                            // selected / reset columns of an FP64 residual batch
-    void *d_rowblk_ = nullptr;                         // (subdomain, 32-row block) list of the FP64 multi-RHS SYMV
-    int nrowblk_ = 0;
-    PcpgState *b_st_ = nullptr;
-    bool b64_off_ = false;                     // FP64 form: the batched form was found not to apply
-    double *b_hist_ = nullptr;                 // FP64 form: relative residuals, [iteration][column]
     cudaGraphExec_t bgraph_ = nullptr;
     int bkernels_per_iter_ = 0;
-    int tc_smem_ = 0, vt_nch_ = 1, vt_qn_ = 64;
+    int b64_cap_ = 0;                          // FP64 form: columns that the batch vectors hold (bK_: of the chunk)
+    cudaGraphExec_t bgraph64_[2] = {nullptr, nullptr};   // its iteration with 16 and with 32 columns
+    int bkernels64_[2] = {0, 0};
+    int tc_smem_ = 0;
     long long aoff_ = 0;                       // 4-byte words per slab array
     // vectors
     int *d_kserr_ = nullptr;                   // time-out flag of the K_reg solves

@@ -1,5 +1,5 @@
 // Batched PCPG (K load cases at once): the mixed-precision form, and from
-// ready_batch64 on the FP64 form of several load cases.
+// width64 on the FP64 form of several load cases.
 //
 // Mixed form:
 // F_i and S_i are applied on the tensor cores as scaled FP16 hi + lo pairs
@@ -773,21 +773,29 @@ int Engine::solve_batch(Problem &p, int nrhs, const double *f_nodal, double *u, 
 // when the rule was set: 8 subdomains of 648 rows 5.3 and 4.5 ms, 32 uneven
 // ones 26.6 and 21.8, 64 uneven ones 101 and 85, 512-subdomain cube 569 and
 // 523 ms).
+//
+// A chunk's width is 16 columns, 32 for more than 16 load cases: it follows
+// from the chunk alone, so that a load case's sums, whose grouping depends on
+// the width, do not depend on the calls before (and a chunk of few does not
+// pay for the columns of an earlier, larger one).
 // ---------------------------------------------------------------------------
-constexpr int B64_MIN = 3;
 
-// Batch vectors for nrhs load cases; false when the batched form does not
-// apply: too many Bc rows per subdomain, no explicit S_i tiles, or vectors
-// that would take more than a quarter of the free device memory.
-bool Engine::ready_batch64(int nrhs) {
-    if (b64_off_ || mixed_ || implicit_ || !d_S_ || nrhs < B64_MIN) return false;
-    const int K = nrhs <= 16 ? 16 : 32;
-    if (bK_ >= K) return true;
-    for (auto &h : hs_)
-        if ((h.c + 6) * K > 2048) {
-            b64_off_ = bK_ == 0;
-            return bK_ > 0;
-        }
+// Columns that nrhs load cases of one call may use, with the batch vectors
+// allocated; 0 when they are solved one at a time: fewer than B64_MIN, no
+// explicit S_i tiles, too many Bc rows per subdomain, or vectors that would
+// take more than a quarter of the device memory that is free or theirs.  When
+// 32 columns do not fit 16 may.
+int Engine::width64(int nrhs) {
+    if (mixed_ || implicit_ || !d_S_ || nrhs < B64_MIN) return 0;
+    int maxcol = 0;
+    for (auto &h : hs_) maxcol = std::max(maxcol, h.c + 6);
+    for (int K = nrhs <= 16 ? 16 : 32; K >= 16; K /= 2)
+        if (maxcol * K <= 2048 && (b64_cap_ >= K || grow_batch64(K))) return K;
+    return 0;
+}
+
+// Batch vectors for K columns instead of the present ones, which stay when there is no room
+bool Engine::grow_batch64(int K) {
     long long tn = 0, nch = 1;
     for (auto &h : hs_) {
         tn = std::max<long long>(tn, h.t_off + h.c + 6);
@@ -797,29 +805,36 @@ bool Engine::ready_batch64(int nrhs) {
                         (9.0 * nlam_ + 2.0 * nslots_ + 2.0 * nfull_ + double(tn) * nch + 3.0 * ngc_total_ +
                          6.0 * nchunks_ + 2.0 * 1184.0 + double(std::max(opt_.max_iter, 0)) + 1.0);
     size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || need > 0.25 * double(fr)) {
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || need > 0.25 * double(fr + bmem_.bytes())) {
         cudaGetLastError();
-        b64_off_ = bK_ == 0;
-        return bK_ > 0;
+        return false;
     }
     if (cudaStreamSynchronize(s_) != cudaSuccess) return false;
-    if (bgraph_) cudaGraphExecDestroy(bgraph_);
-    bgraph_ = nullptr;
-    bK_ = 0;
-    bmem_.clear();
+    const BatchVectors old = *this;
+    DevArena fresh;
     std::string why;
-    into_ = &bmem_;
+    into_ = &fresh;
     int rc = alloc_batch(K, why);
     b_hist_ = alloc<double>((size_t(std::max(opt_.max_iter, 0)) + 1) * K, why, rc);
     into_ = &mem_;
-    if (rc) {                                       // one load case at a time needs none of it
+    if (rc) {
         cudaGetLastError();
-        bmem_.clear();
-        b64_off_ = true;
+        static_cast<BatchVectors &>(*this) = old;
         return false;
     }
-    bK_ = K;
+    bmem_.swap(fresh);                               // the old vectors go with `fresh`, their graphs here
+    for (cudaGraphExec_t &g : bgraph64_) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+    b64_cap_ = K;
     return true;
+}
+
+// columns of the next chunk (at most b64_cap_)
+void Engine::set_width64(int K) {
+    bK_ = K;
+    bnpart_ = std::min(cdivb(nlam_, 256 / K), 1184);
 }
 
 // F and S products, projections and recurrences of one iteration of every running column
@@ -854,23 +869,27 @@ void Engine::op_M_batch64(const double *x, double *z) {
          nullptr);
 }
 
-// load cases [r0, r0 + kc) together: per-column results in run_.st, displacements in d_u_
+// load cases [r0, r0 + kc) together (kc at most the width64 of the call): per-column results in run_.st,
+// displacements in d_u_
 int Engine::solve_chunk64(int r0, int kc, double &ms, std::string &err) {
     BatchRun &r = run_;
-    const int K = bK_;
+    const int K = kc <= 16 ? 16 : 32;
+    set_width64(K);
     if (!run_e0_) {
         CKB(cudaEventCreate(&run_e0_));
         CKB(cudaEventCreate(&run_e1_));
     }
-    if (!bgraph_) {
+    cudaGraphExec_t &graph = bgraph64_[K / 32];
+    int &kernels = bkernels64_[K / 32];
+    if (!graph) {
         cudaGraph_t g;
         CKB(cudaStreamBeginCapture(s_, cudaStreamCaptureModeThreadLocal));
         iteration_batch64();
         CKB(cudaStreamEndCapture(s_, &g));
         size_t nn = 0;
         CKB(cudaGraphGetNodes(g, nullptr, &nn));
-        bkernels_per_iter_ = int(nn);
-        CKB(cudaGraphInstantiate(&bgraph_, g, 0));
+        kernels = int(nn);
+        CKB(cudaGraphInstantiate(&graph, g, 0));
         cudaGraphDestroy(g);
     }
     int rc = batch_rhs(r0, kc, err);
@@ -904,8 +923,8 @@ int Engine::solve_chunk64(int r0, int kc, double &ms, std::string &err) {
     }
     CKB(cudaMemcpyAsync(b_st_, r.st.data(), K * sizeof(PcpgState), cudaMemcpyHostToDevice, s_));
     for (;;) {
-        for (int k = 0; k < std::max(1, opt_.check_every); ++k) CKB(cudaGraphLaunch(bgraph_, s_));
-        launches_ += (long long)std::max(1, opt_.check_every) * bkernels_per_iter_;
+        for (int k = 0; k < std::max(1, opt_.check_every); ++k) CKB(cudaGraphLaunch(graph, s_));
+        launches_ += (long long)std::max(1, opt_.check_every) * kernels;
         CKB(cudaMemcpyAsync(r.st.data(), b_st_, K * sizeof(PcpgState), cudaMemcpyDeviceToHost, s_));
         CKB(cudaStreamSynchronize(s_));
         bool all = true;

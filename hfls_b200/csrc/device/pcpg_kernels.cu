@@ -1,6 +1,7 @@
-// PCPG kernels of the HTFETI path (sm_100a).  All reductions are
-// deterministic (fixed-order trees, no floating-point atomics), so a solve
-// gives the same bits alone and inside a batch.
+// PCPG kernels of the HTFETI path (sm_100a), one load case.  All reductions
+// are deterministic (fixed-order trees, no floating-point atomics), so a
+// repeated solve gives the same bits.  (Load cases solved together go through
+// pcpg_multi.cu, whose sums are grouped by its width: the same to round-off.)
 //
 //  F w = Bf K_HT^+ Bf^T w   (Cluster::mult_Ff, Cluster.cpp:1114-1188):
 //    k_gather_b        x_b = Bf_d^T w             signed gather over the b slots

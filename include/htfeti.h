@@ -172,7 +172,14 @@ int htf_pcpg(htf_ctx *ctx, double *u, htf_stats *stats);
  * force; u[3*n_nodes*n_rhs] receives the displacements as in htf_pcpg.
  * Host buffers in and out; this is the call a serving loop makes per
  * request.  Replaces a repeated Cluster::pcpg with a new rhs
- * (Cluster.cpp:1385-1458) without redoing the setup.                     */
+ * (Cluster.cpp:1385-1458) without redoing the setup.
+ * FP64 form with an explicit preconditioner: three or more load cases of one
+ * call are solved together, up to 32 at a time (a last one or two alone).
+ * Each then has the result that it has alone up to round-off, and always the
+ * same bits for the same number of load cases, whatever calls came before.
+ * The first such call allocates the vectors for it, which stay until
+ * htf_destroy; where they would take more than a quarter of the free device
+ * memory, up to 16 are solved together, or one at a time.                 */
 int htf_solve(htf_ctx *ctx, int n_rhs, const double *f_nodal, double *u, htf_stats *stats);
 
 /* Device timing of the dominant kernels on the library's own stream
