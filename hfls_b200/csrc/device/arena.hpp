@@ -5,6 +5,9 @@
 // the machine call the driver too), so buffers under ARENA_OWN bytes share
 // chunks of ARENA_CHUNK bytes: about 30 calls instead of 160.  Nothing
 // outlives the owner and nothing is shared between owners.
+//
+// A dry arena allocates nothing (its buffers are null) and only counts what
+// the same calls would take.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -16,7 +19,7 @@ namespace htf {
 
 class DevArena {
 public:
-    DevArena() = default;
+    explicit DevArena(bool dry = false) : dry_(dry) {}
     DevArena(const DevArena &) = delete;
     DevArena &operator=(const DevArena &) = delete;
     ~DevArena() { clear(); }
@@ -34,7 +37,7 @@ public:
             left_ = ARENA_CHUNK;
         }
         *p = next_;
-        next_ += bytes;
+        if (!dry_) next_ += bytes;
         left_ -= bytes;
         return cudaSuccess;
     }
@@ -55,6 +58,8 @@ public:
         std::swap(left_, o.left_);
     }
 
+    bool dry() const { return dry_; }
+
     size_t bytes() const {
         size_t t = 0;
         for (auto &b : bufs_) t += b.bytes;
@@ -62,7 +67,8 @@ public:
     }
 
     void clear() {
-        for (auto &b : bufs_) cudaFree(b.p);
+        for (auto &b : bufs_)
+            if (b.p) cudaFree(b.p);
         bufs_.clear();
         next_ = nullptr;
         left_ = 0;
@@ -75,11 +81,12 @@ private:
         size_t bytes;
     };
     cudaError_t own(void **p, size_t bytes) {
-        const cudaError_t e = cudaMalloc(p, bytes);
+        const cudaError_t e = dry_ ? cudaSuccess : cudaMalloc(p, bytes);
         if (e == cudaSuccess) bufs_.push_back({*p, bytes});
         return e;
     }
     std::vector<Buf> bufs_;
+    bool dry_;
     char *next_ = nullptr;
     size_t left_ = 0;
 };

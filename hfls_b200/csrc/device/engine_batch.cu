@@ -242,7 +242,8 @@ int Engine::alloc_batch(int K, std::string &err) {
             for (int I = 0; I < hs_[d].nt; ++I) rb.push_back(make_int2(d, I));
         nrowblk_ = int(rb.size());
         d_rowblk_ = alloc<int2>(rb.size(), err, rc);
-        if (!rc) CKB(cudaMemcpyAsync(d_rowblk_, rb.data(), rb.size() * sizeof(int2), cudaMemcpyHostToDevice, s_));
+        if (!rc && !into_->dry())
+            CKB(cudaMemcpyAsync(d_rowblk_, rb.data(), rb.size() * sizeof(int2), cudaMemcpyHostToDevice, s_));
     }
     b_fullA_ = alloc<double>((size_t)nfull_ * K, err, rc);
     b_fullB_ = alloc<double>((size_t)nfull_ * K, err, rc);
@@ -796,28 +797,20 @@ int Engine::width64(int nrhs) {
 
 // Batch vectors for K columns instead of the present ones, which stay when there is no room
 bool Engine::grow_batch64(int K) {
-    long long tn = 0, nch = 1;
-    for (auto &h : hs_) {
-        tn = std::max<long long>(tn, h.t_off + h.c + 6);
-        nch = std::max<long long>(nch, (h.nb + 127) / 128);
-    }
-    const double need = 8.0 * K *
-                        (9.0 * nlam_ + 2.0 * nslots_ + 2.0 * nfull_ + double(tn) * nch + 3.0 * ngc_total_ +
-                         6.0 * nchunks_ + 2.0 * 1184.0 + double(std::max(opt_.max_iter, 0)) + 1.0);
-    size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || need > 0.25 * double(fr + bmem_.bytes())) {
-        cudaGetLastError();
-        return false;
-    }
-    if (cudaStreamSynchronize(s_) != cudaSuccess) return false;
     const BatchVectors old = *this;
-    DevArena fresh;
     std::string why;
-    into_ = &fresh;
-    int rc = alloc_batch(K, why);
-    b_hist_ = alloc<double>((size_t(std::max(opt_.max_iter, 0)) + 1) * K, why, rc);
-    into_ = &mem_;
-    if (rc) {
+    auto vectors = [&](DevArena &in) {
+        into_ = &in;
+        int rc = alloc_batch(K, why);
+        b_hist_ = alloc<double>((size_t(std::max(opt_.max_iter, 0)) + 1) * K, why, rc);
+        into_ = &mem_;
+        return rc;
+    };
+    DevArena count(true), fresh;
+    size_t fr = 0, tot = 0;
+    if (vectors(count) || cudaMemGetInfo(&fr, &tot) != cudaSuccess ||
+        double(count.bytes()) > 0.25 * double(fr + bmem_.bytes()) || cudaStreamSynchronize(s_) != cudaSuccess ||
+        vectors(fresh)) {
         cudaGetLastError();
         static_cast<BatchVectors &>(*this) = old;
         return false;
