@@ -29,7 +29,7 @@ public:
         if (bytes >= ARENA_OWN) return own(p, bytes);
         if (bytes > left_) {
             void *c = nullptr;
-            if (own(&c, ARENA_CHUNK) != cudaSuccess) {
+            if (own(&c, ARENA_CHUNK, true) != cudaSuccess) {
                 cudaGetLastError();                  // no room for a chunk: the buffer alone may still fit
                 return own(p, bytes);
             }
@@ -45,7 +45,7 @@ public:
     // frees a buffer with memory of its own now; one in a chunk stays until the end
     void release(void *p) {
         for (size_t i = 0; i < bufs_.size(); ++i)
-            if (bufs_[i].p == p && bufs_[i].bytes != ARENA_CHUNK) {
+            if (bufs_[i].p == p && !bufs_[i].chunk) {
                 cudaFree(p);
                 bufs_.erase(bufs_.begin() + i);
                 return;
@@ -79,10 +79,11 @@ private:
     struct Buf {
         void *p;
         size_t bytes;
+        bool chunk;
     };
-    cudaError_t own(void **p, size_t bytes) {
+    cudaError_t own(void **p, size_t bytes, bool chunk = false) {
         const cudaError_t e = dry_ ? cudaSuccess : cudaMalloc(p, bytes);
-        if (e == cudaSuccess) bufs_.push_back({*p, bytes});
+        if (e == cudaSuccess) bufs_.push_back({*p, bytes, chunk});
         return e;
     }
     std::vector<Buf> bufs_;
