@@ -166,6 +166,7 @@ private:
     void op_P(const double *x, double *Px, double *alpha_out, const double *dotv, double *partial,
               PcpgState *st, bool step = false);
     void iteration(PcpgState *st);
+    int iteration_graph(std::string &err);
     void coarse_apply(const double *t, double *s, const PcpgState *st);   // s = M gc, gc summed from t
     void release(void *p);
     int solve_one(Problem &p, int rhs, double *u_dev, int &iters, double &norm0, double &rel,
