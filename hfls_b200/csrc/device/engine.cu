@@ -66,7 +66,7 @@ __global__ void k_gft_partial(const int *, const int *, const int *, const doubl
 __global__ void k_gf_mult(int, const int *, const double *, const double *, double *);
 __global__ void k_update_lam_g(int, const double *, int, const double *, const double *, double *, double *,
                                PcpgState *);
-__global__ void k_update_w(int, const double *, int, const double *, double *, PcpgState *, double *, unsigned *);
+__global__ void k_update_w(int, const double *, int, const double *, double *, PcpgState *, double *, int, unsigned *);
 __global__ void k_init_state(const double *, int, PcpgState *, double, int);
 __global__ void k_axpby(int, double, const double *, double, double *);
 
@@ -539,7 +539,8 @@ int Engine::upload_layout(Problem &p, std::string &err) {
         CK(ksolve_prepare(optin));
         if (ksolve_smem(ks_blocks_) > size_t(optin)) ks_blocks_ = 0;
     }
-    d_hist_ = alloc<double>(size_t(std::max(opt_.max_iter, 0)) + 1, err, rc);
+    nhist_ = int(std::min<long long>(std::max(opt_.max_iter, 0) + 1LL, INT_MAX));
+    d_hist_ = alloc<double>(nhist_, err, rc);
     if (rc) return rc;
     {
         std::vector<int> csp(ncl_ + 1, 0), cs;
@@ -1081,7 +1082,7 @@ void Engine::iteration(PcpgState *st) {
     op_M(d_Pg_, d_z_, st);
     op_P(d_z_, d_Pz_, nullptr, d_g_, d_partial_, st);
     launch_chain(k_update_w, std::min(npart_, 1184), 256, 0, s_, nlam_, d_partial_, npart_, d_Pz_, d_w_, st, d_hist_,
-                 d_count_ + 1);
+                 nhist_, d_count_ + 1);
 }
 
 int Engine::apply(int op, const double *x, double *y, int nrhs, std::string &err) {

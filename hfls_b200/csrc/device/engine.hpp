@@ -285,6 +285,7 @@ private:
     PcpgState *d_st_ = nullptr;
     unsigned *d_count_ = nullptr;              // finished CTAs of the kernels whose last CTA does more (zero between launches)
     double *d_hist_ = nullptr;                 // relative residual per iteration of the running solve
+    int nhist_ = 0;                            // its entries: max_iter + 1
     std::vector<std::vector<double>> hist_;    // per load case (first 64) of the last plain solve
     int npart_ = 0;
     int symv_smem_ = 0;

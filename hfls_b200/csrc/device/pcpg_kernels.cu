@@ -603,9 +603,9 @@ __global__ void __launch_bounds__(256) k_update_lam_g(int n, const double *parti
 // gamma w.  The CTA that finishes last (counter, set back to zero) commits
 // the iteration: gPz and gamma, the count, the convergence test, and the
 // relative residual sqrt(g'Pz)/sqrt(g0'Pz0) of iteration it in hist[it]
-// (hist holds max_iter + 1 entries).
+// (nhist entries: a state set up for timing may run past them).
 __global__ void __launch_bounds__(256) k_update_w(int n, const double *partial, int np, const double *Pz, double *w,
-                                                  PcpgState *st, double *hist, unsigned *counter) {
+                                                  PcpgState *st, double *hist, int nhist, unsigned *counter) {
     __shared__ double red[8];
     pdl_next();
     pdl_wait();
@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(256) k_update_w(int n, const double *partial, 
             st->gPz = gPz;
             st->it += 1;
             st->rel = sqrt(gPz) / st->norm0;
-            if (hist && st->it <= st->max_iter) hist[st->it] = st->rel;
+            if (st->it < nhist) hist[st->it] = st->rel;
             if (!(st->wFw > 0.0) || !isfinite(gPz)) st->done = 2;          // breakdown
             else if (sqrt(gPz) < st->eps * st->norm0) st->done = 1;        // converged
             else if (st->it >= st->max_iter) st->done = 3;                  // max_iter
