@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) k_ksolve(const SubDev *__res
             for (int j = 0; j < 32; ++j) l[j] = j < wk ? col[j * ld] : 0.0;
         };
         auto apply = [&](const double (&l)[32], int k) {
-            ok = ok && bar_wait_cluster(&fwd[k]);
+            ok = ok && warp_agree(bar_wait_cluster(&fwd[k]));
             const double2 *yk = reinterpret_cast<const double2 *>(xs + 32 * k);
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) k_ksolve(const SubDev *__res
     // every y has landed in every CTA of the cluster (in a CTA that owns no later block nothing else waits for
     // y_b), by when no forward step reads one any more either
     for (int b = threadIdx.x; b < nblk && ok; b += blockDim.x) ok = bar_wait_cluster(&fwd[b]);
-    ok = __all_sync(0xffffffffu, ok);
+    ok = warp_agree(ok);
     cluster_sync_all();
     // backward: x_b = L_bb^{-T} (y_b - sum_{k > b} L_kb^T x_k)
     const int mine = first < nblk ? (nblk - 1 - first) / step : -1;
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) k_ksolve(const SubDev *__res
 #pragma unroll
                 for (int j = 0; j < 32; ++j) p[j] = 0.0;
             }
-            ok = ok && bar_wait_cluster(&bwd[k]);
+            ok = ok && warp_agree(bar_wait_cluster(&bwd[k]));
             const double xk = xs[32 * k + lane];                       // zero past the block's rows
 #pragma unroll
             for (int j = 0; j < 32; ++j) p[j] += l[j] * xk;
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(KS_WARPS * 32, 1) k_ksolve(const SubDev *__res
     }
     // no CTA leaves while results are on their way to it
     if (warp == 0 && ok)
-        for (int b = 0; b < nblk && ok; ++b) ok = bar_wait_cluster(&bwd[b]);
+        for (int b = 0; b < nblk && ok; ++b) ok = warp_agree(bar_wait_cluster(&bwd[b]));
     if (!ok && lane == 0) atomicExch(err, HTF_ETIMEDOUT);
     cluster_sync_all();
 }

@@ -39,4 +39,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity) {
     return false;
 }
 
+// one answer for all lanes of a warp: lanes try a barrier by themselves, so at the very limit one may give up on a
+// phase that another still sees complete, and what follows (shuffles, matrix instructions, aligned barriers) wants
+// the whole warp
+__device__ __forceinline__ bool warp_agree(bool ok) { return __all_sync(0xffffffffu, ok); }
+
 }  // namespace htf

@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(SYRK_THREADS, 1) k_syrk_update(const StepDesc 
                     half ^= 1;
                 }
             }
-            if (n >= 2) ok = mbar_wait(&empty[q], ((n >> 1) - 1) & 1);
+            if (n >= 2) ok = warp_agree(mbar_wait(&empty[q], ((n >> 1) - 1) & 1));
             if (!ok) break;
             if (warp == 8 && lane == 0) desc[q] = T;
             if (T.d >= 0) {
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(SYRK_THREADS, 1) k_syrk_update(const StepDesc 
         int row0 = 0, N = 0;
         for (int n = 0;; ++n) {
             const int q = n & 1;
-            ok = mbar_wait(&full[q], (n >> 1) & 1);
+            ok = warp_agree(mbar_wait(&full[q], (n >> 1) & 1));
             if (!ok) break;
             const SyrkTile T = desc[q];
             if (T.d < 0) break;
