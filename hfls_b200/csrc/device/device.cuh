@@ -18,8 +18,9 @@
 //   * b-space vectors (x_b, y_b) are concatenated with per-subdomain offsets
 //     xb_off (multiples of 32).
 #pragma once
-#include <vector>
+#include <cmath>
 #include <cstdint>
+#include <vector>
 
 namespace htf {
 
@@ -94,6 +95,19 @@ struct ClusterDev {
 #else
 #define HTF_HD inline
 #endif
+
+// a / b from r, the reciprocal of b to 4 units in the last place: one
+// multiplication and Markstein's correction (IBM J. Res. Dev. 34, 1990), the
+// remainder in one FMA and the quotient corrected in another.  (Markstein's
+// theorem, the correctly rounded quotient, asks for a correctly rounded r; a
+// reciprocal of 4 ulp leaves an error of at most 0.5 + 2^-44 ulp, so only a
+// quotient that close to a tie may round the other way.)  For quotients and
+// remainders in the normal range.  Three dependent FP64 operations instead of
+// a division's chain, which bounds every substitution of the factorisation.
+HTF_HD double div_by(double a, double b, double r) {
+    const double q = a * r;
+    return fma(fma(-q, b, a), r, q);
+}
 
 // doubles of the factor panels of a subdomain with nr interior DOFs and
 // nbp padded b-set DOFs, and the offset of its first b-set panel

@@ -148,22 +148,11 @@ __global__ void k_regularize(SubDev *subs, int nsub, double *Kbuf) {
 // panels): the diagonal block in one CTA, the panel below it one row per
 // thread, the trailing update keeping one accumulator per 32-column panel and
 // subtracting them in turn in registers, so each trailing tile is read and
-// written once per 64 columns.  The arithmetic is that of two successive
+// written once per 64 columns.  The sums are those of two successive
 // 32-column right-looking steps (per panel: Cholesky of the diagonal block,
-// row-wise substitution with division by the pivot, block update subtracting
-// a 32-term sum), operation for operation.
+// row-wise substitution, block update subtracting a 32-term sum), in their
+// order; quotients by the pivots come from div_by (device.cuh).
 // ---------------------------------------------------------------------------
-// a / b from r, the reciprocal of b to a few units in the last place: one
-// multiplication and Markstein's correction (IBM J. Res. Dev. 34, 1990), the
-// remainder in one FMA and the quotient corrected in another, which leaves the
-// correctly rounded quotient but for ties closer than 2^-50.  Three dependent
-// FP64 operations instead of a division's chain, which bounds every
-// substitution here.
-__device__ __forceinline__ double div_by(double a, double b, double r) {
-    const double q = a * r;
-    return fma(fma(-q, b, a), r, q);
-}
-
 // Thread t holds row t's 32 columns of the current panel in registers and
 // eliminates column by column: the pivot's square root and the finished
 // column go through shared memory, every later column of the row is one
@@ -207,7 +196,7 @@ __global__ void __launch_bounds__(CHOL_STEP) k_potrf_diag(const StepDesc *__rest
                     }
                     a[j] = sqrt(d);
                     piv[j & 1] = a[j];
-                    rpiv[j & 1] = rsqrt(d);         // beside the square root, not after it
+                    rpiv[j & 1] = rsqrt(d);         // beside the square root, not after it: 1 / a[j] to 2 ulp
                 }
                 __syncthreads();
                 if (r > j) a[j] = div_by(a[j], piv[j & 1], rpiv[j & 1]);
