@@ -220,12 +220,13 @@ int Engine::alloc_units(std::string &err) {
     std::vector<int> cands(1, SYMV_DEFAULT_TILES);
     if (opt_.autotune) cands.assign(std::begin(CANDIDATES), std::end(CANDIDATES));
     // A schedule's unit sizes are upper bounds: a problem of few tiles is cut into at least SYMV_MIN_UNITS units
-    // (four CTAs per SM), down to one tile each.  Measured per iteration: 528 tiles (8 subdomains) 59 us with units
-    // of 48 tiles, 41 with 5 to 8, 39 with 1 to 4; 7 900 tiles (32 subdomains) 88 us with 48, 78 with 12, 82 with 4;
-    // from 29 000 tiles on the bound is above 48 and the schedule's own sizes hold (43 000 tiles: 252 us with 32 or
-    // 48, 262 with 16).  One tile at least, not four: a solve of the 8 subdomains takes 2.22 ms instead of 2.11, but
-    // with four the E-contrast problem of __graft_entry__.smoke stops at 151 iterations, one beyond its bar of 148 +-
-    // 2, with one at 149 (with loads moved by 1e-17 the counts are 147 to 153 either way, mean 149.6 and 150.1).
+    // (four CTAs per SM), down to one tile each.  Measured per iteration: 444 tiles (8 subdomains) 59 us with units
+    // of 48 tiles, 41 with 5 to 8, 39 with 1 to 4; 7 100 tiles (32 subdomains) 88 us with 48, 78 with 12, 82 with 4;
+    // from 28 416 tiles on the bound is above 48 and the schedule's own sizes hold (59 000 tiles: 252 us with 32 or
+    // 48, 262 with 16).  Not the fastest minimum: with four tiles instead of one a solve of the 8 subdomains takes
+    // 2.11 ms instead of 2.22.  But that moves the round-off of an E-contrast-1000 problem checked to +-2 iterations
+    // (__graft_entry__.smoke) from 149 to 151 of 148, narrower than the problem itself: loads moved by 1e-17 give
+    // 147 to 153 with either minimum, an oracle run with its input moved by one ulp 148 to 152.
     unit_cap_ = int(std::max<long long>(1, std::min<long long>(ntiles_ / SYMV_MIN_UNITS, 1 << 20)));
     // every unit's row window is at most 32 (ut + 1) rows of 5 doubles: the
     // largest candidate (96 tiles) needs 124 KB, within the 227 KB opt-in limit

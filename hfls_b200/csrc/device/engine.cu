@@ -75,9 +75,9 @@ __global__ void k_axpby(int, double, const double *, double, double *);
 // at strides nfull (full vectors), nt (t), ng (coarse vectors) and na (alpha).
 // Bound by latency: a subdomain is one CTA, so the loads of eight terms are in
 // flight before they are added in order, and the load cases of a chunk, 2 to 5
-// launches each before, run side by side.  64 uneven subdomains, 32 load cases:
-// k_bc_rt 64 x 19 us, k_correct 32 x 18 -> 6 us, k_sub_bct 32 x 12 and k_add_R
-// 32 x 9 us; a solve 57.7 -> 55.1 ms.
+// launches each before, run side by side.  64 subdomains of 8^3 elements, 32
+// load cases: k_bc_rt 64 x 19 us, k_correct 32 x 18 -> 6 us, k_sub_bct 32 x 12
+// and k_add_R 32 x 9 us; a solve 57.7 -> 55.1 ms.
 
 // t_d = [Bc_b z_b ; -R^T y]  (y full, z full)
 __global__ void k_bc_rt(const SubDev *__restrict__ subs, const int *__restrict__ bce_ptr,

@@ -22,8 +22,12 @@
 // the chain of N / 32 blocks (2 us per block and direction).  Against one
 // CTA per subdomain with a block-wide barrier per 32 rows, forward and
 // backward: 8 subdomains of 648 DOFs 1.18 -> 0.09 ms; 64 uneven ones of up to
-// 5 577 57 -> 1.46 ms; 512 of 2 187 (10 GB of factor, read twice) 12.7 ->
+// 5 577 57 -> 1.41 ms; 512 of 2 187 (10 GB of factor, read twice) 12.7 ->
 // 4.5 ms = 4.6 TB/s.
+//
+// Both kernels here multiply by the rounded reciprocal of a pivot, 1.5 ulp a
+// quotient where a division leaves 0.5; the displacements' distance from a
+// 64-bit direct solve is the stopping rule's either way.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -320,13 +324,13 @@ cudaError_t ksolve_launch(const SubDev *subs, const int *order, int nsub, const 
 // Up to 32 right-hand sides per cluster (blockIdx.y: chunk of 32), the same
 // dataflow with a CTA instead of a warp per 32-row block: X_b = L_bb^{-1}
 // (V_b - sum_k L_bk X_k), then the transposed pass.  Results are exchanged
-// through the vectors in global memory, with a transaction barrier per block
+// through the vectors in global memory, with a barrier per block
 // in every CTA of the cluster.  The 32 x 32 x 32 products run on the FP64
 // tensor path out of double-buffered shared memory (both tiles column by
 // column with a stride of 36 doubles: no bank conflicts), factor tiles
 // prefetched two ahead into registers, X one ahead when it is known already;
-// warp w owns row tiles 2 (w / 4), + 1 and one column tile, or, with fewer
-// than 25 right-hand sides, a part of the k range of a column tile, the parts
+// warp w owns row tiles 2 (w / 4), + 1 and one column tile, or, with up to
+// 16 right-hand sides, a part of the k range of a column tile, the parts
 // added in order.  (Fragments loaded straight from global memory touch eight
 // lines per load and were bound by L1: 4.1 ms where this takes 2.2 for 64 x
 // 2 187 DOFs and 32 right-hand sides; one CTA per subdomain took 7.4.)  Also

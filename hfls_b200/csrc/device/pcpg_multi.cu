@@ -27,8 +27,9 @@ __device__ __forceinline__ void dmma_8x8x4(double &d0, double &d1, double a, dou
 // then the lo plane, SWIZZLE_64B K-major.  One CTA per 32 consecutive slots
 // (one K slab of one subdomain: b offsets and padded sizes are multiples of
 // 32); the values go through shared memory so both outputs are written
-// coalesced.  Two columns per thread and two slots per conversion (64 uneven
-// subdomains, 32 columns, 1 964 CTAs, about 45 MB in L2): 17.1 -> 13.6 us.
+// coalesced.  Two columns per thread and two slots per conversion (64
+// subdomains of 8^3 elements, 32 columns, 1 964 CTAs, about 45 MB in L2): 17.1
+// -> 13.6 us.
 __global__ void __launch_bounds__(256) k_gather_multi(int nslots, int K, const int *__restrict__ ptr,
                                                       const int *__restrict__ ent, const double *w,
                                                       const double *__restrict__ weight, double *xb,
@@ -310,7 +311,7 @@ template __global__ void k_coarse_multi<32>(const ClusterDev *, const double *, 
 // threads, thread (lr, j2) the columns 2 j2 and 2 j2 + 1 of the rows
 // lr, lr + 256 / K, ...: 16-byte accesses, half the instructions per byte of
 // one column per thread, by which these kernels (vectors in L2) are bound.  One
-// column per thread -> two, alone: 64 uneven subdomains, 32 columns:
+// column per thread -> two, alone: 64 subdomains of 8^3 elements, 32 columns:
 // k_gf_apply_multi 14.7 -> 10.4 us, updates 11.0 -> 9.3 and 10.6 -> 8.3,
 // k_rows_multi 10.1 -> 10.7; 32 uneven subdomains, 8 load cases in 16 columns:
 // 6.3 -> 5.0, 5.5 -> 4.6, 5.3 -> 5.1, 5.2 -> 4.4 us.
@@ -370,8 +371,9 @@ __device__ __forceinline__ double2 row_value(int r, int K2, const int *__restric
 // outputs in registers (rows rg + RG i, case pairs jg + JG c: conflict-free
 // 16-byte shared-memory reads), summed over the columns in order.  y is read
 // only for the subtraction, so that three CTAs fit an SM: the mixed iteration
-// of 32 load cases 1744 -> 1688 us (512-subdomain cube), 271 -> 268 (64 uneven
-// subdomains, this kernel 22 -> 20 us for 5 us of FP64 operations).
+// of 32 load cases 1744 -> 1688 us (512-subdomain cube), 271 -> 268 (64
+// subdomains of 8^3 elements, this kernel 22 -> 20 us for 5 us of FP64
+// operations).
 template <int K>
 __global__ void __launch_bounds__(256, 3) k_correct_multi(const SubDev *__restrict__ subs,
                                                        const ClusterDev *__restrict__ cl,
@@ -509,8 +511,8 @@ __global__ void __launch_bounds__(128) k_rows_multi(int nlam, int K, const int *
 // the wait, thread (lr / 4, j) walks its entries with 32 x loads in flight, and
 // the sums are added as a tree; k_gt_sum_multi adds the four parts the same
 // way.  Bound by the latency of the x loads, a row of K values each: 60 chunks
-// are 240 CTAs in four parts.  64 uneven subdomains, 32 columns (60 chunks),
-// alone: 15.8 us with one CTA per chunk, 9.8 us in parts.
+// are 240 CTAs in four parts.  64 subdomains of 8^3 elements, 32 columns (60
+// chunks), alone: 15.8 us with one CTA per chunk, 9.8 us in parts.
 constexpr int GFT_PART = 1024 / 4;                 // most entries of a part of a chunk
 __global__ void __launch_bounds__(64) k_gft_partial_multi(int K, const int *__restrict__ chunk_beg,
                                                           const int *__restrict__ chunk_end,
